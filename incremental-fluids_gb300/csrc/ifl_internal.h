@@ -15,7 +15,8 @@
 // 32 lanes contiguous.  A MIC(0) wavefront step of a strip touches exactly one
 // diagonal, so every array is read and written as one contiguous 32-element
 // line per step and a run of steps is one contiguous block (streamed into
-// shared memory by bulk copies).
+// shared memory by bulk copies).  The FP32 form's solves use the same order
+// over tiles of 2 x 4 cells (ts = 1): a lane's element is a tile of eight floats.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -49,22 +50,35 @@ struct DevBody {
     double cpos, spos, cneg, sneg;
 };
 
-// Strip-diagonal index: slot(x, y) = ((s*D + x + l)*32 + l), s = y/32, l = y%32.
-// D (diagonals per strip) covers W + 31 and is padded to a multiple of kSweepBlock.
-constexpr int kSweepBlock = 16;
+// Strip-diagonal index.  ts = 0 (FP64 and Gauss-Seidel solves): cells, slot(x, y)
+// = (s*D + x + l)*32 + l with s = y/32, l = y%32.  ts = 1 (FP32-form solves): tiles
+// of 2 columns x 4 rows, tile (X, Y) = (x/2, y/4), s = Y/32, l = Y%32; a tile
+// diagonal X + l holds the 32 lanes' first columns (4 rows each), then their
+// second columns: slot = (((s*D + X + l)*2 + x%2)*32 + l)*4 + y%4.
+// D (diagonals per strip) covers the columns + the lanes in use, padded to a
+// multiple of the sweeps' bulk-copy block.
+constexpr int kSweepBlock = 16, kTileBlock = 4;
 struct SDIdx {
-    int W, H, S, D;
+    int W, H, S, D, ts;
+    __host__ __device__ __forceinline__ int tw() const { return ts ? (W + 1) >> 1 : W; }  // columns of tiles
+    __host__ __device__ __forceinline__ int th() const { return ts ? (H + 3) >> 2 : H; }  // rows of tiles
     __host__ __device__ __forceinline__ size_t slot(int x, int y) const {
-        const int s = y >> 5, l = y & 31;
-        return ((size_t)s * D + x + l) * 32 + l;
+        if (!ts) {
+            const int s = y >> 5, l = y & 31;
+            return ((size_t)s * D + x + l) * 32 + l;
+        }
+        const int s = y >> 7, l = (y >> 2) & 31;
+        return ((((size_t)s * D + (x >> 1) + l) * 2 + (x & 1)) * 32 + l) * 4 + (y & 3);
     }
-    __host__ __device__ __forceinline__ size_t total() const { return (size_t)S * D * 32; }
-    static SDIdx make(int w, int h) {
+    __host__ __device__ __forceinline__ size_t total() const { return (size_t)S * D * (ts ? 256 : 32); }
+    static SDIdx make(int w, int h, int ts) {
         SDIdx r;
         r.W = w;
         r.H = h;
-        r.S = (h + 31) / 32;
-        r.D = (w + 31 + kSweepBlock - 1) / kSweepBlock * kSweepBlock;
+        r.ts = ts;
+        r.S = (r.th() + 31) / 32;
+        const int lanes = !ts || r.S > 1 ? 32 : r.th(), block = ts ? kTileBlock : kSweepBlock;
+        r.D = (r.tw() + lanes - 1 + block - 1) / block * block;
         return r;
     }
 };
@@ -88,11 +102,11 @@ struct Scene {
     Quant<F> q[4];  // d, t, u, v
     SDIdx sd;          // layout of the pressure-system arrays below
     double *r, *p;     // residual and solution stay FP64 in both forms
-    double *as;        // A*s, accumulated in FP64 (a consistent operator in both forms)
+    double *as;        // A*s (FP32-form pressure solves keep the FP32 values they form there)
     F *rf;             // r in storage precision for the substitutions (aliases r for FP64)
     F *z, *sa, *sb;
     F *adiag, *ax, *ay;
-    F *mic;            // MIC(0) apply record per slot: {lx, ly, pc, neighbour bits}
+    F *mic;            // MIC(0) apply operands: FP64 {lx, ly, pc, neighbour bits} per slot, FP32 form five arrays (k_pcg32.cu)
     double *pc;        // MIC(0) factor, FP64
     uint8_t *nb;
     F *udens, *vdens;
@@ -107,15 +121,39 @@ struct PcgOut {
     double max_error;
 };
 
-// Diagonals per reduction chunk of the PCG's elementwise phases.
+// Diagonals per reduction chunk of the PCG's elementwise phases, a function of
+// the scene alone (its sums must not depend on the launch).  Tiles: one diagonal
+// while the chunks are not many more than a GPU's warps, so that a small scene
+// reaches many SM quarters (an FP64 instruction occupies a quarter for 64-76
+// cycles).
 constexpr int kPcgChunk = 16;
-inline size_t pcg_chunks(const SDIdx &sd) { return ((size_t)sd.S * sd.D + kPcgChunk - 1) / kPcgChunk; }
+__host__ __device__ inline int pcg_chunk_diags(const SDIdx &sd) {
+    if (!sd.ts) return kPcgChunk;
+    const size_t n = (size_t)sd.S * sd.D;
+    return n <= 4096 ? 1 : n <= 8192 ? 2 : 4;
+}
+__host__ __device__ inline size_t pcg_chunks(const SDIdx &sd) {
+    const int c = pcg_chunk_diags(sd);
+    return ((size_t)sd.S * sd.D + c - 1) / c;
+}
+// Partial sums of a solve: maximum and dot product per chunk, sigma per strip
+// (or chunk).
+__host__ __device__ inline size_t pcg_partials(const SDIdx &sd) { return 4 * pcg_chunks(sd) + 4 * (size_t)sd.S; }
+// Halo words of a solve: two rows per strip, of D words (tiles: D + kHaloPad,
+// and at least the columns + 1 words of the rows that the factor hands over
+// between its 32-row sub-strips, two per 64 rows).
+constexpr int kHaloPad = 8;
+__host__ __device__ inline size_t pcg_halo_row(const SDIdx &sd) { return sd.ts ? (size_t)sd.D + kHaloPad : (size_t)sd.D; }
+__host__ __device__ inline size_t pcg_halo_words(const SDIdx &sd) {
+    const size_t sweeps = 2 * (size_t)sd.S * pcg_halo_row(sd), factor = sd.ts ? 4 * (size_t)sd.S * sd.W : 0;
+    return factor > sweeps ? factor : sweeps;
+}
 
 // Scratch for the persistent PCG kernel.
 struct PcgScratch {
-    double *partials;    // 4 reduction slots x pcg_chunks(sd)
-    unsigned *barrier;   // 2 words
-    unsigned long long *halo;  // 2 x S x D boundary rows handed between strips (sentinel protocol)
+    double *partials;    // pcg_partials(sd)
+    unsigned *barrier;   // arrival counter
+    unsigned long long *halo;  // pcg_halo_words(sd): boundary rows handed between strips (sentinel protocol)
     PcgOut *out;
     unsigned long long *iter_total;  // PCG iterations summed over launches
     int max_blocks;

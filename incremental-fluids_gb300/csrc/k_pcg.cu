@@ -41,214 +41,21 @@
 #include <type_traits>
 #include <vector>
 
-#include "ifl_device.cuh"
+#include "pcg_common.cuh"
 
 namespace ifl {
 
+// k_pcg32.cu
+size_t pcg32_smem(int K, int D, int stages);
+const void *pcg32_batch_fn();
+void pcg32_shape(int threads, int D, size_t smem_max, int *block, int *K, int *stages);
+cudaError_t launch_pcg32(PcgArgs<float> A, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
+                         int *blocks_used);
+
 namespace {
 
-// Dynamic shared memory of the PCG kernel, addressed through this symbol so
-// that every ring and halo access compiles to a shared-space instruction.
-extern __shared__ __align__(128) char g_smem[];
-
-// Threads per block: 512 for a scene that has the GPU to itself, 256 in the
-// compact launch used when many scenes run concurrently.
-constexpr int kMaxWarps = 16;
 constexpr int kChunk = kPcgChunk;  // diagonals per reduction chunk of the elementwise phases
-// Diagonals per bulk-copy block of a sweep ring (the layout's padding unit).
-// Halving it lets 16 single-warp blocks share an SM, which measured slower on
-// full batch steps (30.7 M against 36.5 M cell-steps/s): the second warp of a
-// 64-thread block, which works only in the elementwise passes, pays for more.
-constexpr int kB = kSweepBlock;
-// Default polls of a halo-word or barrier wait (about a second); the host may
-// set another limit per solve (PcgConfig::wait_limit).  The mbarrier waits of
-// the bulk-copy rings keep their own fixed limit: they wait for copies this
-// warp issued from this GPU's memory, which always complete, and a timed-out
-// sweep still waits for every copy it issued before it leaves.
-constexpr long long kWaitLimit = 1ll << 22;
-constexpr long long kMbarWaitLimit = 1ll << 20;  // try_wait suspends between polls
-constexpr double kTau = 0.97, kSigma = 0.25, kTol = 1e-5;
-constexpr unsigned long long kSentinel = ~0ull;
-constexpr unsigned FULL = 0xffffffffu;
-
-// Status words a wait checks: the scene's own and one shared by every scene
-// of a batched launch (the same word for a single-scene launch).  A timed-out
-// wait marks both, so every later wait of the launch stops waiting.
-struct Flags {
-    unsigned *scene, *all;
-    long long limit;  // polls of one halo or barrier wait before it gives up
-};
-
-// The blocks that solve one scene: ranks 0..size-1, their barrier words and
-// the per-block partial sums.  A single-scene launch is one team of the whole
-// grid.
-struct Team {
-    int rank, size;
-    unsigned *barrier;
-    double *partials;
-};
-
-template <typename F>
-struct PcgArgs {
-    SDIdx sd;
-    const F *adiag, *ax, *ay;
-    double *pc;
-    F *mic;  // MIC record per slot: {lx, ly, pc, neighbour bits}
-    const uint8_t *nb;
-    double *r, *p, *as;
-    F *rf;  // r in storage precision for the substitutions (== r when F is double)
-    F *z, *sa, *sb;
-    double *partials;
-    unsigned *barrier;
-    Flags fl;
-    unsigned long long *halo;  // [2][S][D]: [0] rows handed upward, [1] rows handed downward
-    PcgOut *out;
-    unsigned long long *iter_total;
-    int mode, limit, pinned;
-    int K, stages;
-    int rowsum_zero;  // 1: pressure matrix (rows sum to zero), 0: heat matrix
-    int all_red;      // 1: every cell takes part in the dot products and AXPYs (unmasked solves)
-};
-
-// ------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// 1-D bulk copy global -> shared (16-byte aligned, size a multiple of 16).
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ bool timed_out(const Flags &f) {
-    return (ld_volatile(f.scene) | ld_volatile(f.all)) & FLAG_TIMEOUT;
-}
-__device__ __forceinline__ void set_timeout(const Flags &f) {
-    atomicOr(f.scene, FLAG_TIMEOUT);
-    if (f.all != f.scene) atomicOr(f.all, FLAG_TIMEOUT);
-}
-
-// Team barrier: arrival counter + generation word, bounded wait.  A team of
-// one block needs only the block barrier.
-__device__ void team_barrier(const Team &T, const Flags &fl) {
-    __syncthreads();
-    if (T.size == 1) return;
-    if (threadIdx.x == 0) {
-        unsigned *bar = T.barrier;
-        unsigned g = ld_volatile(bar + 1);
-        __threadfence();
-        unsigned arrived = atomicAdd(bar, 1u);
-        if (arrived == (unsigned)T.size - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            long long n = 0;
-            while (ld_volatile(bar + 1) == g) {
-                if (++n > fl.limit || timed_out(fl)) {
-                    set_timeout(fl);
-                    break;
-                }
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
-    return v;
-}
-__device__ __forceinline__ double warp_max(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = smax(v, __shfl_down_sync(FULL, v, o));
-    return v;
-}
-
-// ------------------------------------------------------------ halo words
-__device__ __forceinline__ unsigned long long henc(double v) { return (unsigned long long)__double_as_longlong(v); }
-__device__ __forceinline__ unsigned long long henc(float v) { return (unsigned long long)__float_as_uint(v); }
-template <typename V> __device__ __forceinline__ V hdec(unsigned long long w);
-template <> __device__ __forceinline__ double hdec<double>(unsigned long long w) {
-    return __longlong_as_double((long long)w);
-}
-template <> __device__ __forceinline__ float hdec<float>(unsigned long long w) { return __uint_as_float((unsigned)w); }
-
-// Halo rows: shared memory between warps of one block, global memory between
-// blocks.  A channel holds the row's generic address, so one instruction
-// serves both spaces (relaxed, GPU scope; stronger than a shared row needs).
-// One 8-byte access is single-copy atomic, so a reader sees either the
-// sentinel or the whole word.  A halo word carries its value itself, so no
-// other memory access has to be ordered around it: the asm statements are
-// volatile (kept, in program order) but do not clobber memory.  Loads and
-// stores are predicated inside the asm: a sweep step never branches around a
-// halo access.
-struct Chan {
-    unsigned long long *row;  // generic address of the row (word x at row + x)
-    bool valid;
-};
-__device__ __forceinline__ unsigned long long hload(const Chan &c, int x) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(v) : "l"(c.row + x));
-    return v;
-}
-// The word at x where p holds, else `other`.
-__device__ __forceinline__ unsigned long long hload_if(const Chan &c, int x, bool p, unsigned long long other) {
-    unsigned long long v = other;
-    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.relaxed.gpu.u64 %0, [%1];\n}\n"
-                 : "+l"(v)
-                 : "l"(c.row + x), "r"((unsigned)p));
-    return v;
-}
-__device__ __forceinline__ void hstore_if(const Chan &c, int x, unsigned long long v, bool p) {
-    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q st.relaxed.gpu.u64 [%0], %1;\n}\n" ::"l"(c.row + x),
-                 "l"(v), "r"((unsigned)p));
-}
-
-// Halo words of one sub-block: lane l < n needs the word at column xs[l]
-// (need), prefetched in w.  Lanes whose word is still the sentinel poll it
-// (bounded; the whole warp loops together, only in this slow path); then the
-// sentinel goes back for the next sweep.  A timed-out wait yields 0.
-__device__ __forceinline__ unsigned long long halo_take_warp(const Chan &c, int x, bool need, unsigned long long w,
-                                                             const Flags &flags) {
-    if (__any_sync(FULL, need && w == kSentinel)) {
-        long long n = 0;
-        bool given_up = false;
-        for (;;) {
-            const bool wait = need && w == kSentinel && !given_up;
-            if (!__any_sync(FULL, wait)) break;
-            if (wait) {
-                w = hload(c, x);
-                if (w == kSentinel && (++n > flags.limit || timed_out(flags))) {
-                    set_timeout(flags);
-                    given_up = true;
-                }
-            }
-        }
-        if (given_up) w = 0ull;
-    }
-    hstore_if(c, x, kSentinel, need);
-    return w;
-}
+constexpr int kB = kSweepBlock;    // diagonals per bulk-copy block of a sweep ring (the layout's padding unit)
 
 // --------------------------------------------------------------- sweeps
 // Per-warp shared-memory ring: `stages` buffers, each holding kB diagonals
@@ -266,9 +73,8 @@ __device__ __forceinline__ unsigned long long halo_take_warp(const Chan &c, int 
 // The same warp state carries the staging area of the elementwise passes:
 // sbuf/sbytes (this warp's share of the block's ring memory, idle outside the
 // sweeps), the staging mbarrier at sbar and its completed phases sphase.
-template <typename F>
 struct Ring {
-    static constexpr unsigned kSlot = kB * 32 * sizeof(F);
+    static constexpr unsigned kSlot = kB * 32 * sizeof(double);
     static constexpr unsigned kStageBytes = 6 * kSlot;
     unsigned buf;   // byte offset of this warp's stages in g_smem
     unsigned bars;  // byte offset of this warp's mbarriers in g_smem
@@ -286,8 +92,7 @@ struct Ring {
 // and completes, and a stage is re-armed only after its previous phase
 // completed, so the ring never leaves a bulk copy writing shared memory behind
 // (every sweep consumes every block it issued).
-template <typename F>
-__device__ __forceinline__ void ring_wait(Ring<F> &R, const Flags &flags) {
+__device__ __forceinline__ void ring_wait(Ring &R, const Flags &flags) {
     const unsigned st = R.ci % R.stages, parity = (R.ci / R.stages) & 1u;
     long long n = 0;
     while (!R.dead && !mbar_try_wait(R.bar(st), parity)) {
@@ -300,18 +105,18 @@ __device__ __forceinline__ void ring_wait(Ring<F> &R, const Flags &flags) {
     R.ci++;
 }
 
-template <int KIND, typename F>
-__device__ __forceinline__ void ring_issue(Ring<F> &R, const PcgArgs<F> &A, int s, int blk) {
+template <int KIND>
+__device__ __forceinline__ void ring_issue(Ring &R, const PcgArgs<double> &A, int s, int blk) {
     if (R.dead) {
         R.ii++;
         return;
     }
-    constexpr unsigned S1 = Ring<F>::kSlot;
+    constexpr unsigned S1 = Ring::kSlot;
     const int D = A.sd.D;
     const int d0 = (KIND == 2) ? D - (blk + 1) * kB : blk * kB;
     const size_t off = ((size_t)s * D + d0) * 32;
     const unsigned st = R.ii % R.stages;
-    char *dst = g_smem + R.buf + st * Ring<F>::kStageBytes;
+    char *dst = g_smem + R.buf + st * Ring::kStageBytes;
     uint64_t *bar = R.bar(st);
     if (KIND == 0) {
         mbar_expect_tx(bar, 3 * S1 + kB * 32);
@@ -331,48 +136,19 @@ __device__ __forceinline__ void ring_issue(Ring<F> &R, const PcgArgs<F> &A, int 
     R.ii++;
 }
 
-__device__ __forceinline__ void ld4(const float *p, float &a, float &b, float &c, float &d) {
-    const float4 v = *(const float4 *)p;
-    a = v.x; b = v.y; c = v.z; d = v.w;
-}
 __device__ __forceinline__ void ld4(const double *p, double &a, double &b, double &c, double &d) {
     const double2 v0 = *(const double2 *)p, v1 = *(const double2 *)(p + 2);
     a = v0.x; b = v0.y; c = v1.x; d = v1.y;
-}
-__device__ __forceinline__ void st4(float *p, float a, float b, float c, float d) {
-    *(float4 *)p = make_float4(a, b, c, d);
 }
 __device__ __forceinline__ void st4(double *p, double a, double b, double c, double d) {
     *(double2 *)p = make_double2(a, b);
     *(double2 *)(p + 2) = make_double2(c, d);
 }
-// Float-float numbers (hi + lo, |lo| <= ulp(hi)/2): an exact product of two
-// floats and a sum with an error-free two-sum of the high parts (Knuth's
-// TwoSum; the library is compiled without contraction, so these stay exact).
-struct FF {
-    float hi, lo;
-};
-__device__ __forceinline__ FF ff_prod(float a, float b) {
-    const float p = a * b;
-    return FF{p, fmaf(a, b, -p)};
-}
-__device__ __forceinline__ FF ff_add(FF x, FF y) {
-    const float s = x.hi + y.hi;
-    const float bb = s - x.hi;
-    const float err = (x.hi - (s - bb)) + (y.hi - bb);
-    const float lo = err + x.lo + y.lo;
-    const float hi = s + lo;
-    return FF{hi, lo - (hi - s)};
-}
-
-// t - a*b: one fused multiply-add in the FP32 form; two roundings in FP64, as
-// the reference computes it (the FP64 path must stay bit-identical).
-__device__ __forceinline__ float msub(float t, float a, float b) { return fmaf(-a, b, t); }
+// t - a*b with two roundings, as the reference computes it (the FP64 path must
+// stay bit-identical; the library is compiled without contraction).
 __device__ __forceinline__ double msub(double t, double a, double b) { return t - a * b; }
-__device__ __forceinline__ unsigned nb_of(float w) { return __float_as_uint(w); }
 __device__ __forceinline__ unsigned nb_of(double w) { return (unsigned)__double_as_longlong(w); }
-__device__ __forceinline__ float nb_word(unsigned b, float) { return __uint_as_float(b); }
-__device__ __forceinline__ double nb_word(unsigned b, double) { return __longlong_as_double((long long)b); }
+__device__ __forceinline__ double nb_word(unsigned b) { return __longlong_as_double((long long)b); }
 
 // One strip of a wavefront sweep.  `in` is the halo row written by the
 // neighbouring strip this one depends on (IN says at compile time whether it
@@ -384,18 +160,15 @@ __device__ __forceinline__ double nb_word(unsigned b, double) { return __longlon
 // each boundary value as soon as the chain computes it) and issues its
 // stores.
 //
-// Halo words: the FP32 forward sweep hands over the pair (q, aPlusY*precon)
-// of the strip's top cell packed in one 8-byte word, so the strip above needs
-// no load of its lower neighbour's MIC(0) record; the other sweeps hand over
-// the value alone (the factor and the FP64 forward sweep load the lower
-// neighbour's coefficients with the prefetch).
-template <int KIND, typename F, bool IN>
-__device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan in, const Chan out) {
-    using V = typename std::conditional<KIND == 0, double, F>::type;
-    constexpr int kHB = sizeof(F) == 8 ? 4 : 8;
+// Halo words hand over the value alone (the factor and the forward sweep load
+// the lower neighbour's coefficients with the prefetch).
+template <int KIND, bool IN>
+__device__ void sweep_strip(const PcgArgs<double> &A, int s, Ring &R, const Chan in, const Chan out) {
+    using F = double;
+    using V = double;
+    constexpr int kHB = 4;
     constexpr bool bwd = KIND == 2;
-    constexpr bool kPair = KIND == 1 && sizeof(F) == 4;  // packed (q, ly) words
-    constexpr unsigned S1 = Ring<F>::kSlot;
+    constexpr unsigned S1 = Ring::kSlot;
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     const int W = sd.W, H = sd.H, D = sd.D;
@@ -412,13 +185,6 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
 
     V prev = V(0);                   // result of the previous cell in sweep order
     F prev_a = F(0), prev_b = F(0);  // forward: lx, ly of that cell; factor: ax, ay
-    // FP32 form, forward solve: this lane's sum of q*q over its cells (sigma,
-    // see pcg_job), fused FP32 products over one staged block of diagonals,
-    // then added in FP64 (keeps the FP64 pipe, 1/64 of the FP32 rate on this
-    // part, off the per-cell path).
-    constexpr bool kQQ = KIND == 1 && sizeof(F) == 4;
-    double qq = 0.0;
-
     // Halo prefetch: lane l < kHB holds the word of the column that the
     // waiting lane reaches at step t0 + l, and where needed the lower
     // neighbour's coefficients.
@@ -436,7 +202,7 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
                     spre_a = axp[k];
                     spre_b = ayp[k];
                 }
-            } else if constexpr (KIND == 1 && !kPair) {
+            } else if constexpr (KIND == 1) {
                 if (need) {
                     F a, b, c, d;
                     ld4(micp + 4 * sd.slot(xc, s * 32 - 1), a, b, c, d);
@@ -449,23 +215,22 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
     if (lane == 0) {
         fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
         const int pro = nblk < R.stages - 1 ? nblk : R.stages - 1;
-        for (int b = 0; b < pro; b++) ring_issue<KIND, F>(R, A, s, b);
+        for (int b = 0; b < pro; b++) ring_issue<KIND>(R, A, s, b);
     }
     prefetch(0);
     __syncwarp();
     for (int blk = 0; blk < nblk; blk++) {
         if (blk + R.stages - 1 < nblk) {
             __syncwarp();
-            if (lane == 0) ring_issue<KIND, F>(R, A, s, blk + R.stages - 1);
+            if (lane == 0) ring_issue<KIND>(R, A, s, blk + R.stages - 1);
         }
         const unsigned st = R.ci % R.stages;
         ring_wait(R, A.fl);
-        const char *sbuf = g_smem + R.buf + st * Ring<F>::kStageBytes;
+        const char *sbuf = g_smem + R.buf + st * Ring::kStageBytes;
         const F *g0 = (const F *)sbuf;
         const F *g1 = (const F *)(sbuf + S1);
         const F *g2 = (const F *)(sbuf + 2 * S1);
         const uint8_t *gnb = (const uint8_t *)(sbuf + 3 * S1);
-        float qq32 = 0.f;
         for (int sub = 0; sub < kB / kHB; sub++) {
             const int t0 = blk * kB + sub * kHB;
             // stage this sub-block's operands in registers
@@ -542,14 +307,8 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
                     F ly_d = __shfl_up_sync(FULL, prev_b, 1);
                     if constexpr (IN) {
                         F hq, hly;
-                        if constexpr (kPair) {
-                            const unsigned long long wj = __shfl_sync(FULL, hw, jj);
-                            hq = __uint_as_float((unsigned)wj);
-                            hly = __uint_as_float((unsigned)(wj >> 32));
-                        } else {
-                            hq = hdec<F>(__shfl_sync(FULL, hw, jj));
-                            hly = __shfl_sync(FULL, hb, jj);
-                        }
+                        hq = hdec<F>(__shfl_sync(FULL, hw, jj));
+                        hly = __shfl_sync(FULL, hb, jj);
                         if (lane == 0) {
                             q_d = hq;
                             ly_d = hly;
@@ -579,12 +338,7 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
                 {
                     const int t = t0 + jj;
                     const int x = (bwd ? D - 1 - t : t) - lane;
-                    unsigned long long wv;
-                    if constexpr (kPair)
-                        wv = (unsigned long long)__float_as_uint(val) | ((unsigned long long)__float_as_uint(o2[jj]) << 32);
-                    else
-                        wv = henc(val);
-                    hstore_if(out, x, wv, producer && rowok && x >= 0 && x < W);
+                    hstore_if(out, x, henc(val), producer && rowok && x >= 0 && x < W);
                 }
             }
             // stores
@@ -602,32 +356,22 @@ __device__ void sweep_strip(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan i
                         const double pcv = res[jj];
                         if (self) pcp[i] = pcv;
                         st4(micp + 4 * i, self ? (F)((double)o1[jj] * pcv) : F(0),
-                            self ? (F)((double)o2[jj] * pcv) : F(0), self ? (F)pcv : F(0), nb_word(b, F(0)));
+                            self ? (F)((double)o2[jj] * pcv) : F(0), self ? (F)pcv : F(0), nb_word(b));
                     } else {
-                        if (b & NB_SELF) {
-                            zout[i] = res[jj];
-                            if constexpr (kQQ) qq32 = fmaf((float)res[jj], (float)res[jj], qq32);
-                        }
+                        if (b & NB_SELF) zout[i] = res[jj];
                     }
                 }
             }
         }
-        if constexpr (kQQ) qq += (double)qq32;
-    }
-    if constexpr (kQQ) {
-        // the strip's partial: lanes by a fixed shuffle tree (independent of
-        // which warp of which team sweeps the strip)
-        qq = warp_sum(qq);
-        if (lane == 0) A.partials[2 * (size_t)((sd.S * D + kChunk - 1) / kChunk) + s] = qq;
     }
     __syncwarp();
 }
 
-template <int KIND, typename F>
-__device__ __forceinline__ void sweep_strip_any(const PcgArgs<F> &A, int s, Ring<F> &R, const Chan in,
+template <int KIND>
+__device__ __forceinline__ void sweep_strip_any(const PcgArgs<double> &A, int s, Ring &R, const Chan in,
                                                 const Chan out) {
-    if (in.valid) sweep_strip<KIND, F, true>(A, s, R, in, out);
-    else sweep_strip<KIND, F, false>(A, s, R, in, out);
+    if (in.valid) sweep_strip<KIND, true>(A, s, R, in, out);
+    else sweep_strip<KIND, false>(A, s, R, in, out);
 }
 
 // Sweep of all strips of this block.  The team's T.size*K sweeping warps take
@@ -643,8 +387,8 @@ __device__ __forceinline__ void sweep_strip_any(const PcgArgs<F> &A, int s, Ring
 // boundary row over through its own global row (a shared row would be reused
 // by the next round while its reader may still need it).
 // hsm_off: byte offset in g_smem of the K-1 shared halo rows (D words each).
-template <int KIND, typename F>
-__device__ void sweep(const PcgArgs<F> &A, const Team &T, Ring<F> &R, unsigned hsm_off, int nstrips_blk) {
+template <int KIND>
+__device__ void sweep(const PcgArgs<double> &A, const Team &T, Ring &R, unsigned hsm_off, int nstrips_blk) {
     const int w = threadIdx.x >> 5;
     if (w >= nstrips_blk) return;
     const SDIdx sd = A.sd;
@@ -670,7 +414,7 @@ __device__ void sweep(const PcgArgs<F> &A, const Team &T, Ring<F> &R, unsigned h
                 in = (one_round && w + 1 < nstrips_blk) ? smem_row(w) : glob_row(down + (size_t)(s + 1) * D);
             if (s > 0) out = (one_round && w > 0) ? smem_row(w - 1) : glob_row(down + (size_t)s * D);
         }
-        sweep_strip_any<KIND, F>(A, s, R, in, out);
+        sweep_strip_any<KIND>(A, s, R, in, out);
     }
 }
 
@@ -685,8 +429,7 @@ __host__ __device__ __forceinline__ unsigned ring_offset(int K, int D) {
 }
 
 // Per-warp ring and staging state; the mbarriers are initialised once per launch.
-template <typename F>
-__device__ void ring_init(Ring<F> &R, int K, int stages) {
+__device__ void ring_init(Ring &R, int K, int stages) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     R.bars = 32u * warp;
     R.stages = stages;
@@ -723,8 +466,7 @@ __device__ __forceinline__ int unit_rows(unsigned area, unsigned bytes_per_row) 
 // Wait for the unit in flight.  Like the ring, a timeout elsewhere does not
 // shorten it (the copies complete); a copy that never completes marks the
 // staging area dead, after which the warp issues and waits for nothing more.
-template <typename F>
-__device__ __forceinline__ void stage_wait(Ring<F> &R, const Flags &flags) {
+__device__ __forceinline__ void stage_wait(Ring &R, const Flags &flags) {
     long long n = 0;
     while (!R.sdead && !mbar_try_wait(R.stage_bar(), R.sphase & 1u)) {
         if (++n > kMbarWaitLimit) {
@@ -757,8 +499,9 @@ __device__ __forceinline__ unsigned clipped_bytes(int lo, int hi, int rows) {
 // One complete solve (factor and/or PCG, by A.mode) of one scene by team T.
 // The shared halo rows must hold the sentinel on entry; they hold it again on
 // exit (every word a strip hands on is taken by its neighbour).
-template <typename F, int kThreads>
-__device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *sm) {
+template <int kThreads>
+__device__ void pcg_job(const PcgArgs<double> &A, Team &T, Ring &R, double *sm) {
+    using F = double;
     constexpr int kWarps = kThreads / 32;
     const SDIdx sd = A.sd;
     const int W = sd.W, H = sd.H, D = sd.D;
@@ -783,8 +526,8 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
     // loads (from L2: other blocks wrote them before the team barrier) are
     // issued eight at a time, so a scene of thousands of chunks costs a few
     // memory latencies, not one per 32 chunks.
-    // n: the slot's number of partials (chunks; strips for sigma).
-    auto chunk_total = [&](int slot, bool is_max, int n) -> double {
+    auto chunk_total = [&](int slot, bool is_max) -> double {
+        const int n = nchunk;
         if (threadIdx.x < 32) {
             double acc = 0.0;
             const double *pt = A.partials + (size_t)slot * nchunk;
@@ -807,12 +550,11 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
     // sweeping warps of this block that own at least one strip
     int nstrips_blk = sd.S - T.rank * A.K;
     nstrips_blk = nstrips_blk < 0 ? 0 : (nstrips_blk > A.K ? A.K : nstrips_blk);
-    constexpr bool kF32 = !std::is_same<F, double>::value;
     const unsigned hsm_off = halo_offset(A.K);
-    R.buf = ring_offset(A.K, D) + (unsigned)warp * A.stages * Ring<F>::kStageBytes;
+    R.buf = ring_offset(A.K, D) + (unsigned)warp * A.stages * Ring::kStageBytes;
 
     // Staging area of this warp: its share of the block's ring memory.
-    R.sbytes = (A.K * A.stages * Ring<F>::kStageBytes / kWarps) & ~127u;
+    R.sbytes = (A.K * A.stages * Ring::kStageBytes / kWarps) & ~127u;
     R.sbuf = ring_offset(A.K, D) + (unsigned)warp * R.sbytes;
     // Lane 0 of a warp starts a unit's copies: the warp's reads of the previous
     // unit are done (syncwarp), then a proxy fence orders them before the
@@ -824,11 +566,10 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
         return true;
     };
 
-    // sigma = z . r over the red cells (3-conjugate-gradients/Fluid.cpp:356, 376).
-    // FP64 form: a separate pass after the backward solve, z_i * r_i as the
-    // reference forms them (FP64 products on the sweeping warp's chain would
-    // cost the wavefront more than the pass).  Staged: z, r and the neighbour
-    // bits of a unit.
+    // sigma = z . r over the red cells (3-conjugate-gradients/Fluid.cpp:356, 376):
+    // a separate pass after the backward solve, z_i * r_i as the reference forms
+    // them (these products on the sweeping warp's chain would cost the wavefront
+    // more than the pass).  Staged: z, r and the neighbour bits of a unit.
     auto dot_zr = [&]() {
         constexpr unsigned kRow = 32u * (sizeof(F) + 8 + 1);
         const int U = unit_rows(R.sbytes, kRow);
@@ -855,24 +596,10 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
             chunk_put(2, c, acc, false);
         }
     };
-    // FP32 form: sigma is taken as q . q, q = L^-1 r the forward solve's result.
-    // The MIC(0) apply is z = L^-T L^-1 r with L's diagonal 1/precon and its
-    // strictly lower part aPlus*precon of the column's cell (the forward solve's
-    // coefficients; the backward solve uses the same ones transposed, also after
-    // FP32 rounding), so z . r = (L^-1 r) . (L^-1 r) exactly, and in floating
-    // point within the rounding of the two triangular solves.  The forward sweep
-    // adds q*q up per strip (slot 2 holds one partial per strip): no pass over z
-    // and r and no team barrier for it.  Cells outside the masked MIC(0) work
-    // hold q = 0 (and r = 0: the right-hand side and A*s vanish there), so they
-    // add nothing to either form.
     auto sigma_of_sweeps = [&]() -> double {
-        if constexpr (kF32) {
-            return chunk_total(2, false, sd.S);
-        } else {
-            dot_zr();
-            team_barrier(T, A.fl);
-            return chunk_total(2, false, nchunk);
-        }
+        dot_zr();
+        team_barrier(T, A.fl);
+        return chunk_total(2, false);
     };
 
     // s = z + beta*s (first iteration: s = z), then z' = A s and z'.s over a
@@ -1008,47 +735,14 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
 #pragma unroll
                     for (int q = 0; q < 5; q++)
                         sv[q] = iter == 0 ? vz[q] : ((vn[q] & NB_RED) ? F(vz[q] + vs[q] * fbeta) : vs[q]);
-                    // FP64 form: FP64 accumulation in the reference's order.  FP32
-                    // form, pressure matrices (rows sum to zero in the reference:
-                    // aDiag = sum of the face factors, each off-diagonal = -factor):
-                    // the form sum_j a_ij (s_j - s_i), in FP32 fused multiply-adds.
-                    // It keeps the zero row sums exactly (with the FP32-rounded aDiag
-                    // the plain form left a tiny, non-zero eigenvalue that made CG
-                    // stagnate on some scenes, up to the 2000-iteration cap), and its
-                    // terms carry no cancellation between the diagonal and the
-                    // neighbours, so FP32 accumulation suffices: against a
-                    // float-float sum, the 512-scene batch ran the same iteration
-                    // counts (to 3 of 639 on the longest solve) with a pressure error
-                    // against the FP64 reference of 1.5e-6 (8e-7), 7 % faster.
-                    // Other FP32-form matrices (heat): a float-float sum of the
-                    // exact products on the FP32 pipes (GB300 runs FP64 at 1/64 of
-                    // the FP32 rate).
-                    double t;
-                    if constexpr (kF32) {
-                        if (A.rowsum_zero) {
-                            float tf = 0.f;
+                    // accumulated in the reference's order
+                    double t = va[0] * sv[0];
 #pragma unroll
-                            for (int q = 1; q < 5; q++)
-                                if (fl & (2u << q)) tf = fmaf(va[q], sv[q] - sv[0], tf);
-                            t = (double)tf;
-                        } else {
-                            FF acc = ff_prod(va[0], sv[0]);
-#pragma unroll
-                            for (int q = 1; q < 5; q++)
-                                if (fl & (2u << q)) acc = ff_add(acc, ff_prod(va[q], sv[q]));
-                            t = (double)acc.hi + (double)acc.lo;
-                        }
-                    } else {
-                        t = (double)va[0] * (double)sv[0];
-#pragma unroll
-                        for (int q = 1; q < 5; q++)
-                            t = (fl & (2u << q)) ? t + (double)va[q] * (double)sv[q] : t;
-                    }
+                    for (int q = 1; q < 5; q++) t = (fl & (2u << q)) ? t + va[q] * sv[q] : t;
                     const size_t i = (size_t)(r0 + u) * 32 + lane;
                     sn[i] = in ? sv[0] : F(0);
                     asp[i] = in ? t : 0.0;
-                    if (in && (vn[0] & NB_RED))
-                        dacc = kF32 ? fma(t, (double)sv[0], dacc) : dacc + t * (double)sv[0];
+                    if (in && (vn[0] & NB_RED)) dacc = dacc + t * sv[0];
                 }
             }
             chunk_put(1, c, dacc, false);
@@ -1067,7 +761,6 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
         const F *__restrict__ snp = (iter & 1) ? A.sa : A.sb;  // the s this iteration's matvec wrote
         double *__restrict__ pp = A.p;
         double *__restrict__ rp = A.r;
-        F *rfp = A.rf;  // aliases r in the FP64 form (not written there)
         if (lane == 0) fence_proxy_async_global();
         for (int c = c_begin; c < c_end; c++) {
             unsigned long long mx = 0ull;  // bits of the largest |r| so far
@@ -1099,12 +792,9 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
                     }
                     if (red) {
                         const size_t i = (size_t)(r0 + u) * 32 + lane;
-                        // FP32 form: one rounding per update (fused); FP64 form: the
-                        // reference's two
-                        pp[i] = kF32 ? fma((double)ssn[k], alpha, sp[k]) : sp[k] + (double)ssn[k] * alpha;
-                        const double rn = kF32 ? fma(sas[k], -alpha, sr[k]) : sr[k] + sas[k] * -alpha;
+                        pp[i] = sp[k] + ssn[k] * alpha;
+                        const double rn = sr[k] + sas[k] * -alpha;
                         rp[i] = rn;
-                        if (kF32) rfp[i] = (F)rn;
                         // std::max(maxError, |r|) on the bit patterns: non-negative
                         // doubles order as unsigned integers; a NaN (above +inf) is
                         // skipped, as (maxError < NaN) is false
@@ -1119,7 +809,7 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
     };
 
     if (A.mode & PCG_FACTOR) {
-        sweep<0, F>(A, T, R, hsm_off, nstrips_blk);
+        sweep<0>(A, T, R, hsm_off, nstrips_blk);
         team_barrier(T, A.fl);
     }
     if (!(A.mode & PCG_SOLVE)) return;
@@ -1130,19 +820,17 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
         for (int row = c * kChunk; row < min(rows, (c + 1) * kChunk); row++) {
             const size_t i = (size_t)row * 32 + lane;
             A.p[i] = 0.0;
-            if (kF32) A.rf[i] = (F)A.r[i];
             if (A.nb[i] & NB_RED) mx = smax(mx, fabs(A.r[i]));
         }
         chunk_put(0, c, mx, true);
     }
-    if (kF32) team_barrier(T, A.fl);  // FP32 copy of r complete
     // z = M^-1 r  (:351)
-    sweep<1, F>(A, T, R, hsm_off, nstrips_blk);
+    sweep<1>(A, T, R, hsm_off, nstrips_blk);
     team_barrier(T, A.fl);
-    sweep<2, F>(A, T, R, hsm_off, nstrips_blk);
+    sweep<2>(A, T, R, hsm_off, nstrips_blk);
     team_barrier(T, A.fl);
 
-    double maxError = chunk_total(0, true, nchunk);
+    double maxError = chunk_total(0, true);
     double sigma = sigma_of_sweeps();
     int iterations = 0, status;
     if (A.pinned >= 0 ? A.pinned == 0 : maxError < kTol) {
@@ -1159,21 +847,21 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
             if (A.all_red) matvec(iter, beta, std::true_type{});
             else matvec(iter, beta, std::false_type{});
             team_barrier(T, A.fl);
-            const double alpha = sigma / chunk_total(1, false, nchunk);
+            const double alpha = sigma / chunk_total(1, false);
             // p += alpha s; r -= alpha z'; maxError = |r|_inf  (:363-366)
             if (A.all_red) axpy(iter, alpha, std::true_type{});
             else axpy(iter, alpha, std::false_type{});
             team_barrier(T, A.fl);
-            maxError = chunk_total(0, true, nchunk);
+            maxError = chunk_total(0, true);
             iterations = iter + 1;
             if (A.pinned >= 0 ? iterations >= A.pinned : maxError < kTol) {
                 status = 0;
                 break;
             }
             // z = M^-1 r; sigmaNew = z.r  (:372-376)
-            sweep<1, F>(A, T, R, hsm_off, nstrips_blk);
+            sweep<1>(A, T, R, hsm_off, nstrips_blk);
             team_barrier(T, A.fl);
-            sweep<2, F>(A, T, R, hsm_off, nstrips_blk);
+            sweep<2>(A, T, R, hsm_off, nstrips_blk);
             team_barrier(T, A.fl);
             const double sigmaNew = sigma_of_sweeps();
             beta = sigmaNew / sigma;
@@ -1189,135 +877,63 @@ __device__ void pcg_job(const PcgArgs<F> &A, const Team &T, Ring<F> &R, double *
     }
 }
 
-template <typename F, int kThreads>
-__global__ void __launch_bounds__(kThreads, 1) pcg_kernel(PcgArgs<F> A) {
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) pcg_kernel(PcgArgs<double> A) {
     __shared__ double sm[kMaxWarps + 1];
-    const Team T{(int)blockIdx.x, (int)gridDim.x, A.barrier, A.partials};
-    Ring<F> R;
+    Team T{(int)blockIdx.x, (int)gridDim.x, A.barrier, 0u};
+    Ring R;
     ring_init(R, A.K, A.stages);
     const size_t nh = (size_t)(A.K > 1 ? A.K - 1 : 0) * A.sd.D;
     for (size_t k = threadIdx.x; k < nh; k += kThreads)
         ((unsigned long long *)(g_smem + halo_offset(A.K)))[k] = kSentinel;
     __syncthreads();
-    pcg_job<F, kThreads>(A, T, R, sm);
+    pcg_job<kThreads>(A, T, R, sm);
 }
 
-// ------------------------------------------------------------ batched solves
-// Many independent scenes in one cooperative launch.  The grid is cut into
-// teams; a team of g blocks solves scenes of up to g*K strips.  Teams of one
-// size form a class and take that class's scenes from a shared queue (largest
-// estimated work first), so a team that finishes early takes the next scene.
-struct BatchTeams {
-    const int2 *block_team;   // per block: {team, rank in team}
-    const int2 *team;         // per team: {blocks, class}
-    const int2 *class_range;  // per class: {offset, count} into class_jobs
-    const int *class_jobs;    // job indices, each class in queue order
-    int *class_next;          // queue heads (zero at launch)
-    int *team_job;            // job taken by each team
-    unsigned *team_bar;       // two barrier words per team (zero at launch)
-    unsigned *all;            // launch-wide status word
-    const int4 *ctl;          // per job: {pinned pressure, pinned heat, limit pressure, limit heat}
-    // Placement of teams across SMs: the hardware puts consecutive blocks of a
-    // launch on the same few SMs, so a team of consecutive block indices would
-    // share those SMs' pipes.  Each block instead takes the slot
-    // (its rank on its SM) x nsm + (its SM's dense index), and teams are built
-    // from consecutive slots, i.e. from blocks on different SMs.
-    const short *sm_dense;    // %smid -> dense SM index (-1: unknown); 1024 entries
-    int *sm_fill;             // blocks placed per SM (zero at launch)
-    unsigned *grid_bar;       // two barrier words over the whole grid (zero at launch)
-    unsigned *remap_fail;     // set when a block could not be placed (zero at launch)
-    int nsm, per, remap;
-    long long wait_limit;     // polls of one halo or barrier wait
-};
-
-// At most 128 registers per thread whatever the block size.
-template <typename F, int kThreads>
+// Many independent scenes in one cooperative launch (see BatchTeams).  At most
+// 128 registers per thread whatever the block size.
+template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 512 / kThreads)
-    pcg_batch_kernel(const PcgArgs<F> *jobs, BatchTeams B, int mode, int heat, int pinned, int K, int stages) {
+    pcg_batch_kernel(const PcgArgs<double> *jobs, BatchTeams B, int mode, int heat, int pinned, int K, int stages) {
     __shared__ double sm[kMaxWarps + 1];
-    __shared__ PcgArgs<F> sA;
+    __shared__ PcgArgs<double> sA;
     __shared__ int s_slot;
-    const Flags launch_fl{B.all, B.all, B.wait_limit};
-    if (threadIdx.x == 0) {
-        int slot = (int)blockIdx.x;
-        if (B.remap) {
-            unsigned smid;
-            asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-            const int d = smid < 1024u ? B.sm_dense[smid] : -1;
-            const int k = d >= 0 ? atomicAdd(B.sm_fill + d, 1) : B.per;
-            if (d >= 0 && k < B.per) slot = k * B.nsm + d;
-            else atomicOr(B.remap_fail, 1u);
-        }
-        s_slot = slot;
-    }
-    if (B.remap) {
-        // every block learns whether all of them were placed, then all follow the same rule
-        const Team G{(int)blockIdx.x, (int)gridDim.x, B.grid_bar, nullptr};
-        team_barrier(G, launch_fl);
-        if (threadIdx.x == 0 && ld_volatile(B.remap_fail)) s_slot = (int)blockIdx.x;
-    }
-    __syncthreads();
-    const int2 bt = B.block_team[s_slot];
+    const int2 bt = batch_slot(B, &s_slot);
     const int2 tm = B.team[bt.x];
-    Team T{bt.y, tm.x, B.team_bar + 2 * bt.x, nullptr};
-    Ring<F> R;
+    Team T{bt.y, tm.x, B.team_bar + kBarStride * bt.x, 0u};
+    Ring R;
     ring_init(R, K, stages);
     __syncthreads();
-    for (;;) {
-        if (T.rank == 0 && threadIdx.x == 0) {
-            const int2 cr = B.class_range[tm.y];
-            const int k = atomicAdd(B.class_next + tm.y, 1);
-            *(volatile int *)(B.team_job + bt.x) = k < cr.y ? B.class_jobs[cr.x + k] : -1;
-        }
-        team_barrier(T, launch_fl);
-        const int j = *(volatile int *)(B.team_job + bt.x);
-        if (j < 0) break;
-        for (int k = threadIdx.x; k < (int)(sizeof(PcgArgs<F>) / 4); k += kThreads)
-            ((unsigned *)&sA)[k] = ((const unsigned *)(jobs + j))[k];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const int4 c = B.ctl[j];
-            sA.mode = mode;
-            sA.limit = heat ? c.w : c.z;
-            sA.pinned = pinned >= -1 ? pinned : (heat ? c.y : c.x);
-            sA.K = K;
-            sA.stages = stages;
-            sA.fl.all = B.all;
-            sA.fl.limit = B.wait_limit;
-        }
+    while (batch_take<double>(B, T, bt.x, tm.y, jobs, sA, mode, heat, pinned, K, stages)) {
         // halo rows start at the sentinel: the shared rows of this block
         // (their length changes with the scene) and the scene's global rows
         const size_t nh = (size_t)(K > 1 ? K - 1 : 0) * sA.sd.D;
         for (size_t k = threadIdx.x; k < nh; k += kThreads)
             ((unsigned long long *)(g_smem + halo_offset(K)))[k] = kSentinel;
-        const size_t ng = 2 * (size_t)sA.sd.S * sA.sd.D;
+        const size_t ng = pcg_halo_words(sA.sd);
         for (size_t k = (size_t)T.rank * kThreads + threadIdx.x; k < ng; k += (size_t)T.size * kThreads)
             sA.halo[k] = kSentinel;
-        T.partials = sA.partials;
         team_barrier(T, sA.fl);
-        pcg_job<F, kThreads>(sA, T, R, sm);
+        pcg_job<kThreads>(sA, T, R, sm);
     }
 }
 
 // Strips per block: the rings of the sweeping warps and the halo rows between
 // them must fit in shared memory.
+constexpr int kStrips = 2, kStages = 3;
+size_t pcg64_smem(int K, int D, int stages) { return ring_offset(K, D) + (size_t)K * stages * Ring::kStageBytes; }
 template <typename F>
-int strips_per_block() {
-    return sizeof(F) == 8 ? 2 : 4;
-}
-constexpr int kStages = 3;
-template <typename F>
-size_t smem_bytes(int K, int D, int stages = kStages) {
-    return ring_offset(K, D) + (size_t)K * stages * Ring<F>::kStageBytes;
+size_t smem_bytes(int K, int D, int stages) {
+    return sizeof(F) == 8 ? pcg64_smem(K, D, stages) : pcg32_smem(K, D, stages);
 }
 
-template <typename F, int kThreads>
+template <int kThreads>
 int max_coresident(size_t smem) {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(pcg_kernel<F, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pcg_kernel<F, kThreads>, kThreads, smem);
+    cudaFuncSetAttribute(pcg_kernel<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, pcg_kernel<kThreads>, kThreads, smem);
     return sms * (per > 2 ? 2 : per);
 }
 
@@ -1401,14 +1017,18 @@ __global__ void matrix_to_f32_kernel(const double *a, const double *b, const dou
 }
 }  // namespace
 
-template <typename F>
-cudaError_t launch_pcg_with(PcgArgs<F> A, const SDIdx &sd, const PcgScratch &X, const PcgConfig &cfg,
-                            cudaStream_t st, int *blocks_used);
+static cudaError_t launch_pcg64(PcgArgs<double> A, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
+                                int *blocks_used);
 
-template <typename F>
-cudaError_t launch_pcg(const Scene<F> &S, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
-                       int *blocks_used) {
-    return launch_pcg_with<F>(make_args(S, X, cfg.heat), S.sd, X, cfg, st, blocks_used);
+template <>
+cudaError_t launch_pcg<double>(const Scene<double> &S, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
+                               int *blocks_used) {
+    return launch_pcg64(make_args(S, X, cfg.heat), X, cfg, st, blocks_used);
+}
+template <>
+cudaError_t launch_pcg<float>(const Scene<float> &S, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
+                              int *blocks_used) {
+    return launch_pcg32(make_args(S, X, cfg.heat), X, cfg, st, blocks_used);
 }
 
 cudaError_t launch_pcg_f32(const Scene<double> &S, const PcgF32 &M, const PcgScratch &X, const PcgConfig &cfg,
@@ -1418,23 +1038,22 @@ cudaError_t launch_pcg_f32(const Scene<double> &S, const PcgF32 &M, const PcgScr
         matrix_to_f32_kernel<<<(int)std::min<size_t>((n + 255) / 256, 152 * 8), 256, 0, st>>>(
             S.adiag, S.ax, S.ay, M.adiag, M.ax, M.ay, n);
     }
-    return launch_pcg_with<float>(make_args_f32(S, M, X, cfg.heat), S.sd, X, cfg, st, blocks_used);
+    return launch_pcg32(make_args_f32(S, M, X, cfg.heat), X, cfg, st, blocks_used);
 }
 
-template <typename F>
-cudaError_t launch_pcg_with(PcgArgs<F> A, const SDIdx &sd, const PcgScratch &X, const PcgConfig &cfg,
-                            cudaStream_t st, int *blocks_used) {
+static cudaError_t launch_pcg64(PcgArgs<double> A, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
+                                int *blocks_used) {
+    const SDIdx &sd = A.sd;
     A.mode = cfg.mode;
     A.limit = cfg.limit;
     A.pinned = cfg.pinned;
-    A.K = strips_per_block<F>();
-    if (A.K > sd.S) A.K = sd.S;
+    A.K = std::min(kStrips, sd.S);
     A.stages = kStages;
     A.fl.limit = cfg.wait_limit > 0 ? cfg.wait_limit : kWaitLimit;
-    const size_t smem = smem_bytes<F>(A.K, sd.D);
+    const size_t smem = pcg64_smem(A.K, sd.D, A.stages);
     const int threads = 512;
-    const void *fn = (const void *)pcg_kernel<F, 512>;
-    int maxb = max_coresident<F, 512>(smem);
+    const void *fn = (const void *)pcg_kernel<512>;
+    int maxb = max_coresident<512>(smem);
     if (maxb > X.max_blocks) maxb = X.max_blocks;
     const int need = (sd.S + A.K - 1) / A.K;  // blocks that own strips
     if (maxb < need) return cudaErrorInvalidConfiguration;
@@ -1445,7 +1064,7 @@ cudaError_t launch_pcg_with(PcgArgs<F> A, const SDIdx &sd, const PcgScratch &X, 
     if (want < need) want = need;
     int G = want < maxb ? want : maxb;
     if (blocks_used) *blocks_used = G;
-    cudaError_t e = cudaMemsetAsync(X.barrier, 0, 2 * sizeof(unsigned), st);
+    cudaError_t e = cudaMemsetAsync(X.barrier, 0, sizeof(unsigned), st);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(X.halo, 0xff, 2 * (size_t)sd.S * sd.D * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -1459,6 +1078,7 @@ struct PcgBatchPlan {
     int n = 0;
     PcgShape shape{};
     int grid = 0;      // co-resident blocks of the launch
+    int block = 0, K = 0, stages = 0;  // threads, strips and ring stages of a block
     int max_team = 128;  // largest team the planner may form
     size_t smem = 0;
     std::vector<int> strips, diags, cells;
@@ -1490,9 +1110,10 @@ size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 
 template <typename F>
 const void *batch_fn(int threads) {
-    if (threads == 32) return (const void *)pcg_batch_kernel<F, 32>;
-    if (threads == 64) return (const void *)pcg_batch_kernel<F, 64>;
-    return threads == 128 ? (const void *)pcg_batch_kernel<F, 128> : (const void *)pcg_batch_kernel<F, 256>;
+    if (sizeof(F) == 4) return pcg32_batch_fn();
+    if (threads == 32) return (const void *)pcg_batch_kernel<32>;
+    if (threads == 64) return (const void *)pcg_batch_kernel<64>;
+    return threads == 128 ? (const void *)pcg_batch_kernel<128> : (const void *)pcg_batch_kernel<256>;
 }
 }  // namespace
 
@@ -1510,11 +1131,13 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
         return fail("unsupported batched PCG shape");
     int dmax = 0;
     for (int i = 0; i < n; i++) dmax = std::max(dmax, scenes[i]->sd.D);
-    const size_t smem = smem_bytes<F>(shape.K, dmax, shape.stages);
     const void *fn = batch_fn<F>(shape.threads);
     int dev = 0, sms = 0, per = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    int block = shape.threads, K = shape.K, stages = shape.stages;
+    if (sizeof(F) == 4) pcg32_shape(shape.threads, dmax, optin - sizeof(PcgArgs<F>) - 2048, &block, &K, &stages);
+    const size_t smem = smem_bytes<F>(K, dmax, stages);
     // the attribute stays at the device maximum, so a launch (or a graph
     // replay) of any plan is valid whatever plan was created last
     if (smem + sizeof(PcgArgs<F>) + 1024 > (size_t)optin ||
@@ -1523,7 +1146,7 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
         return fail("shared memory per block exceeds the device limit");
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, shape.threads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, block, smem);
     const int grid = sms * per;
     if (grid < 1) return fail("too few co-resident blocks for the batched PCG shape");
 
@@ -1532,6 +1155,9 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
     P->n = n;
     P->shape = shape;
     P->grid = grid;
+    P->block = block;
+    P->K = K;
+    P->stages = stages;
     P->smem = smem;
     for (int i = 0; i < n; i++) {
         P->strips.push_back(scenes[i]->sd.S);
@@ -1561,13 +1187,13 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
     const size_t o_cn = off;
     off += (kMaxClasses + 1) * sizeof(int);
     const size_t o_tb = off;
-    off += 2 * grid * sizeof(unsigned);
+    off += kBarStride * grid * sizeof(unsigned);
     const size_t o_all = off;
     off += sizeof(unsigned);
     const size_t o_fill = off;
     off += sms * sizeof(int);
     const size_t o_gbar = off;
-    off += 2 * sizeof(unsigned);
+    off += sizeof(unsigned);
     const size_t o_rfail = off;
     off += sizeof(unsigned);
     P->zero_bytes = off - P->zero_off;
@@ -1814,9 +1440,9 @@ cudaError_t launch_pcg_batch(PcgBatchPlan *P, const PcgConfig &cfg, cudaStream_t
     const PcgArgs<F> *jobs = (const PcgArgs<F> *)P->jobs[cfg.heat ? 1 : 0];
     BatchTeams B = P->B;
     B.wait_limit = cfg.wait_limit > 0 ? cfg.wait_limit : kWaitLimit;
-    int mode = cfg.mode, heat = cfg.heat, pinned = cfg.pinned, K = P->shape.K, stages = P->shape.stages;
+    int mode = cfg.mode, heat = cfg.heat, pinned = cfg.pinned, K = P->K, stages = P->stages;
     void *args[] = {&jobs, &B, &mode, &heat, &pinned, &K, &stages};
-    return cudaLaunchCooperativeKernel(batch_fn<F>(P->shape.threads), dim3(P->grid), dim3(P->shape.threads), args,
+    return cudaLaunchCooperativeKernel(batch_fn<F>(P->shape.threads), dim3(P->grid), dim3(P->block), args,
                                        P->smem, st);
 }
 
@@ -1827,10 +1453,6 @@ template PcgBatchPlan *pcg_batch_create<float>(const Scene<float> *const *, cons
 template cudaError_t launch_pcg_batch<double>(PcgBatchPlan *, const PcgConfig &, cudaStream_t);
 template cudaError_t launch_pcg_batch<float>(PcgBatchPlan *, const PcgConfig &, cudaStream_t);
 
-template cudaError_t launch_pcg<double>(const Scene<double> &, const PcgScratch &, const PcgConfig &,
-                                        cudaStream_t, int *);
-template cudaError_t launch_pcg<float>(const Scene<float> &, const PcgScratch &, const PcgConfig &,
-                                       cudaStream_t, int *);
 template int pcg_max_blocks<double>();
 template int pcg_max_blocks<float>();
 

@@ -92,7 +92,7 @@ extern "C" int ifl_pcg_solve_noalloc(int w, int h, const double *adiag, const do
     using namespace ifl;
     if (w < 2 || h < 2 || max_iter < 0 || !adiag || !aplusx || !aplusy || !rhs || !p || !stats)
         return IFL_ERR_ARG;
-    const SDIdx sd = SDIdx::make(w, h);
+    const SDIdx sd = SDIdx::make(w, h, 0);
     if ((size_t)sd.S * sd.D > kMaxStripDiagonals) return IFL_ERR_UNSUPPORTED;  // beyond the scratch size
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return IFL_ERR_CUDA;
@@ -123,7 +123,7 @@ extern "C" int ifl_pcg_solve_noalloc(int w, int h, const double *adiag, const do
     S.flags = take<unsigned>(cur, 8);
     PcgScratch X{};
     X.halo = take<unsigned long long>(cur, 2 * (size_t)sd.S * sd.D);
-    X.partials = take<double>(cur, 4 * pcg_chunks(sd));
+    X.partials = take<double>(cur, pcg_partials(sd));
     X.barrier = take<unsigned>(cur, 2);
     X.iter_total = take<unsigned long long>(cur, 1);
     X.out = (PcgOut *)stats;  // the solve writes its outcome straight into the caller's struct

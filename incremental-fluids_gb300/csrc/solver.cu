@@ -458,7 +458,10 @@ class SolverImpl final : public SolverBase {
     void carve(char *base, Carver &c) {
         const size_t N = (size_t)P_ * rows_;
         const bool geo = prm_.variant >= IFL_SOLID;
-        S_.sd = SDIdx::make(prm_.w, prm_.h);
+        // FP32-form PCG solves work on 2 x 4 tiles (k_pcg32.cu)
+        f32_solves_ = prm_.variant == IFL_FLIP && prm_.precision == IFL_FP32;
+        const bool tiled = f32_solves_ || (sizeof(F) == 4 && prm_.variant > IFL_GS);
+        S_.sd = SDIdx::make(prm_.w, prm_.h, tiled ? 1 : 0);
         const size_t NS = S_.sd.total();
         S_.variant = prm_.variant;
         S_.w = prm_.w;
@@ -506,7 +509,7 @@ class SolverImpl final : public SolverBase {
         S_.adiag = c.take<F>(base, NS);
         S_.ax = c.take<F>(base, NS);
         S_.ay = c.take<F>(base, NS);
-        S_.mic = c.take<F>(base, 4 * NS);
+        S_.mic = c.take<F>(base, (sizeof(F) == 4 ? 5 : 4) * NS);
         S_.pc = c.take<double>(base, NS);
         S_.nb = c.take<uint8_t>(base, NS);
         if (prm_.variant >= IFL_VARDENS) {
@@ -520,12 +523,11 @@ class SolverImpl final : public SolverBase {
         S_.nbodies = 0;
         S_.flags = c.take<unsigned>(base, 8);
         M_ = PcgF32{};
-        f32_solves_ = prm_.variant == IFL_FLIP && prm_.precision == IFL_FP32;
         if (f32_solves_) {  // FP32-form solves beside the FP64 fields and particles
             M_.adiag = c.take<float>(base, NS);
             M_.ax = c.take<float>(base, NS);
             M_.ay = c.take<float>(base, NS);
-            M_.mic = c.take<float>(base, 4 * NS);
+            M_.mic = c.take<float>(base, 5 * NS);
             M_.rf = c.take<float>(base, NS);
             M_.z = c.take<float>(base, NS);
             M_.sa = c.take<float>(base, NS);
@@ -555,9 +557,9 @@ class SolverImpl final : public SolverBase {
             X_.ctl = c.take<int>(base, FC_WORDS);
         }
         scratch_.max_blocks = max_blocks_;
-        scratch_.partials = c.take<double>(base, 4 * pcg_chunks(S_.sd));
+        scratch_.partials = c.take<double>(base, pcg_partials(S_.sd));
         scratch_.barrier = c.take<unsigned>(base, 2);
-        scratch_.halo = c.take<unsigned long long>(base, 2 * (size_t)S_.sd.S * S_.sd.D);
+        scratch_.halo = c.take<unsigned long long>(base, pcg_halo_words(S_.sd));
         scratch_.out = c.take<PcgOut>(base, 2);
         scratch_.iter_total = c.take<unsigned long long>(base, 1);
     }
