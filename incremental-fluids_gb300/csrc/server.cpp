@@ -109,6 +109,8 @@ class Server {
                     err_ = batch_->error();
                     return e;
                 }
+                // now: members that leave with this step take the batch with them
+                pin_shape();
                 if (fresh) {
                     // a new membership: building the batch, plus what its first
                     // step spends beyond a steady step (plan, graph capture)
@@ -268,7 +270,6 @@ class Server {
         return IFL_OK;
     }
 
-  public:
     // After the first step of an autotuned batch: keep its shape for later batches.
     void pin_shape() {
         if (!tune_pending_ || !batch_) return;
@@ -287,7 +288,6 @@ class Server {
         }
     }
 
-  private:
     ifl_server_params p_;
     ifl_batch_options opt_;
     std::chrono::steady_clock::time_point t0_;
@@ -310,9 +310,7 @@ void server_destroy(Server *s) { delete s; }
 double server_now(const Server *s) { return s->now(); }
 int server_submit(Server *s, const ifl_request &r, int64_t *id) { return s->submit(r, id); }
 int server_step(Server *s, int *a, int *q) {
-    int e = s->step(a, q);
-    if (e == IFL_OK) s->pin_shape();
-    return e;
+    return s->step(a, q);
 }
 int server_completions(Server *s, ifl_completion *o, int cap, int *n) { return s->completions(o, cap, n); }
 int server_read_field(Server *s, int64_t id, int field, void *host, size_t bytes, int dtype) {
