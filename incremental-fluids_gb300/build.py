@@ -22,8 +22,8 @@ OUT_DIR = os.path.join(PKG, "ifluids")
 BUILD_DIR = os.path.join(PKG, "_build")
 LIB = os.path.join(OUT_DIR, "libifluids.so")
 
-SOURCES = ["k_fields.cu", "k_pcg.cu", "k_pcg32.cu", "k_flip.cu", "k_gs.cu", "solver.cu", "batch.cu", "noalloc.cu", "server.cpp", "capi.cpp"]
-HEADERS = ["ifl_internal.h", "ifl_device.cuh", "pcg_common.cuh", "solver.h"]
+SOURCES = ["k_fields.cu", "k_pcg.cu", "k_pcg32.cu", "k_pcg64.cu", "k_flip.cu", "k_gs.cu", "solver.cu", "batch.cu", "noalloc.cu", "server.cpp", "capi.cpp"]
+HEADERS = ["ifl_internal.h", "ifl_device.cuh", "pcg_common.cuh", "pcg_ring.cuh", "pcg_job.cuh", "solver.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-O2,-ffp-contract=off",
          "-I" + os.path.join(PKG, "..", "include")]

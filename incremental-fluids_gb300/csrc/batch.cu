@@ -53,7 +53,7 @@ template <typename F>
 std::vector<PcgShape> candidate_shapes() {
     if (sizeof(F) == 4)
         return {{128, 1, 4}, {128, 1, 3}, {64, 1, 3}, {64, 1, 4}, {256, 1, 4}, {256, 2, 3}, {128, 2, 2}};
-    return {{128, 1, 2}, {256, 2, 3}, {128, 2, 2}, {64, 1, 3}, {64, 1, 2}, {32, 1, 2}, {32, 1, 3}};
+    return {{128, 1, 4}, {128, 1, 3}, {64, 1, 4}, {256, 1, 4}, {256, 2, 4}, {128, 2, 3}};
 }
 
 template <typename F>
@@ -380,14 +380,13 @@ class BatchImpl final : public BatchBase {
     // 512-scene step by less than its step-to-step spread.
     double plan_cost(int i, int g) const {
         constexpr bool f32 = sizeof(F) == 4;
-        constexpr double kTau = f32 ? 0.085 : 0.33, kLag = f32 ? 6.5 : 6.4, kElemNs = f32 ? 6.0 : 24.0;
+        constexpr double kTau = f32 ? 0.085 : 0.075, kLag = f32 ? 6.5 : 4.1, kElemNs = f32 ? 6.0 : 8.0;
         const Scene<F> &S = scene(i);
         const int P = g * shape_.K, Sn = S.sd.S;
         const double Dt = S.sd.D * kTau;
         const double sweep = std::max((Sn - 1) * kLag + Dt, ((Sn - 1) / P) * Dt + ((Sn - 1) % P) * kLag + Dt);
-        const double elem = 1e-3 * kElemNs * (double)S.w * S.h / g * ((f32 ? 128.0 : 64.0) / shape_.threads);
-        const double bars = f32 ? (g == 1 ? 6.0 : 12.0) : g == 1 ? 1.6 : 12.0 + 4.8 * std::log2((double)g);
-        return iters_[i] * (2.0 * sweep + elem + bars);
+        const double elem = 1e-3 * kElemNs * (double)S.w * S.h / g * (128.0 / shape_.threads);
+        return iters_[i] * (2.0 * sweep + elem + (g == 1 ? 6.0 : 12.0));
     }
 
     int schedule() {

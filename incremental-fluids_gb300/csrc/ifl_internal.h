@@ -106,7 +106,7 @@ struct Scene {
     F *rf;             // r in storage precision for the substitutions (aliases r for FP64)
     F *z, *sa, *sb;
     F *adiag, *ax, *ay;
-    F *mic;            // MIC(0) apply operands: FP64 {lx, ly, pc, neighbour bits} per slot, FP32 form five arrays (k_pcg32.cu)
+    F *mic;            // MIC(0) apply operands, five values per slot (pcg_ring.cuh)
     double *pc;        // MIC(0) factor, FP64
     uint8_t *nb;
     F *udens, *vdens;
@@ -122,15 +122,16 @@ struct PcgOut {
 };
 
 // Diagonals per reduction chunk of the PCG's elementwise phases, a function of
-// the scene alone (its sums must not depend on the launch).  Tiles: one diagonal
-// while the chunks are not many more than a GPU's warps, so that a small scene
-// reaches many SM quarters (an FP64 instruction occupies a quarter for 64-76
-// cycles).
-constexpr int kPcgChunk = 16;
+// the scene alone (its sums must not depend on the launch).  One diagonal while
+// the chunks are not many more than a GPU's warps, so that a small scene reaches
+// many SM quarters (an FP64 instruction occupies a quarter for 64-76 cycles).  A
+// chunk lies inside a strip: it divides the sweeps' block.
 __host__ __device__ inline int pcg_chunk_diags(const SDIdx &sd) {
-    if (!sd.ts) return kPcgChunk;
     const size_t n = (size_t)sd.S * sd.D;
-    return n <= 4096 ? 1 : n <= 8192 ? 2 : 4;
+    const int most = sd.ts ? kTileBlock : kSweepBlock;
+    int c = 1;
+    while (c < most && n > (size_t)4096 * c) c *= 2;
+    return c;
 }
 __host__ __device__ inline size_t pcg_chunks(const SDIdx &sd) {
     const int c = pcg_chunk_diags(sd);
@@ -139,13 +140,13 @@ __host__ __device__ inline size_t pcg_chunks(const SDIdx &sd) {
 // Partial sums of a solve: maximum and dot product per chunk, sigma per strip
 // (or chunk).
 __host__ __device__ inline size_t pcg_partials(const SDIdx &sd) { return 4 * pcg_chunks(sd) + 4 * (size_t)sd.S; }
-// Halo words of a solve: two rows per strip, of D words (tiles: D + kHaloPad,
-// and at least the columns + 1 words of the rows that the factor hands over
-// between its 32-row sub-strips, two per 64 rows).
+// Halo words of a solve: two rows per strip, of D + kHaloPad words, and at least
+// the W words of each row that the factor hands over between 32-row sub-strips
+// (four per tile strip).
 constexpr int kHaloPad = 8;
-__host__ __device__ inline size_t pcg_halo_row(const SDIdx &sd) { return sd.ts ? (size_t)sd.D + kHaloPad : (size_t)sd.D; }
+__host__ __device__ inline size_t pcg_halo_row(const SDIdx &sd) { return (size_t)sd.D + kHaloPad; }
 __host__ __device__ inline size_t pcg_halo_words(const SDIdx &sd) {
-    const size_t sweeps = 2 * (size_t)sd.S * pcg_halo_row(sd), factor = sd.ts ? 4 * (size_t)sd.S * sd.W : 0;
+    const size_t sweeps = 2 * (size_t)sd.S * pcg_halo_row(sd), factor = (sd.ts ? 4 : 1) * (size_t)sd.S * sd.W;
     return factor > sweeps ? factor : sweeps;
 }
 

@@ -41,52 +41,15 @@
 //
 // r and p are FP64; the matvec is FP32 (its results are stored as they are
 // formed), dot products, the maximum norm, alpha and beta are FP64.
-#include <algorithm>
-#include <cstring>
-#include <type_traits>
-
-#include "pcg_common.cuh"
+#include "pcg_ring.cuh"
 
 namespace ifl {
 
 namespace {
 
-constexpr int kT = kTileBlock;                    // tile diagonals per block of a ring
+constexpr int kT = Lay<float>::kSteps;            // tile diagonals per block of a ring
+constexpr unsigned kVec = kVecBytes<float>;
 constexpr int kDepth = 2;                         // steps whose operands are in registers (divides kT)
-constexpr unsigned kVecBytes = kT * 1024u;        // a block of one array
-constexpr unsigned kHaloAt = 4u * kVecBytes;      // halo words of a block behind the operands of the backward sweep
-constexpr unsigned kStageBytes = kHaloAt + 128u;  // a ring stage
-constexpr int kMaxStages = 8;
-constexpr int kRoles = 3;                         // warps that work on one strip: sweep, load, prepare
-constexpr int kSums = 16;                         // partial sums of a reduction (see total32)
-
-// ---------------------------------------------------------- conversions
-// float <-> double on the integer pipe.  A conversion instruction takes an FP64
-// slot (19 cycles per warp and SM on this part), these take about eight integer
-// instructions (2 cycles).  Zeros and normal numbers here; subnormals,
-// infinities and NaN take the instruction.
-__device__ __forceinline__ double to_f64(float f) {
-    const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
-    unsigned hi = (t >> 3) + 0x38000000u, lo = u << 29;
-    if (t - 0x00800000u >= 0x7f000000u) {  // zero, subnormal, infinity, NaN
-        if (t != 0u) return (double)f;
-        hi = 0u;
-        lo = 0u;
-    }
-    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
-}
-// Round to nearest even, as the instruction.
-__device__ __forceinline__ float to_f32(double d) {
-    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), t = hi & 0x7fffffffu;
-    if (t - 0x38100000u >= 0x0fe00000u) {  // outside [2^-126, 2^128): zero, subnormal result, overflow, NaN
-        if ((t | lo) != 0u) return (float)d;
-        return __uint_as_float(hi & 0x80000000u);
-    }
-    unsigned m = ((t - 0x38000000u) << 3) | (lo >> 29);
-    const unsigned rest = lo & 0x1fffffffu;
-    m += (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
-    return __uint_as_float(m | (hi & 0x80000000u));
-}
 
 // Float-float numbers (hi + lo, |lo| <= ulp(hi)/2): an exact product of two
 // floats and a sum with an error-free two-sum of the high parts (Knuth's
@@ -122,191 +85,29 @@ __device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
     return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
 }
 
-// The MIC(0) coefficients lie as the sweeps read them, a tile diagonal's arrays
-// side by side, one base address for all: -al and -bd for the forward sweep (512
-// floats per tile diagonal), then, behind them all, dd, -a and -b for the
-// backward sweep (768 floats).  k: the cell's slot.
-enum { C_AL = 0, C_BD = 1, C_DD = 0, C_A = 1, C_B = 2 };
-__device__ __forceinline__ float *fwd_coef(const PcgArgs<float> &A, size_t k, int arr) {
-    return A.mic + (k >> 8) * 512 + arr * 256 + (k & 255);
-}
-__device__ __forceinline__ float *bwd_coef(const PcgArgs<float> &A, size_t k, int arr) {
-    return A.mic + 2 * A.sd.total() + (k >> 8) * 768 + arr * 256 + (k & 255);
-}
-
-// --------------------------------------------------------------- sweeps
-// A strip's ring in shared memory: `stages` buffers of kT tile diagonals,
-//   [r][al, bd per diagonal] (forward) or [y][dd, a, b per diagonal] (backward),
-//   then the kT halo words of the block.
-// Three warps share it, each with its own running position (stage, mbarrier
-// parity):
-//  * the loader waits for a free stage, starts two bulk copies into it, takes the
-//    block's halo words as they arrive and puts them behind the operands;
-//  * the preparer (backward) waits for the copies, multiplies y by dd in place and
-//    adds up sigma;
-//  * the sweeping warp waits for both (`ready`), stores its results and hands its
-//    boundary row on, and frees the stage.
-// Every wait is bounded.  A timeout elsewhere in the launch does not shorten the
-// mbarrier waits: the copies were issued from this GPU's memory and complete,
-// and the loader's halo polls give up by themselves, so a timed-out sweep still
-// consumes every block it issued and no bulk copy is left behind in shared memory.
-// A ring is `dead` once an mbarrier wait ran out all the same: its warp then
-// waits and issues no more.
-struct Ring32 {
-    unsigned buf;   // byte offset of the stages in g_smem
-    unsigned bars;  // byte offset of the mbarriers, kMaxStages of each kind
-    int stages, st;
-    unsigned parity;
-    bool dead;
-    enum { COPIED = 0, READY = 1, FREE = 2, KINDS = 3 };
-    __device__ __forceinline__ uint64_t *bar(int kind, int at) const {
-        return (uint64_t *)(g_smem + bars) + kind * kMaxStages + at;
-    }
-    __device__ __forceinline__ unsigned stage(int at) const { return buf + (unsigned)at * kStageBytes; }
-    __device__ __forceinline__ void next() {
-        st = st + 1 == stages ? 0 : st + 1;
-        parity ^= st == 0 ? 1u : 0u;
-    }
-    __device__ __forceinline__ void skip(int n) {  // n blocks that this warp has no part in
-        const int at = st + n;
-        st = at % stages;
-        parity ^= (unsigned)(at / stages) & 1u;
-    }
-};
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Whether a phase is complete, without waiting for it (try_wait suspends).
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok)
-                 : "r"(smem_u32(bar)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// Whole warp: the phase `parity` of a barrier.
-__device__ __forceinline__ void ring32_wait(Ring32 &R, uint64_t *bar, unsigned parity, const Flags &flags) {
-    if (__all_sync(FULL, R.dead || mbar_try_wait(bar, parity))) return;
-    long long n = 0;
-    while (!__all_sync(FULL, mbar_try_wait(bar, parity))) {
-        if (++n > kMbarWaitLimit + flags.limit) {
-            set_timeout(flags);
-            R.dead = true;
-            break;
-        }
-    }
-}
-
-// The loader's part of one strip.  Halo words: at step t the waiting lane needs
-// the boundary values of one tile column, two floats in one 8-byte word, at
-// in_word(t) of the neighbour's row (t <= D - 32; beyond, the coefficient is
-// zero).  Lane i polls the word of the i-th step from the first block that waits
-// for words, so one round of loads (about 700 cycles) serves up to eight blocks.
-template <bool BWD, bool IN>
-__device__ __noinline__ void load32_strip(const PcgArgs<float> &A, int s, Ring32 &ring, const Chan in) {
-    constexpr int kC = BWD ? 3 : 2;  // coefficient arrays
-    Ring32 R = ring;
-    const Flags flags = A.fl;
-    const int lane = threadIdx.x & 31;
-    const int D = A.sd.D, nblk = D / kT;
-    const size_t row0 = (size_t)s * D + (BWD ? D - kT : 0);  // first tile diagonal of the first block
-    const float *vec = (BWD ? A.z : A.rf) + row0 * 256;
-    const float *cf = BWD ? bwd_coef(A, row0 * 256, C_DD) : fwd_coef(A, row0 * 256, C_AL);
-    fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
-    int issued = 0, ready = 0;   // blocks whose copies are started, whose halo words are in place
-    int rst = R.st;              // stage of block `ready`
-    unsigned long long w = kSentinel;
-    bool given_up = false;
-    long long polls = 0;
-    while (ready < nblk) {
-        // start copies into free stages; wait for one only when there is nothing else to do
-        while (issued < nblk && issued < ready + R.stages) {
-            uint64_t *fr = R.bar(Ring32::FREE, R.st);
-            if (!__all_sync(FULL, R.dead || mbar_test(fr, R.parity ^ 1u))) {
-                if (issued > ready) break;
-                ring32_wait(R, fr, R.parity ^ 1u, flags);
-            }
-            if (lane == 0) {
-                // forward, the sweeping warp itself waits for the copies; `copied` keeps pace
-                uint64_t *ready_bar = R.bar(Ring32::READY, R.st), *copied = R.bar(Ring32::COPIED, R.st);
-                uint64_t *tx = BWD ? copied : ready_bar;
-                char *dst = g_smem + R.stage(R.st);
-                mbar_expect_tx(tx, (1u + kC) * kVecBytes);
-                bulk_g2s(dst, vec, kVecBytes, tx);
-                bulk_g2s(dst + kVecBytes, cf, kC * kVecBytes, tx);
-                if (!BWD) mbar_arrive(copied);
-                if (!IN) mbar_arrive(ready_bar);
-            }
-            vec += BWD ? -kT * 256 : kT * 256;
-            cf += (BWD ? -kT * 256 : kT * 256) * kC;
-            R.next();
-            issued++;
-            if (!IN) ready++;
-        }
-        if constexpr (IN) {
-            const int t = ready * kT + lane;
-            const bool need = t <= D - 32;
-            unsigned long long *word = in.row + (BWD ? D - 32 - t : t + 32);
-            if (need && w == kSentinel && !given_up) {
-                asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(w) : "l"(word));
-                if (w != kSentinel) asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(word), "l"(kSentinel));
-            }
-            if (!need) w = 0ull;
-            const unsigned have = __ballot_sync(FULL, w != kSentinel || given_up);
-            // blocks from `ready` on whose words are all there
-            int k = min(__ffs(~have) - 1 < 0 ? 32 : __ffs(~have) - 1, (issued - ready) * kT) / kT;
-            if (k > 0) {
-                polls = 0;
-                const int q = lane / kT;
-                int st = rst + q;
-                st -= st >= R.stages ? R.stages : 0;
-                if (q < k)
-                    *(volatile unsigned long long *)(g_smem + R.stage(st) + kHaloAt + 8 * (lane % kT)) = given_up && w == kSentinel ? 0ull : w;
-                __syncwarp();
-                if (lane < k) {
-                    int at = rst + lane;
-                    at -= at >= R.stages ? R.stages : 0;
-                    mbar_arrive(R.bar(Ring32::READY, at));
-                }
-                w = __shfl_down_sync(FULL, w, k * kT);
-                if (lane >= 32 - k * kT) w = kSentinel;
-                ready += k;
-                rst += k;
-                rst -= rst >= R.stages ? R.stages : 0;
-            } else if (++polls > flags.limit || ((polls & 15) == 0 && __any_sync(FULL, timed_out(flags)))) {
-                if (!given_up) set_timeout(flags);
-                given_up = true;
-            }
-        }
-    }
-    ring = R;
-    __syncwarp();
-}
-
 // The preparer's part of one backward strip: y becomes dd y, and sigma = z.r =
-// sum of dd y^2 (see pcg32_job) is added up: sums of two fused FP32 products per
+// sum of dd y^2 (see pcg_job) is added up: sums of two fused FP32 products per
 // row of the tiles and step, over a block, then FP64.
-__device__ __noinline__ void prepare32_strip(const PcgArgs<float> &A, int s, Ring32 &ring) {
-    Ring32 R = ring;
+__device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<float> &ring) {
+    Ring<float> R = ring;
     const Flags flags = A.fl;
     const int lane = threadIdx.x & 31, nblk = A.sd.D / kT;
     double qq = 0.0;
     for (int blk = 0; blk < nblk; blk++) {
-        ring32_wait(R, R.bar(Ring32::COPIED, R.st), R.parity, flags);
+        ring_wait(R, R.bar(Ring<float>::COPIED, R.st), R.parity, flags);
         char *g = g_smem + R.stage(R.st) + lane * 16;
         float4 qs = zero4();
 #pragma unroll
         for (int j = kT - 1; j >= 0; j--) {
             float4 *y = (float4 *)(g + j * 1024);
-            const float4 *dd = (const float4 *)(g + kVecBytes + j * 3 * 1024);
+            const float4 *dd = (const float4 *)(g + kVec + j * 3 * 1024);
             const float4 y0 = y[0], y1 = y[32], q0 = mul4(dd[0], y0), q1 = mul4(dd[32], y1);
             y[0] = q0;
             y[32] = q1;
             qs = fma4(q1, y1, fma4(q0, y0, qs));
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(R.bar(Ring32::READY, R.st));
+        if (lane == 0) mbar_arrive(R.bar(Ring<float>::READY, R.st));
         qq += to_f64((qs.x + qs.y) + (qs.z + qs.w));
         R.next();
     }
@@ -326,11 +127,11 @@ __device__ __noinline__ void prepare32_strip(const PcgArgs<float> &A, int s, Rin
 // at X + 32 of the row (forward; the lane starts at X = -31) or at X (backward).
 // Words of columns that no step waits for are written along and never read.
 // Functions of their own: inlined, the solve's registers spill into their steps.
-template <bool BWD, bool IN>
-__device__ __noinline__ void sweep32_strip(const PcgArgs<float> &A, int s, Ring32 &ring, const Chan out) {
+template <bool REF, bool BWD, bool IN>
+__device__ __noinline__ void sweep_strip(const PcgArgs<float> &A, int s, Ring<float> &ring, const Chan out) {
     // the vector operand (r, or dd y) and two coefficient arrays behind it (backward: a and b, after dd)
     constexpr int kC = BWD ? 3 : 2, kSkip = BWD ? 1 : 0;
-    Ring32 R = ring;
+    Ring<float> R = ring;
     const Flags flags = A.fl;
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
@@ -343,7 +144,7 @@ __device__ __noinline__ void sweep32_strip(const PcgArgs<float> &A, int s, Ring3
     // operands of step j of the block into buffer j % kDepth
     auto load = [&](int j) {
         const int i = j % kDepth, jj = BWD ? kT - 1 - j : j;
-        const char *v = g + jj * 1024, *c = g + kVecBytes + (jj * kC + kSkip) * 1024;
+        const char *v = g + jj * 1024, *c = g + kVec + (jj * kC + kSkip) * 1024;
         o0[i][0] = *(const float4 *)v;
         o1[i][0] = *(const float4 *)(v + 512);
 #pragma unroll
@@ -355,13 +156,13 @@ __device__ __noinline__ void sweep32_strip(const PcgArgs<float> &A, int s, Ring3
     float4 n = zero4();        // the previous tile's column next to this one
     float g0 = 0.f, g1 = 0.f;  // boundary row of the previous lane (columns 0, 1)
     for (int blk = 0; blk < nblk; blk++) {
-        ring32_wait(R, R.bar(Ring32::READY, R.st), R.parity, flags);
+        ring_wait(R, R.bar(Ring<float>::READY, R.st), R.parity, flags);
         g = g_smem + R.stage(R.st) + lane * 16;
 #pragma unroll
         for (int j = 0; j < kDepth; j++) load(j);
         float2 halo[kT];  // all of the block's halo words at once: no step waits for its own
         if constexpr (IN) {
-            const float2 *h = (const float2 *)(g - lane * 16 + kHaloAt);
+            const float2 *h = (const float2 *)(g - lane * 16 + kHaloAt<float>);
 #pragma unroll
             for (int j = 0; j < kT; j++) halo[j] = h[j];
         }
@@ -409,190 +210,13 @@ __device__ __noinline__ void sweep32_strip(const PcgArgs<float> &A, int s, Ring3
             g1 = h1;
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(R.bar(Ring32::FREE, R.st));
+        if (lane == 0) mbar_arrive(R.bar(Ring<float>::FREE, R.st));
         R.next();
         zp += BWD ? -kT * 64 : kT * 64;
         op += BWD ? -kT : kT;
     }
     ring = R;
     __syncwarp();
-}
-
-// Shared-memory layout of a block: ring mbarriers (of each strip) | the halo rows
-// between its strips, K-1 upward and K-1 downward (apart, since each direction
-// leaves words behind that it never reads) | the rings.
-__host__ __device__ __forceinline__ unsigned halo32_offset(int K) { return 8u * Ring32::KINDS * kMaxStages * K; }
-__host__ __device__ __forceinline__ unsigned ring32_offset(int K, int D) {
-    const size_t nh = 2 * (size_t)(K > 1 ? K - 1 : 0) * (D + kHaloPad);
-    return (unsigned)(((halo32_offset(K) + nh * 8 + 127) / 128) * 128);
-}
-
-// Sweep of all strips of this block: warps 0..K-1 sweep, K..2K-1 load for them,
-// 2K..3K-1 prepare.  The team's T.size*K sweeping warps take
-// the strips round-robin: warp `base` sweeps strips base, base + P, base + 2P,
-// ... (P = T.size*K), in increasing order for the forward solve and in
-// decreasing order for the backward solve, so that every strip waits only on a
-// strip that is swept earlier by its own warp or by another warp in the same or
-// an earlier round (no cycle).  When every warp has a single strip, the halo
-// rows between the warps of one block live in shared memory; otherwise every
-// strip hands its boundary row over through its own global row (a shared row
-// would be reused by the next round while its reader may still need it).
-template <bool BWD>
-__device__ void sweep32(const PcgArgs<float> &A, const Team &T, Ring32 &R) {
-    const int role = (threadIdx.x >> 5) / A.K, w = (threadIdx.x >> 5) % A.K;
-    const SDIdx sd = A.sd;
-    int nstrips_blk = sd.S - T.rank * A.K;
-    nstrips_blk = nstrips_blk > A.K ? A.K : nstrips_blk;
-    if (role >= kRoles || w >= nstrips_blk) return;
-    const int P = T.size * A.K;
-    const int base = T.rank * A.K + w;
-    const size_t row = pcg_halo_row(sd);
-    unsigned long long *up = A.halo, *down = A.halo + (size_t)sd.S * row;
-    auto smem_row = [&](int k) {
-        const unsigned at = (unsigned)(((BWD ? A.K - 1 : 0) + k) * row);
-        return Chan{(unsigned long long *)(g_smem + halo32_offset(A.K) + 8u * at), true};
-    };
-    auto glob_row = [&](unsigned long long *r) { return Chan{r, true}; };
-    const bool one_round = sd.S <= P;
-    const int nmine = (sd.S - base + P - 1) / P;  // strips of this warp
-    for (int j0 = 0; j0 < nmine; j0++) {
-        const int s = base + (BWD ? nmine - 1 - j0 : j0) * P;
-        Chan in{nullptr, false}, out{nullptr, false};
-        if (!BWD) {  // rows travel upward: strip s takes from s-1, gives to s+1
-            if (s > 0) in = (one_round && w > 0) ? smem_row(w - 1) : glob_row(up + (size_t)(s - 1) * row);
-            if (s + 1 < sd.S)
-                out = (one_round && w + 1 < nstrips_blk) ? smem_row(w) : glob_row(up + (size_t)s * row);
-        } else {     // downward: strip s takes from s+1, gives to s-1
-            if (s + 1 < sd.S)
-                in = (one_round && w + 1 < nstrips_blk) ? smem_row(w) : glob_row(down + (size_t)(s + 1) * row);
-            if (s > 0) out = (one_round && w > 0) ? smem_row(w - 1) : glob_row(down + (size_t)s * row);
-        }
-        if (role == 0) {
-            if (in.valid) sweep32_strip<BWD, true>(A, s, R, out);
-            else sweep32_strip<BWD, false>(A, s, R, out);
-        } else if (role == 1) {
-            if (in.valid) load32_strip<BWD, true>(A, s, R, in);
-            else load32_strip<BWD, false>(A, s, R, in);
-        } else if (BWD) {
-            prepare32_strip(A, s, R);
-        } else {
-            R.skip(sd.D / kT);
-        }
-    }
-}
-
-// --------------------------------------------------------------- factor
-// buildPreconditioner (3-conjugate-gradients/Fluid.cpp:253-269): FP64
-// arithmetic in the reference's order (the factor is bit-identical), so the
-// step's ~35 FP64 instructions at 64 cycles each (one warp of an SM quarter)
-// are what it costs: rows, not tiles, are spread over the warps - lane l of a
-// warp walks row 32 q + l, one column behind lane l - 1 - and the scattered
-// accesses to the tile layout hide behind them.  A cell forms the terms that
-// its right and upper neighbours subtract from their diagonals (the same
-// products the reference forms there) and writes their al and bd.  The upper
-// term of row 32 q - 1 arrives through a halo row of W words.
-template <bool IN>
-__device__ __noinline__ void factor32_rows(const PcgArgs<float> &A, int q, const Chan in, const Chan out) {
-    const int lane = threadIdx.x & 31;
-    const SDIdx sd = A.sd;
-    const int W = sd.W, H = sd.H, y = 32 * q + lane;
-    const bool rowok = y < H;
-    const size_t base = sd.slot(0, rowok ? y : 0), above = sd.slot(0, y + 1 < H ? y + 1 : 0);
-    auto at = [](size_t row, int x) { return row + (size_t)(x >> 1) * 256 + (x & 1) * 128; };
-    // operands of the step after the current one
-    float ndiag = 0.f, nax = 0.f, nay = 0.f;
-    unsigned nbits = 0u;
-    unsigned long long nword = kSentinel;
-    auto prefetch = [&](int t) {
-        const int x = t - lane;
-        if (rowok && x >= 0 && x < W) {
-            const size_t k = at(base, x);
-            ndiag = A.adiag[k];
-            nax = A.ax[k];
-            nay = A.ay[k];
-            nbits = A.nb[k];
-        }
-        if constexpr (IN) nword = hload_if(in, t, lane == 0 && t < W, kSentinel);
-    };
-    double left = 0.0, upper = 0.0;  // terms for the right and the upper neighbour of the previous cell
-    prefetch(0);
-    for (int t = 0; t < W + 31; t++) {
-        const int x = t - lane;
-        const bool active = rowok && x >= 0 && x < W;
-        const double diag = to_f64(ndiag), ax = to_f64(nax), ay = to_f64(nay);
-        const unsigned b = active ? nbits : 0u;
-        double down = __shfl_up_sync(FULL, upper, 1);
-        if constexpr (IN) {
-            const bool need = lane == 0 && t < W;
-            const unsigned long long w = halo_take_warp(in, t, need, nword, A.fl);
-            if (need) down = hdec<double>(w);
-        }
-        if (t + 1 < W + 31) prefetch(t + 1);
-        double ev = diag;
-        if (b & NB_LEFT) ev = ev - left;
-        if (b & NB_DOWN) ev = ev - down;
-        if (ev < kSigma * diag) ev = diag;
-        const double pcv = 1.0 / sqrt(ev);
-        const double px = ax * pcv, py = ay * pcv, txy = kTau * px * py;
-        left = px * px + txy;
-        upper = py * py + txy;
-        const bool self = b & NB_SELF;
-        const double p2 = self ? pcv * pcv : 0.0;
-        const float va = to_f32(ax * p2), vb = to_f32(ay * p2);
-        if (active) {
-            const size_t k = at(base, x);
-            if (self) A.pc[k] = pcv;
-            *bwd_coef(A, k, C_A) = -va;
-            *bwd_coef(A, k, C_B) = -vb;
-            *bwd_coef(A, k, C_DD) = to_f32(p2);
-            if (x + 1 < W) *fwd_coef(A, at(base, x + 1), C_AL) = -va;
-            if (y + 1 < H) *fwd_coef(A, at(above, x), C_BD) = -vb;
-        }
-        hstore_if(out, x, henc(upper), out.valid && lane == 31 && active);
-    }
-}
-
-// ------------------------------------------------------------------ solve
-// Sum (or maximum) of n partials in a fixed order that depends on n alone:
-// virtual warp v < kSums adds the partials v*32 + lane + 512 k in order of k,
-// its lanes follow a fixed shuffle tree, and so do the kSums results.  Every
-// block forms the same bits, whatever its number of warps.
-__device__ __forceinline__ double total32(const double *pt, int n, bool is_max, double *sm) {
-    const int warps = blockDim.x >> 5;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (n <= 32) {  // every warp for itself
-        double acc = lane < n ? __ldcg(pt + lane) : 0.0;
-        for (int o = 16; o > 0; o >>= 1) {
-            if (o >= n) continue;
-            const double w = __shfl_down_sync(FULL, acc, o);
-            acc = is_max ? smax(acc, w) : acc + w;
-        }
-        return __shfl_sync(FULL, acc, 0);
-    }
-    for (int v = warp; v < kSums; v += warps) {
-        double acc = 0.0;
-        if (v * 32 < n) {
-            for (int i0 = v * 32 + lane; i0 < n; i0 += 4 * 32 * kSums) {
-                double w[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) w[j] = i0 + j * 32 * kSums < n ? __ldcg(pt + i0 + j * 32 * kSums) : 0.0;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (i0 + j * 32 * kSums < n) acc = is_max ? smax(acc, w[j]) : acc + w[j];
-            }
-            acc = is_max ? warp_max(acc) : warp_sum(acc);
-        }
-        if (lane == 0) sm[v] = acc;
-    }
-    __syncthreads();
-    double acc = sm[lane & (kSums - 1)];
-    const int used = (n + 31) / 32;  // sums beyond are zero
-    for (int o = kSums / 2; o > 0; o >>= 1) {
-        if (o >= used) continue;
-        const double w = __shfl_xor_sync(FULL, acc, o);
-        acc = is_max ? smax(acc, w) : acc + w;
-    }
-    return __shfl_sync(FULL, acc, 0);
 }
 
 // What a lane needs to find its tile: (strip, lane) and the tile grid.
@@ -622,7 +246,7 @@ struct Tiles {
 // carry no cancellation between the diagonal and the neighbours.  Heat
 // matrices: a float-float sum of the exact products.
 template <bool ROWSUM>
-__device__ __noinline__ void matvec32(const PcgArgs<float> &A, int iter, float beta, int c_begin, int c_end, int c_step, int kc) {
+__device__ __noinline__ void matvec(const PcgArgs<float> &A, int iter, float beta, int c_begin, int c_end, int c_step, int kc) {
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     const int D = sd.D;
@@ -778,23 +402,9 @@ __device__ __forceinline__ unsigned live4(const PcgArgs<float> &A, const SDIdx &
 }
 static_assert(NB_RED == 32, "live4 picks bit 5 of each cell's byte");
 
-// std::max(maxError, |r|) on the bit patterns: non-negative doubles order as
-// unsigned integers; a NaN (above +inf) is skipped, as (maxError < NaN) is false.
-__device__ __forceinline__ void max_bits(unsigned long long &mx, double r) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
-    if (b <= 0x7ff0000000000000ull && b > mx) mx = b;
-}
-__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(FULL, v, o);
-        v = w > v ? w : v;
-    }
-    return v;
-}
-
 // p += alpha s; r -= alpha z'; maxError = |r|_inf  (:363-366)
-template <bool ROWSUM, bool MASKED>
-__device__ __noinline__ void axpy32(const PcgArgs<float> &A, int iter, double alpha, int c_begin, int c_end, int c_step, int kc) {
+template <bool REF, bool ROWSUM, bool MASKED>
+__device__ __noinline__ void axpy(const PcgArgs<float> &A, int iter, double alpha, int c_begin, int c_end, int c_step, int kc) {
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     const int D = sd.D;
@@ -853,7 +463,7 @@ __device__ __noinline__ void axpy32(const PcgArgs<float> &A, int iter, double al
 
 // p = 0; maxError = |r|_inf (3-conjugate-gradients/Fluid.cpp:350, 354); FP32 copy of r.
 template <bool MASKED>
-__device__ __noinline__ void start32(const PcgArgs<float> &A, int c_begin, int c_end, int c_step, int kc) {
+__device__ __noinline__ void start(const PcgArgs<float> &A, int c_begin, int c_end, int c_step, int kc) {
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     for (int c = c_begin; c < c_end; c += c_step) {
@@ -881,206 +491,22 @@ __device__ __noinline__ void start32(const PcgArgs<float> &A, int c_begin, int c
     }
 }
 
-// One complete solve (factor and/or PCG, by A.mode) of one scene by team T.
-// The halo words must hold the sentinel on entry; those that a sweep waits for
-// hold it again on exit (every word that is waited for is taken).
-// The elementwise passes work on chunks of pcg_chunk_diags(sd) tile diagonals,
-// dealt out to the team's warps in turn.  Every reduction is summed per chunk
-// (per strip for sigma), then over the partials in a fixed order, so the result
-// depends on the scene alone, not on the number of blocks or warps that solve
-// it: a scene gives bit-identical results in a single-scene launch, in any
-// batch and with any launch shape.
-// sigma = z.r is taken as y.(dd y), y the forward solve's result: z.r =
-// (L^-T D L^-1 r).r = (L^-1 r).D(L^-1 r) exactly, and in floating point within
-// the rounding of the two triangular solves.  Cells outside the masked MIC(0)
-// work have dd = 0 and add nothing.
-__device__ void pcg32_job(const PcgArgs<float> &A, Team &T, Ring32 &R, double *sm) {
-    const int warps = blockDim.x >> 5;
-    const SDIdx sd = A.sd;
-    const int warp = threadIdx.x >> 5;
-    const int kc = pcg_chunk_diags(sd);
-    const int nchunk = (int)pcg_chunks(sd);
-    const int nwarps = T.size * warps;
-    // chunks c_begin, c_begin + nwarps, ...: every SM quarter gets as many, few or many
-    const int c_begin = warp * T.size + T.rank, c_end = nchunk;
-    R.buf = ring32_offset(A.K, sd.D) + (unsigned)(warp % A.K) * A.stages * kStageBytes;
-    const bool masked = !A.all_red, pressure = A.rowsum_zero;
-    const double *part = A.partials;
-
-    if (A.mode & PCG_FACTOR) {
-        const int nq = (sd.H + 31) / 32;
-        for (int q = warp * T.size + T.rank; q < nq; q += nwarps) {
-            const Chan in{A.halo + (size_t)(q > 0 ? q - 1 : 0) * sd.W, q > 0}, out{A.halo + (size_t)q * sd.W, q + 1 < nq};
-            if (q > 0) factor32_rows<true>(A, q, in, out);
-            else factor32_rows<false>(A, q, in, out);
-        }
-        team_barrier(T, A.fl);
-    }
-    if (!(A.mode & PCG_SOLVE)) return;
-
-    if (masked) start32<true>(A, c_begin, c_end, nwarps, kc);
-    else start32<false>(A, c_begin, c_end, nwarps, kc);
-    team_barrier(T, A.fl);
-    // z = M^-1 r  (:351)
-    sweep32<false>(A, T, R);
-    team_barrier(T, A.fl);
-    sweep32<true>(A, T, R);
-    team_barrier(T, A.fl);
-
-    double maxError = total32(part, nchunk, true, sm);
-    double sigma = total32(part + 2 * nchunk, sd.S, false, sm + 2 * kSums);
-    int iterations = 0, status;
-    if (A.pinned >= 0 ? A.pinned == 0 : maxError < kTol) {
-        status = 1;
-    } else {
-        status = 2;
-        double beta = 0.0;
-        // the search direction alternates between sa and sb (the matvec reads one
-        // and writes the other): iteration k writes sb when k is even
-        for (int iter = 0; iter < A.limit; iter++) {
-            // block-uniform: every thread of the block leaves together
-            if ((iter & 15) == 0 && __syncthreads_or(threadIdx.x == 0 && timed_out(A.fl))) break;
-            if (pressure) matvec32<true>(A, iter, (float)beta, c_begin, c_end, nwarps, kc);
-            else matvec32<false>(A, iter, (float)beta, c_begin, c_end, nwarps, kc);
-            team_barrier(T, A.fl);
-            const double alpha = sigma / total32(part + nchunk, nchunk, false, sm + kSums);
-            if (!pressure) axpy32<false, true>(A, iter, alpha, c_begin, c_end, nwarps, kc);
-            else if (masked) axpy32<true, true>(A, iter, alpha, c_begin, c_end, nwarps, kc);
-            else axpy32<true, false>(A, iter, alpha, c_begin, c_end, nwarps, kc);
-            team_barrier(T, A.fl);
-            maxError = total32(part, nchunk, true, sm);
-            iterations = iter + 1;
-            if (A.pinned >= 0 ? iterations >= A.pinned : maxError < kTol) {
-                status = 0;
-                break;
-            }
-            // z = M^-1 r; sigmaNew = z.r  (:372-376)
-            sweep32<false>(A, T, R);
-            team_barrier(T, A.fl);
-            sweep32<true>(A, T, R);
-            team_barrier(T, A.fl);
-            const double sigmaNew = total32(part + 2 * nchunk, sd.S, false, sm + 2 * kSums);
-            beta = sigmaNew / sigma;
-            sigma = sigmaNew;
-        }
-        if (status == 2) iterations = A.limit;
-    }
-    if (T.rank == 0 && threadIdx.x == 0) {
-        A.out->iterations = iterations;
-        A.out->status = status;
-        A.out->max_error = maxError;
-        atomicAdd(A.iter_total, (unsigned long long)iterations);
-    }
-}
-
-// Ring state of this warp (its role's position); the mbarriers are initialised
-// once per launch.
-__device__ void ring32_init(Ring32 &R, int K, int stages) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    R.buf = 0u;
-    R.bars = 8u * Ring32::KINDS * kMaxStages * (warp % K);
-    R.stages = stages;
-    R.st = 0;
-    R.parity = 0u;
-    R.dead = false;
-    if (lane == 0 && warp < K) {
-        for (int k = 0; k < stages; k++) {
-            mbar_init(R.bar(Ring32::COPIED, k), 1);
-            mbar_init(R.bar(Ring32::READY, k), 2);
-            mbar_init(R.bar(Ring32::FREE, k), 1);
-        }
-        fence_mbar_init();
-    }
-}
-
-// 168 registers per thread.
-constexpr int kMaxThreads32 = 384;
-
-__global__ void __launch_bounds__(kMaxThreads32, 1) pcg32_kernel(PcgArgs<float> A) {
-    __shared__ double sm[3 * kSums];
-    Team T{(int)blockIdx.x, (int)gridDim.x, A.barrier, 0u};
-    Ring32 R;
-    ring32_init(R, A.K, A.stages);
-    const size_t nh = 2 * (size_t)(A.K > 1 ? A.K - 1 : 0) * pcg_halo_row(A.sd);
-    for (size_t k = threadIdx.x; k < nh; k += blockDim.x)
-        ((unsigned long long *)(g_smem + halo32_offset(A.K)))[k] = kSentinel;
-    __syncthreads();
-    pcg32_job(A, T, R, sm);
-}
-
-// Many independent scenes in one cooperative launch (see BatchTeams).
-__global__ void __launch_bounds__(kMaxThreads32, 1)
-    pcg32_batch_kernel(const PcgArgs<float> *jobs, BatchTeams B, int mode, int heat, int pinned, int K, int stages) {
-    __shared__ double sm[3 * kSums];
-    __shared__ PcgArgs<float> sA;
-    __shared__ int s_slot;
-    const int2 bt = batch_slot(B, &s_slot);
-    const int2 tm = B.team[bt.x];
-    Team T{bt.y, tm.x, B.team_bar + kBarStride * bt.x, 0u};
-    Ring32 R;
-    ring32_init(R, K, stages);
-    __syncthreads();
-    while (batch_take<float>(B, T, bt.x, tm.y, jobs, sA, mode, heat, pinned, K, stages)) {
-        // halo rows start at the sentinel: the shared rows of this block
-        // (their length changes with the scene) and the scene's global rows
-        const size_t nh = 2 * (size_t)(K > 1 ? K - 1 : 0) * pcg_halo_row(sA.sd);
-        for (size_t k = threadIdx.x; k < nh; k += blockDim.x)
-            ((unsigned long long *)(g_smem + halo32_offset(K)))[k] = kSentinel;
-        const size_t ng = pcg_halo_words(sA.sd);
-        for (size_t k = (size_t)T.rank * blockDim.x + threadIdx.x; k < ng; k += (size_t)T.size * blockDim.x)
-            sA.halo[k] = kSentinel;
-        team_barrier(T, sA.fl);
-        pcg32_job(sA, T, R, sm);
-    }
-}
-
-constexpr int kSingleThreads = 256, kSingleStages = 6;
-
 }  // namespace
 
-size_t pcg32_smem(int K, int D, int stages) { return ring32_offset(K, D) + (size_t)K * stages * kStageBytes; }
+}  // namespace ifl
 
-const void *pcg32_batch_fn() { return (const void *)pcg32_batch_kernel; }
-// What a shape {threads, strips per block, stages} comes to: at least a strip's
-// three warps per strip, as many strips and stages as threads and shared memory
-// allow (smem: bytes of a block).
+#include "pcg_job.cuh"
+
+namespace ifl {
+
+size_t pcg32_smem(int K, int D, int stages) { return pcg_smem<float>(K, D, stages); }
+const void *pcg32_batch_fn() { return (const void *)pcg_batch_kernel<float>; }
 void pcg32_shape(int threads, int D, size_t smem_max, int *block, int *K, int *stages) {
-    *K = std::min(*K, kMaxThreads32 / (32 * kRoles));
-    while (*stages > 2 && pcg32_smem(*K, D, *stages) > smem_max) (*stages)--;
-    while (*K > 1 && pcg32_smem(*K, D, *stages) > smem_max) (*K)--;
-    *block = std::max(threads, 32 * kRoles * *K);
+    pcg_shape<float>(threads, D, smem_max, block, K, stages);
 }
-
 cudaError_t launch_pcg32(PcgArgs<float> A, const PcgScratch &X, const PcgConfig &cfg, cudaStream_t st,
                          int *blocks_used) {
-    const SDIdx &sd = A.sd;
-    A.mode = cfg.mode;
-    A.limit = cfg.limit;
-    A.pinned = cfg.pinned;
-    // A strip per SM: two would hand over through its shared memory, but in the
-    // backward sweep they also share its bandwidth (copies, preparer and sweep
-    // move 11 KB per step, 86 cycles).
-    A.K = 1;
-    A.stages = kSingleStages;
-    A.fl.limit = cfg.wait_limit > 0 ? cfg.wait_limit : kWaitLimit;
-    const size_t smem = pcg32_smem(A.K, sd.D, A.stages);
-    const void *fn = (const void *)pcg32_kernel;
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    // one block per SM; small scenes: as many blocks as give every chunk an SM
-    // quarter (FP64 instructions of one quarter do not overlap)
-    const int want = std::max((sd.S + A.K - 1) / A.K, (int)((pcg_chunks(sd) + 3) / 4));
-    const int G = std::max(1, std::min(std::min(sms, X.max_blocks), want));
-    if (blocks_used) *blocks_used = G;
-    e = cudaMemsetAsync(X.barrier, 0, sizeof(unsigned), st);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(X.halo, 0xff, pcg_halo_words(sd) * sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
-    void *args[] = {&A};
-    return cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kSingleThreads), args, smem, st);
+    return launch_single<float>(A, X, cfg, st, blocks_used);
 }
 
 }  // namespace ifl

@@ -20,9 +20,9 @@ namespace {
 constexpr size_t kMaxStripDiagonals = 2304;
 constexpr size_t kMaxSlots = kMaxStripDiagonals * 32;
 constexpr size_t kMaxBlocks = 512;
-// FP64 arrays per slot: adiag, ax, ay, pc, r, p, as, z, sa, sb (10) + MIC record (4)
-constexpr size_t kScratchBytes = kMaxSlots * (14 * 8 + 1) + 2 * kMaxStripDiagonals * 8 +
-                                 4 * kMaxBlocks * 8 + 1024;
+// FP64 arrays per slot: adiag, ax, ay, pc, r, p, as, z, sa, sb (10) + MIC operands (5)
+constexpr size_t kScratchBytes = kMaxSlots * (15 * 8 + 1) + 4 * kMaxStripDiagonals * 8 +
+                                 4 * kMaxStripDiagonals * 8 + 32 * 1024;
 
 // The shared scratch.  Every GPU that loads the library holds it until exit.
 static __device__ __align__(256) unsigned char g_pcg_scratch[kScratchBytes];
@@ -111,7 +111,7 @@ extern "C" int ifl_pcg_solve_noalloc(int w, int h, const double *adiag, const do
     S.ax = take<double>(cur, n);
     S.ay = take<double>(cur, n);
     S.pc = take<double>(cur, n);
-    S.mic = take<double>(cur, 4 * n);
+    S.mic = take<double>(cur, 5 * n);
     S.r = take<double>(cur, n);
     S.rf = S.r;
     S.p = take<double>(cur, n);
@@ -122,7 +122,7 @@ extern "C" int ifl_pcg_solve_noalloc(int w, int h, const double *adiag, const do
     S.nb = take<uint8_t>(cur, n);
     S.flags = take<unsigned>(cur, 8);
     PcgScratch X{};
-    X.halo = take<unsigned long long>(cur, 2 * (size_t)sd.S * sd.D);
+    X.halo = take<unsigned long long>(cur, pcg_halo_words(sd));
     X.partials = take<double>(cur, pcg_partials(sd));
     X.barrier = take<unsigned>(cur, 2);
     X.iter_total = take<unsigned long long>(cur, 1);
@@ -131,8 +131,10 @@ extern "C" int ifl_pcg_solve_noalloc(int w, int h, const double *adiag, const do
     if ((size_t)(cur - (unsigned char *)base) > kScratchBytes) return IFL_ERR_UNSUPPORTED;
 
     // The array keeps the previous call's contents: clear what must start at
-    // zero (neighbour bits of the padding slots, status word).
-    if (cudaMemsetAsync(S.nb, 0, n, st) != cudaSuccess || cudaMemsetAsync(S.flags, 0, 8 * sizeof(unsigned), st) != cudaSuccess)
+    // zero (the padding slots of what the solve reads everywhere, status word).
+    if (cudaMemsetAsync(S.nb, 0, n, st) != cudaSuccess || cudaMemsetAsync(S.r, 0, n * sizeof(double), st) != cudaSuccess ||
+        cudaMemsetAsync(S.mic, 0, 5 * n * sizeof(double), st) != cudaSuccess ||
+        cudaMemsetAsync(S.flags, 0, 8 * sizeof(unsigned), st) != cudaSuccess)
         return IFL_ERR_CUDA;
     dim3 b(32, 8), g((w + 31) / 32, (h + 7) / 8);
     noalloc_in_kernel<<<g, b, 0, st>>>(sd, adiag, aplusx, aplusy, rhs, S.adiag, S.ax, S.ay, S.r, S.nb);

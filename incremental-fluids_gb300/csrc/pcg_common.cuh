@@ -46,7 +46,7 @@ struct PcgArgs {
     SDIdx sd;
     const F *adiag, *ax, *ay;
     double *pc;
-    F *mic;  // FP64: MIC(0) record per slot {lx, ly, pc, neighbour bits}; FP32 form: five coefficient arrays (k_pcg32.cu)
+    F *mic;  // MIC(0) apply operands, five values per slot (pcg_ring.cuh)
     const uint8_t *nb;
     double *r, *p, *as;
     F *rf;  // r in storage precision for the substitutions (== r when F is double)
@@ -61,6 +61,7 @@ struct PcgArgs {
     int K, stages;
     int rowsum_zero;  // 1: pressure matrix (rows sum to zero), 0: heat matrix
     int all_red;      // 1: every cell takes part in the dot products and AXPYs (unmasked solves)
+    int ref;          // FP64: 1: the reference's own arithmetic (k_pcg64.cu)
 };
 
 // ------------------------------------------------------------ PTX helpers

@@ -1,0 +1,385 @@
+// pcg_ring.cuh - the parts of the PCG kernels that do not depend on what a lane
+// does in a step of a sweep: the ring that feeds a sweeping warp, the MIC(0)
+// factor, fixed-order sums (k_pcg64.cu, k_pcg32.cu).
+#pragma once
+#include <algorithm>
+#include <cstring>
+#include <type_traits>
+
+#include "pcg_common.cuh"
+
+namespace ifl {
+
+namespace {
+
+// The order of the sums that scenes with bodies keep in FP64 (k_pcg64.cu): chunks
+// of kRefChunk diagonals, in which each lane adds its cells in the order of the
+// diagonals and the lanes follow a shuffle tree; then lane l of one warp adds the
+// chunks l, l + 32, ... and the lanes follow the same tree.
+constexpr int kRefChunk = 16;
+__device__ __forceinline__ int ref_chunks(const SDIdx &sd) { return sd.S * sd.D / kRefChunk; }
+__device__ __forceinline__ double ref_total(const double *pt, int n, double *sm) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        double acc = 0.0;
+        for (int c0 = lane; c0 < n; c0 += 32 * 8) {
+            double v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = c0 + 32 * j < n ? __ldcg(pt + c0 + 32 * j) : 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (c0 + 32 * j < n) acc = acc + v[j];
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) sm[0] = acc;
+    }
+    __syncthreads();
+    return sm[0];
+}
+
+// Steps of a ring block, and cells of a diagonal (see SDIdx).
+template <typename F> struct Lay;
+template <> struct Lay<double> { static constexpr int kSteps = 8, kCells = 32; };
+template <> struct Lay<float> { static constexpr int kSteps = kTileBlock, kCells = 256; };
+template <typename F> constexpr unsigned kVecBytes = Lay<F>::kSteps * Lay<F>::kCells * sizeof(F);  // a block of one array
+template <typename F> constexpr unsigned kHaloAt = 4u * kVecBytes<F>;       // its halo words, behind four arrays
+template <typename F> constexpr unsigned kStageBytes = kHaloAt<F> + 128u;   // a ring stage
+constexpr int kMaxStages = 8;
+constexpr int kMaxThreads = 384;  // of a block (168 registers per thread)
+constexpr int kRoles = 3;   // warps that work on one strip: sweep, load, prepare
+constexpr int kSums = 16;   // partial sums of a reduction (see total_of)
+
+// ---------------------------------------------------------- conversions
+// float <-> double on the integer pipe.  A conversion instruction takes an FP64
+// slot (19 cycles per warp and SM on this part), these take about eight integer
+// instructions (2 cycles).  Zeros and normal numbers here; subnormals,
+// infinities and NaN take the instruction.
+__device__ __forceinline__ double to_f64(float f) {
+    const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
+    unsigned hi = (t >> 3) + 0x38000000u, lo = u << 29;
+    if (t - 0x00800000u >= 0x7f000000u) {  // zero, subnormal, infinity, NaN
+        if (t != 0u) return (double)f;
+        hi = 0u;
+        lo = 0u;
+    }
+    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
+}
+// Round to nearest even, as the instruction.
+__device__ __forceinline__ float to_f32(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), t = hi & 0x7fffffffu;
+    if (t - 0x38100000u >= 0x0fe00000u) {  // outside [2^-126, 2^128): zero, subnormal result, overflow, NaN
+        if ((t | lo) != 0u) return (float)d;
+        return __uint_as_float(hi & 0x80000000u);
+    }
+    unsigned m = ((t - 0x38000000u) << 3) | (lo >> 29);
+    const unsigned rest = lo & 0x1fffffffu;
+    m += (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
+    return __uint_as_float(m | (hi & 0x80000000u));
+}
+
+template <typename F> __device__ __forceinline__ F from_f64(double d);
+template <> __device__ __forceinline__ double from_f64<double>(double d) { return d; }
+template <> __device__ __forceinline__ float from_f64<float>(double d) { return to_f32(d); }
+__device__ __forceinline__ double to_f64(double d) { return d; }
+
+// The MIC(0) coefficients lie as the sweeps read them, a diagonal's arrays side by
+// side: those of the forward sweep, then, behind them all, those of the backward
+// sweep.  In the L D L^T form -al, -bd and dd, -a, -b (k_pcg32.cu); in the
+// reference's own form (REF, see k_pcg64.cu) lx of the left cell, ly of the lower
+// cell, pc and lx, ly, pc, with lx = aPlusX pc and ly = aPlusY pc.
+template <bool REF, bool BWD> constexpr int kCoefs = REF || BWD ? 3 : 2;
+enum { C_LEFT = 0, C_DOWN = 1, C_RIGHT = 1, C_UP = 2, C_DD = 0, R_RIGHT = 0, R_UP = 1, R_PC = 2 };
+// Array `arr` of the cell with slot k.
+template <bool REF, bool BWD, typename F>
+__device__ __forceinline__ F *coef(const PcgArgs<F> &A, size_t k, int arr) {
+    constexpr int n = Lay<F>::kCells, c = kCoefs<REF, BWD>;
+    return A.mic + (BWD ? kCoefs<REF, false> * A.sd.total() : 0) + (k / n) * (c * n) + arr * n + k % n;
+}
+
+// --------------------------------------------------------------- sweeps
+// A strip's ring in shared memory: `stages` buffers of kSteps diagonals,
+//   [r][al, bd per diagonal] (forward) or [y][dd, a, b per diagonal] (backward),
+//   then the halo words of the block's steps.
+// Three warps share it, each with its own running position (stage, mbarrier
+// parity):
+//  * the loader waits for a free stage, starts two bulk copies into it, takes the
+//    block's halo words as they arrive and puts them behind the operands;
+//  * the preparer (backward, L D L^T form) waits for the copies, multiplies y by dd in place and
+//    adds up sigma;
+//  * the sweeping warp waits for both (`ready`), stores its results and hands its
+//    boundary row on, and frees the stage.
+// Every wait is bounded.  A timeout elsewhere in the launch does not shorten the
+// mbarrier waits: the copies were issued from this GPU's memory and complete,
+// and the loader's halo polls give up by themselves, so a timed-out sweep still
+// consumes every block it issued and no bulk copy is left behind in shared memory.
+// A ring is `dead` once an mbarrier wait ran out all the same: its warp then
+// waits and issues no more.
+template <typename F>
+struct Ring {
+    unsigned buf;   // byte offset of the stages in g_smem
+    unsigned bars;  // byte offset of the mbarriers, kMaxStages of each kind
+    int stages, st;
+    unsigned parity;
+    bool dead;
+    enum { COPIED = 0, READY = 1, FREE = 2, KINDS = 3 };
+    __device__ __forceinline__ uint64_t *bar(int kind, int at) const {
+        return (uint64_t *)(g_smem + bars) + kind * kMaxStages + at;
+    }
+    __device__ __forceinline__ unsigned stage(int at) const { return buf + (unsigned)at * kStageBytes<F>; }
+    __device__ __forceinline__ void next() {
+        st = st + 1 == stages ? 0 : st + 1;
+        parity ^= st == 0 ? 1u : 0u;
+    }
+    __device__ __forceinline__ void skip(int n) {  // n blocks that this warp has no part in
+        const int at = st + n;
+        st = at % stages;
+        parity ^= (unsigned)(at / stages) & 1u;
+    }
+};
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Whether a phase is complete, without waiting for it (try_wait suspends).
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Whole warp: the phase `parity` of a barrier.
+template <typename F>
+__device__ __forceinline__ void ring_wait(Ring<F> &R, uint64_t *bar, unsigned parity, const Flags &flags) {
+    if (__all_sync(FULL, R.dead || mbar_try_wait(bar, parity))) return;
+    long long n = 0;
+    while (!__all_sync(FULL, mbar_try_wait(bar, parity))) {
+        if (++n > kMbarWaitLimit + flags.limit) {
+            set_timeout(flags);
+            R.dead = true;
+            break;
+        }
+    }
+}
+
+// The loader's part of one strip.  Halo words: at step t the waiting lane needs
+// the boundary value of one column (a double, or the two floats of a tile's
+// columns) in one 8-byte word of the neighbour's row (t <= D - 32; beyond, the
+// coefficient is zero).  Lane i polls the word of the i-th step from the first block that waits
+// for words, so one round of loads (about 700 cycles) serves up to eight blocks.
+template <typename F, bool REF, bool BWD, bool IN>
+__device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &ring, const Chan in) {
+    constexpr int kC = kCoefs<REF, BWD>;  // coefficient arrays
+    constexpr bool kPrepared = BWD && !REF;  // the preparer stands between the copies and the sweep
+    constexpr int kT = Lay<F>::kSteps, kCells = Lay<F>::kCells;
+    constexpr unsigned kVec = kVecBytes<F>;
+    Ring<F> R = ring;
+    const Flags flags = A.fl;
+    const int lane = threadIdx.x & 31;
+    const int D = A.sd.D, nblk = D / kT;
+    const size_t row0 = (size_t)s * D + (BWD ? D - kT : 0);  // first diagonal of the first block
+    const F *vec = (BWD ? A.z : A.rf) + row0 * kCells;
+    const F *cf = coef<REF, BWD>(A, row0 * kCells, 0);
+    fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
+    int issued = 0, ready = 0;   // blocks whose copies are started, whose halo words are in place
+    int rst = R.st;              // stage of block `ready`
+    unsigned long long w = kSentinel;
+    bool given_up = false;
+    long long polls = 0;
+    while (ready < nblk) {
+        // start copies into free stages; wait for one only when there is nothing else to do
+        while (issued < nblk && issued < ready + R.stages) {
+            uint64_t *fr = R.bar(Ring<F>::FREE, R.st);
+            if (!__all_sync(FULL, R.dead || mbar_test(fr, R.parity ^ 1u))) {
+                if (issued > ready) break;
+                ring_wait(R, fr, R.parity ^ 1u, flags);
+            }
+            if (lane == 0) {
+                // without a preparer the sweeping warp itself waits for the copies; `copied` keeps pace
+                uint64_t *ready_bar = R.bar(Ring<F>::READY, R.st), *copied = R.bar(Ring<F>::COPIED, R.st);
+                uint64_t *tx = kPrepared ? copied : ready_bar;
+                char *dst = g_smem + R.stage(R.st);
+                mbar_expect_tx(tx, (1u + kC) * kVec);
+                bulk_g2s(dst, vec, kVec, tx);
+                bulk_g2s(dst + kVec, cf, kC * kVec, tx);
+                if (!kPrepared) mbar_arrive(copied);
+                if (!IN) mbar_arrive(ready_bar);
+            }
+            vec += BWD ? -kT * kCells : kT * kCells;
+            cf += (BWD ? -kT * kCells : kT * kCells) * kC;
+            R.next();
+            issued++;
+            if (!IN) ready++;
+        }
+        if constexpr (IN) {
+            const int t = ready * kT + lane;
+            const bool need = t <= D - 32;
+            unsigned long long *word = in.row + (BWD ? D - 32 - t : t + 32);
+            if (need && w == kSentinel && !given_up) {
+                asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(w) : "l"(word));
+                if (w != kSentinel) asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(word), "l"(kSentinel));
+            }
+            if (!need) w = 0ull;
+            const unsigned have = __ballot_sync(FULL, w != kSentinel || given_up);
+            // blocks from `ready` on whose words are all there
+            int k = min(__ffs(~have) - 1 < 0 ? 32 : __ffs(~have) - 1, (issued - ready) * kT) / kT;
+            if (k > 0) {
+                polls = 0;
+                const int q = lane / kT;
+                int st = rst + q;
+                st -= st >= R.stages ? R.stages : 0;
+                if (q < k)
+                    *(volatile unsigned long long *)(g_smem + R.stage(st) + kHaloAt<F> + 8 * (lane % kT)) = given_up && w == kSentinel ? 0ull : w;
+                __syncwarp();
+                if (lane < k) {
+                    int at = rst + lane;
+                    at -= at >= R.stages ? R.stages : 0;
+                    mbar_arrive(R.bar(Ring<F>::READY, at));
+                }
+                w = __shfl_down_sync(FULL, w, k * kT);
+                if (lane >= 32 - k * kT) w = kSentinel;
+                ready += k;
+                rst += k;
+                rst -= rst >= R.stages ? R.stages : 0;
+            } else if (++polls > flags.limit || ((polls & 15) == 0 && __any_sync(FULL, timed_out(flags)))) {
+                if (!given_up) set_timeout(flags);
+                given_up = true;
+            }
+        }
+    }
+    ring = R;
+    __syncwarp();
+}
+
+// --------------------------------------------------------------- factor
+// buildPreconditioner (3-conjugate-gradients/Fluid.cpp:253-269): FP64
+// arithmetic in the reference's order (the factor is bit-identical), so the
+// step's ~35 FP64 instructions at 64 cycles each (one warp of an SM quarter)
+// are what it costs: rows, not tiles, are spread over the warps - lane l of a
+// warp walks row 32 q + l, one column behind lane l - 1 - and the scattered
+// accesses to the tile layout hide behind them.  A cell forms the terms that
+// its right and upper neighbours subtract from their diagonals (the same
+// products the reference forms there) and writes their al and bd.  The upper
+// term of row 32 q - 1 arrives through a halo row of W words.
+template <typename F, bool REF, bool IN>
+__device__ __noinline__ void factor_rows(const PcgArgs<F> &A, int q, const Chan in, const Chan out) {
+    const int lane = threadIdx.x & 31;
+    const SDIdx sd = A.sd;
+    const int W = sd.W, H = sd.H, y = 32 * q + lane;
+    const bool rowok = y < H;
+    const size_t base = sd.slot(0, rowok ? y : 0), above = sd.slot(0, y + 1 < H ? y + 1 : 0);
+    auto at = [](size_t row, int x) { return sizeof(F) == 8 ? row + (size_t)x * 32 : row + (size_t)(x >> 1) * 256 + (x & 1) * 128; };
+    // operands of the step after the current one
+    F ndiag = F(0), nax = F(0), nay = F(0);
+    unsigned nbits = 0u;
+    unsigned long long nword = kSentinel;
+    auto prefetch = [&](int t) {
+        const int x = t - lane;
+        if (rowok && x >= 0 && x < W) {
+            const size_t k = at(base, x);
+            ndiag = A.adiag[k];
+            nax = A.ax[k];
+            nay = A.ay[k];
+            nbits = A.nb[k];
+        }
+        if constexpr (IN) nword = hload_if(in, t, lane == 0 && t < W, kSentinel);
+    };
+    double left = 0.0, upper = 0.0;  // terms for the right and the upper neighbour of the previous cell
+    prefetch(0);
+    for (int t = 0; t < W + 31; t++) {
+        const int x = t - lane;
+        const bool active = rowok && x >= 0 && x < W;
+        const double diag = to_f64(ndiag), ax = to_f64(nax), ay = to_f64(nay);
+        const unsigned b = active ? nbits : 0u;
+        double down = __shfl_up_sync(FULL, upper, 1);
+        if constexpr (IN) {
+            const bool need = lane == 0 && t < W;
+            const unsigned long long w = halo_take_warp(in, t, need, nword, A.fl);
+            if (need) down = hdec<double>(w);
+        }
+        if (t + 1 < W + 31) prefetch(t + 1);
+        double ev = diag;
+        if (b & NB_LEFT) ev = ev - left;
+        if (b & NB_DOWN) ev = ev - down;
+        if (ev < kSigma * diag) ev = diag;
+        const double pcv = 1.0 / sqrt(ev);
+        const double px = ax * pcv, py = ay * pcv, txy = kTau * px * py;
+        left = px * px + txy;
+        upper = py * py + txy;
+        const bool self = b & NB_SELF;
+        const double p2 = !self ? 0.0 : REF ? pcv : pcv * pcv;
+        const F va = from_f64<F>(ax * p2), vb = from_f64<F>(ay * p2);
+        if (active) {
+            const size_t k = at(base, x);
+            const F dd = from_f64<F>(p2), sign = REF ? F(1) : F(-1);
+            if (self) A.pc[k] = pcv;
+            *coef<REF, true>(A, k, REF ? R_RIGHT : C_RIGHT) = sign * va;
+            *coef<REF, true>(A, k, REF ? R_UP : C_UP) = sign * vb;
+            *coef<REF, true>(A, k, REF ? R_PC : C_DD) = dd;
+            if (REF) *coef<REF, false>(A, k, R_PC) = dd;
+            if (x + 1 < W) *coef<REF, false>(A, at(base, x + 1), C_LEFT) = sign * va;
+            if (y + 1 < H) *coef<REF, false>(A, at(above, x), C_DOWN) = sign * vb;
+        }
+        hstore_if(out, x, henc(upper), out.valid && lane == 31 && active);
+    }
+}
+
+// Sum (or maximum) of n partials in a fixed order that depends on n alone:
+// virtual warp v < kSums adds the partials v*32 + lane + 512 k in order of k,
+// its lanes follow a fixed shuffle tree, and so do the kSums results.  Every
+// block forms the same bits, whatever its number of warps.
+__device__ __forceinline__ double total_of(const double *pt, int n, bool is_max, double *sm) {
+    const int warps = blockDim.x >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (n <= 32) {  // every warp for itself
+        double acc = lane < n ? __ldcg(pt + lane) : 0.0;
+        for (int o = 16; o > 0; o >>= 1) {
+            if (o >= n) continue;
+            const double w = __shfl_down_sync(FULL, acc, o);
+            acc = is_max ? smax(acc, w) : acc + w;
+        }
+        return __shfl_sync(FULL, acc, 0);
+    }
+    for (int v = warp; v < kSums; v += warps) {
+        double acc = 0.0;
+        if (v * 32 < n) {
+            for (int i0 = v * 32 + lane; i0 < n; i0 += 4 * 32 * kSums) {
+                double w[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) w[j] = i0 + j * 32 * kSums < n ? __ldcg(pt + i0 + j * 32 * kSums) : 0.0;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (i0 + j * 32 * kSums < n) acc = is_max ? smax(acc, w[j]) : acc + w[j];
+            }
+            acc = is_max ? warp_max(acc) : warp_sum(acc);
+        }
+        if (lane == 0) sm[v] = acc;
+    }
+    __syncthreads();
+    double acc = sm[lane & (kSums - 1)];
+    const int used = (n + 31) / 32;  // sums beyond are zero
+    for (int o = kSums / 2; o > 0; o >>= 1) {
+        if (o >= used) continue;
+        const double w = __shfl_xor_sync(FULL, acc, o);
+        acc = is_max ? smax(acc, w) : acc + w;
+    }
+    return __shfl_sync(FULL, acc, 0);
+}
+
+// std::max(maxError, |r|) on the bit patterns: non-negative doubles order as
+// unsigned integers; a NaN (above +inf) is skipped, as (maxError < NaN) is false.
+__device__ __forceinline__ void max_bits(unsigned long long &mx, double r) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+    if (b <= 0x7ff0000000000000ull && b > mx) mx = b;
+}
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long w = __shfl_xor_sync(FULL, v, o);
+        v = w > v ? w : v;
+    }
+    return v;
+}
+
+}  // namespace
+
+}  // namespace ifl
