@@ -93,11 +93,17 @@ __device__ __noinline__ void sweep_strip(const PcgArgs<double> &A, int s, Ring<d
 #pragma unroll
         for (int j = 0; j < kT; j++) {
             const int jj = BWD ? kT - 1 - j : j;
-            const char *c = g + kVec + (jj * kC + kSkip) * 256 + lane * 8;
+            const char *c = g + kVec + (jj * kC + kSkip) * 256;
+            const double2 pair = *(const double2 *)(c + lane * 16);
             o[j][0] = *(const double *)(g + jj * 256 + lane * 8);
-#pragma unroll
-            for (int e = 1; e < kO; e++) o[j][e] = *(const double *)(c + (e - 1) * 256);
-            if constexpr (IN) halo[j] = *(const double *)(g + kHaloAt<double> + 8 * j);
+            o[j][1] = pair.x;
+            o[j][2] = pair.y;
+            if constexpr (REF) o[j][3] = *(const double *)(c + 512 + lane * 8);
+            if (IN && (j & 1) == 0) {
+                const double2 word = *(const double2 *)(g + kHaloAt<double> + 8 * j);
+                halo[j] = word.x;
+                halo[j + 1] = word.y;
+            }
         }
 #pragma unroll
         for (int j = 0; j < kT; j++) {
@@ -131,13 +137,14 @@ struct Cells {
 };
 
 // s = z + beta*s (first iteration: s = z) and z' = A s on diagonal d
-// (3-conjugate-gradients/Fluid.cpp:361-362, 375, 315-332); returns z'.s of this
-// lane's cell.  A lane forms the new s of its cell and of the cells left and
+// (3-conjugate-gradients/Fluid.cpp:361-362, 375, 315-332); returns this lane's z'
+// and in *sv its s.  A lane forms the new s of its cell and of the cells left and
 // right of it; the lower neighbour is lane-1's left cell and the upper one
 // lane+1's right cell, which arrive by shuffle; lanes 0 and 31 take theirs from
 // the adjacent strips.  A neighbour that does not exist has a zero coefficient.
 template <bool REF>
-__device__ __forceinline__ double matvec_row(const PcgArgs<double> &A, const Cells &T, int s, int d, int iter, double beta) {
+__device__ __forceinline__ double matvec_row(const PcgArgs<double> &A, const Cells &T, int s, int d, int iter, double beta,
+                                             double *sv) {
     const int lane = T.lane, D = A.sd.D;
     const double *so = (iter & 1) ? A.sb : A.sa;
     double *sn = (iter & 1) ? A.sa : A.sb;
@@ -188,11 +195,8 @@ __device__ __forceinline__ double matvec_row(const PcgArgs<double> &A, const Cel
         sn[k] = C;
         A.as[k] = t;
     }
+    *sv = in ? C : 0.0;
     return in ? t : 0.0;
-}
-// The s that iteration `iter` writes at diagonal d.
-__device__ __forceinline__ double s_of(const PcgArgs<double> &A, const Cells &T, int d, int iter) {
-    return T.in(d) ? ((iter & 1) ? A.sa : A.sb)[T.at(d)] : 0.0;
 }
 
 // The matvec and z'.s over this warp's chunks.
@@ -206,8 +210,9 @@ __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double b
         const Cells T(sd, s, lane);
         double dacc = 0.0;
         for (int u = 0; u < kc; u++) {
-            const double t = matvec_row<false>(A, T, s, d0 + u, iter, beta);
-            dacc = fma(t, s_of(A, T, d0 + u, iter), dacc);
+            double v;
+            const double t = matvec_row<false>(A, T, s, d0 + u, iter, beta, &v);
+            dacc = fma(t, v, dacc);
         }
         dacc = warp_sum(dacc);
         if (lane == 0) A.partials[pcg_chunks(sd) + c] = dacc;
@@ -216,50 +221,42 @@ __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double b
 
 // ---- the reference's arithmetic, with sums over chunks of kRefChunk diagonals
 
-// The matvec: the warps of a block take the diagonals of up to three chunks in
-// turn and leave the products z' s in shared memory; a warp per chunk then adds
-// them in order.  (A warp per chunk, start to end, is 16 diagonals of 21 FP64
-// instructions one after the other, 10 us.)
-__device__ __noinline__ void ref_matvec(const PcgArgs<double> &A, const Team &T, int iter, double beta) {
-    __shared__ double prod[kMaxThreads / 128][kRefChunk][32];
+// Dot product of two operands by the chunk: the warps of a block form a chunk's
+// products, a diagonal each in turn, and leave them in shared memory; one warp
+// then adds them in order.  (A warp per chunk, start to end, takes four times as
+// long: 16 diagonals of up to 21 FP64 instructions, one after the other.)
+template <typename Product>
+__device__ __forceinline__ void ref_dot(const PcgArgs<double> &A, const Team &T, double *partials, Product product) {
+    __shared__ double prod[kRefChunk][32];
     const SDIdx sd = A.sd;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int set = warps / 4 > 0 ? warps / 4 : 1, n = ref_chunks(sd);
-    for (int c0 = T.rank * set; c0 < n; c0 += T.size * set) {
-        for (int i = warp; i < set * kRefChunk; i += warps) {
-            const int row = c0 * kRefChunk + i, s = row / sd.D, d = row - s * sd.D;
-            if (row >= n * kRefChunk) continue;
-            const Cells C(sd, s, lane);
-            const double t = matvec_row<true>(A, C, s, d, iter, beta);
-            prod[i / kRefChunk][i % kRefChunk][lane] = t * s_of(A, C, d, iter);
-        }
+    for (int c = T.rank; c < ref_chunks(sd); c += T.size) {
+        const int s = c * kRefChunk / sd.D, d0 = c * kRefChunk - s * sd.D;  // a chunk lies inside one strip
+        const Cells C(sd, s, lane);
+        for (int u = warp; u < kRefChunk; u += warps) prod[u][lane] = product(C, s, d0 + u);
         __syncthreads();
-        if (warp < set && c0 + warp < n) {
-            double dacc = 0.0;
-            for (int u = 0; u < kRefChunk; u++) dacc = dacc + prod[warp][u][lane];
-            dacc = warp_sum(dacc);
-            if (lane == 0) A.partials[pcg_chunks(sd) + c0 + warp] = dacc;
+        if (warp == 0) {
+            double acc = 0.0;
+#pragma unroll
+            for (int u = 0; u < kRefChunk; u++) acc = acc + prod[u][lane];
+            acc = warp_sum(acc);
+            if (lane == 0) partials[c] = acc;
         }
         __syncthreads();
     }
 }
-
+__device__ __noinline__ void ref_matvec(const PcgArgs<double> &A, const Team &T, int iter, double beta) {
+    ref_dot(A, T, A.partials + pcg_chunks(A.sd), [&](const Cells &C, int s, int d) {
+        double v;
+        const double t = matvec_row<true>(A, C, s, d, iter, beta, &v);
+        return t * v;
+    });
+}
 // sigma = z.r over the red cells (3-conjugate-gradients/Fluid.cpp:356, 376); z is
 // zero outside the masked MIC(0) work.
 __device__ __noinline__ void ref_dot_zr(const PcgArgs<double> &A, const Team &T) {
-    const SDIdx sd = A.sd;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, n = ref_chunks(sd);
-    for (int c = warp * T.size + T.rank; c < n; c += T.size * warps) {
-        const int s = c * kRefChunk / sd.D, d0 = c * kRefChunk - s * sd.D;
-        const Cells C(sd, s, lane);
-        double prod[kRefChunk], acc = 0.0;
-#pragma unroll
-        for (int u = 0; u < kRefChunk; u++) prod[u] = C.in(d0 + u) ? A.z[C.at(d0 + u)] * A.r[C.at(d0 + u)] : 0.0;
-#pragma unroll
-        for (int u = 0; u < kRefChunk; u++) acc = acc + prod[u];
-        acc = warp_sum(acc);
-        if (lane == 0) A.partials[2 * pcg_chunks(sd) + c] = acc;
-    }
+    ref_dot(A, T, A.partials + 2 * pcg_chunks(A.sd),
+            [&](const Cells &C, int, int d) { return C.in(d) ? A.z[C.at(d)] * A.r[C.at(d)] : 0.0; });
 }
 
 // p += alpha s; r -= alpha z'; maxError = |r|_inf  (:363-366).  MASKED: only the

@@ -86,14 +86,17 @@ __device__ __forceinline__ double to_f64(double d) { return d; }
 // side: those of the forward sweep, then, behind them all, those of the backward
 // sweep.  In the L D L^T form -al, -bd and dd, -a, -b (k_pcg32.cu); in the
 // reference's own form (REF, see k_pcg64.cu) lx of the left cell, ly of the lower
-// cell, pc and lx, ly, pc, with lx = aPlusX pc and ly = aPlusY pc.
+// cell, pc and lx, ly, pc, with lx = aPlusX pc and ly = aPlusY pc.  FP64: a cell's
+// two neighbour coefficients side by side (one 16-byte load of the sweep).
 template <bool REF, bool BWD> constexpr int kCoefs = REF || BWD ? 3 : 2;
 enum { C_LEFT = 0, C_DOWN = 1, C_RIGHT = 1, C_UP = 2, C_DD = 0, R_RIGHT = 0, R_UP = 1, R_PC = 2 };
 // Array `arr` of the cell with slot k.
 template <bool REF, bool BWD, typename F>
 __device__ __forceinline__ F *coef(const PcgArgs<F> &A, size_t k, int arr) {
-    constexpr int n = Lay<F>::kCells, c = kCoefs<REF, BWD>;
-    return A.mic + (BWD ? kCoefs<REF, false> * A.sd.total() : 0) + (k / n) * (c * n) + arr * n + k % n;
+    constexpr int n = Lay<F>::kCells, c = kCoefs<REF, BWD>, pair = BWD && !REF ? 1 : 0;
+    F *row = A.mic + (BWD ? kCoefs<REF, false> * A.sd.total() : 0) + (k / n) * (c * n);
+    if (sizeof(F) == 8 && (arr == pair || arr == pair + 1)) return row + pair * n + (k % n) * 2 + arr - pair;
+    return row + arr * n + k % n;
 }
 
 // --------------------------------------------------------------- sweeps
