@@ -158,6 +158,7 @@ struct PcgScratch {
     PcgOut *out;
     unsigned long long *iter_total;  // PCG iterations summed over launches
     int max_blocks;
+    unsigned long long *gs;  // gs_words(sd): the Gauss-Seidel solve's ring of sweeps (steps 1-2)
 };
 
 enum { PCG_FACTOR = 1, PCG_SOLVE = 2 };
@@ -203,11 +204,12 @@ struct PcgF32 {
 };
 cudaError_t launch_pcg_f32(const Scene<double> &S, const PcgF32 &M, const PcgScratch &X, const PcgConfig &c,
                            cudaStream_t st, int *blocks_used);
-// Gauss-Seidel solve of steps 1-2 (k_gs.cu): one CTA, h <= gs_max_rows().
+// Gauss-Seidel solve of steps 1-2 (k_gs.cu): h <= gs_max_rows().
 template <typename F>
 cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int limit, int pinned, cudaStream_t st,
                       long long wait_limit = 0);
 int gs_max_rows();
+size_t gs_words(const SDIdx &sd, int sms);  // words of PcgScratch::gs
 
 // Batched PCG: many scenes in one cooperative launch (k_pcg.cu).  The plan
 // holds the per-scene job tables and the team/queue tables on the device.

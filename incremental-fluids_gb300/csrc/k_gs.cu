@@ -5,274 +5,359 @@
 // five-point stencil with solid walls, p kept from the previous step, until
 // the largest change of a sweep is below 1e-5 or 600 sweeps.
 //
-// A lexicographic sweep is a recurrence on the new values of the left and
-// lower cells and the old values of the right and upper cells - the shape of
-// the MIC(0) forward substitution - so it runs as a strip wavefront and gives
-// the reference's values (and therefore its sweep counts) exactly: one warp
-// per 32-row strip, lane l on row 32s + l, step d visits the cell x = d - l of
-// every lane (one contiguous strip-diagonal line of p and r).  The left value
-// is the lane's own previous result, the lower one comes from lane l - 1 by
-// shuffle, or for lane 0 from the strip below once that strip has published
-// the diagonal; the right and upper values are the previous sweep's.
+// What bounds it: a cell is a chain of FP64 operations, each 64 cycles of its
+// warp on this part, and a sweep on its own is a recurrence along W + H
+// diagonals.  But sweep k + 1 needs only the values that sweep k left two
+// diagonals ahead of it, so many sweeps run at a time, each on a warp of its
+// own, and 600 sweeps take about 600 x 4 diagonal steps instead of 600 x (W + 31).
+// Every value, and so the sweep count, is that of the sequential loop.
 //
-// Consecutive sweeps overlap: sweep k reads the previous values from buffer
-// k & 1 and writes buffer (k + 1) & 1 (p and the scene's otherwise unused A*s
-// array), so a strip starts sweep k + 1 as soon as the strip above it has
-// passed the columns it needs in sweep k, instead of waiting for the whole
-// sweep.  The convergence test of sweep k is taken at the start of sweep
-// k + 2 (every strip has then finished sweep k), so at most one sweep runs
-// ahead of the test; when sweep k converged that extra sweep is discarded
-// (its output went to the other buffer).  The sweep count and every value are
-// those of the sequential loop.
+// Worker (s, j) is one warp: strip s (32 rows), sweeps j, j + J, j + 2J, ...
+// Lane l is on row 32s + l; step d visits the cell x = d - l of every lane (one
+// contiguous strip-diagonal line).  The left value is the lane's own previous
+// result, the lower one lane l - 1's by shuffle; the right one is the previous
+// sweep's value of the own row, the upper one lane l + 1's right one.  Lane 0
+// takes its lower value from strip s - 1's worker of the same sweep, lane 31 its
+// upper one from strip s + 1's worker of the previous sweep.
 //
-// The work per cell is FP64 (GB300 runs FP64 at 1/64 of the FP32 rate), so
-// every strip gets an SM of its own: one single-warp CTA per strip in a
-// cooperative launch, spread one per SM by a shared-memory reservation.
-// Strips hand over through L2 (progress counters, values read with
-// ld.global.cg); the maximum change of a sweep is the maximum of the per-strip
-// maxima, which every CTA forms itself.  Every wait is bounded; a timeout sets
-// the status word and an abort word that releases every other wait.
+// Hand-over: sweep k writes ring buffer (k + 1) mod B.  An entry is 16 bytes, the
+// value and the sweep's tag, stored and loaded as one: a reader that finds its
+// tag has the value, with no counter or fence behind it.  A worker loads the
+// entries of a step one step ahead (a step is about the L2's latency) and loads
+// again those that had not come.
+//
+// Convergence: the strips of a sweep pass its largest change on, the last strip
+// decides (`verdict`: the first converged sweep so far), and sweep k starts once
+// the verdict of sweep k - L is in and open.  So up to L - 1 sweeps run ahead of
+// the decision; their buffers are dropped.  B = L + 1 buffers: sweep k + B starts
+// after sweep k + 1 is complete (nobody reads sweep k any more) and found not
+// converged (sweep k is not the result).
+//
+// 600 sweeps at 128 x 128: 116 ms with one sweep and the head of the next in
+// flight, a hand-over with a fence every four diagonals and a division per cell.
+//
+// Every wait is bounded; a timeout sets the status word and an abort word that
+// releases every other wait.
+#include <algorithm>
+
 #include "ifl_device.cuh"
 
 namespace ifl {
 
 namespace {
 
-constexpr int kGB = 8;          // steps per block of neighbour-strip prefetches
-constexpr int kMaxSlots = 4;    // per-sweep maxima kept (sweep k in slot k % 4)
 constexpr double kGsTol = 1e-5;
+constexpr unsigned FULL = 0xffffffffu;
+
+struct __align__(16) Entry {
+    double v;
+    unsigned long long tag;  // sweep + 2 (the initial p counts as sweep -1); 0: empty
+};
 
 struct GsArgs {
     const double *r;
-    double *buf[2];  // p (sweep k reads buf[k & 1], writes buf[(k + 1) & 1])
+    double *p;
     SDIdx sd;
     double scale;  // timestep / (density * hx * hx)
     int limit, pinned;
-    long long spin_limit;  // polls of one progress-counter wait before the solve gives up
+    long long spin_limit;  // polls of one wait before the solve gives up
     PcgOut *out;
     unsigned *flags;
     unsigned long long *iter_total;
-    unsigned long long *prog;  // S progress counters (steps done over all sweeps), then the abort word
-    double *smax;              // kMaxSlots x S per-strip maxima
+    int J, L;              // sweeps in flight per strip; sweeps that may run ahead of a verdict
+    Entry *ring;           // L + 1 buffers of p
+    Entry *down, *up;      // -scale p of every strip's last and first row, by buffer, strip and column
+    Entry *change;         // L + 1 x S: largest change of a sweep up to strip s
+    Entry *verdict;        // L + 1: first converged sweep + 1, or 0 (as bits of v)
+    unsigned long long *abort;
 };
 
+// ------------------------------------------------------------- hand-over
+__device__ __forceinline__ Entry ld_entry(const Entry *e) {
+    Entry r;
+    unsigned long long v;
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+                 : "=l"(v), "=l"(r.tag)
+                 : "l"(e)
+                 : "memory");
+    r.v = __longlong_as_double((long long)v);
+    return r;
+}
+__device__ __forceinline__ void st_entry(Entry *e, double v, unsigned long long tag) {
+    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(e),
+                 "l"(__double_as_longlong(v)), "l"(tag)
+                 : "memory");
+}
 __device__ __forceinline__ bool gs_aborted(const GsArgs &A) {
-    return *(const volatile unsigned long long *)(A.prog + A.sd.S) != 0ull;
+    return *(const volatile unsigned long long *)A.abort != 0ull;
 }
 __device__ __forceinline__ void gs_abort(const GsArgs &A) {
     atomicOr(A.flags, FLAG_TIMEOUT);
-    *(volatile unsigned long long *)(A.prog + A.sd.S) = 1ull;
+    *(volatile unsigned long long *)A.abort = 1ull;
 }
-// Lane-0 wait until strip i has done `need` steps in total.
-__device__ __forceinline__ void gs_wait(const GsArgs &A, int i, unsigned long long need, unsigned long long &seen) {
-    if (seen >= need) return;
+// Whole warp: the entry with this tag, and what its writer did before (acquire).
+__device__ __forceinline__ double gs_wait(const GsArgs &A, const Entry *e, unsigned long long tag) {
+    Entry c = ld_entry(e);
     long long spins = 0;
-    while ((seen = *(const volatile unsigned long long *)(A.prog + i)) < need) {
-        if (gs_aborted(A)) return;
+    while (__any_sync(FULL, c.tag != tag)) {
         if (++spins > A.spin_limit) gs_abort(A);
+        if (gs_aborted(A)) break;
+        c = ld_entry(e);
     }
+    __threadfence();
+    return __shfl_sync(FULL, c.v, 0);
 }
-// Whole warp: every strip has done `need` steps (finished a sweep).
-__device__ __forceinline__ void gs_wait_all(const GsArgs &A, unsigned long long need) {
-    const int lane = threadIdx.x & 31;
-    for (int i = lane; i < A.sd.S; i += 32) {
-        unsigned long long seen = 0;
-        gs_wait(A, i, need, seen);
+// Whole warp, after its loads and stores: hands an entry on with them (release).
+__device__ __forceinline__ void gs_publish(Entry *e, double v, unsigned long long tag) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+        st_entry(e, v, tag);
     }
     __syncwarp();
-    __threadfence();
-}
-// Maximum change of sweep k over all strips (whole warp; order-free, and NaN
-// changes are ignored as std::max(maxDelta, NaN) ignores them).
-__device__ __forceinline__ double gs_sweep_max(const GsArgs &A, int k) {
-    const int lane = threadIdx.x & 31;
-    const double *slot = A.smax + (size_t)(k % kMaxSlots) * A.sd.S;
-    double m = 0.0;
-    for (int i = lane; i < A.sd.S; i += 32) m = smax(m, __ldcg(slot + i));
-    for (int o = 16; o > 0; o >>= 1) m = smax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    return m;
 }
 
+// -------------------------------------------------------------- division
+// x / d, rounded as the division instruction sequence rounds it, for a divisor
+// known in advance (four FP64 operations; the division takes nine times one, 562
+// cycles): q = x (zh + zl) with zh + zl = 1/d to twice the precision is within an
+// ulp of the quotient (N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in
+// advance", IEEE Trans. Computers 53, 2004), so its remainder is exact and
+// one step with zh = RN(1/d) rounds correctly (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34, 1990).  Holds where nothing underflows or overflows: 2^-100 <= d <= 2^100
+// and 2^-800 <= |x| < 2^800.  A zero divides to itself.
+struct Divisor {
+    double d, zh, zl;
+    __device__ __forceinline__ void set(double v) {
+        d = v;
+        zh = 1.0 / v;
+        zl = fma(-v, zh, 1.0) / v;
+    }
+};
+__device__ __forceinline__ unsigned biased_exponent(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
+__device__ __forceinline__ bool is_zero(double x) { return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u; }
+
 __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
-    extern __shared__ unsigned char spread[];  // reserves the SM; never touched
+    extern __shared__ unsigned char spread[];  // spreads the workers over the SMs; never touched
     (void)spread;
-    const int lane = threadIdx.x, s = blockIdx.x, S = A.sd.S;
-    const int w = A.sd.W, h = A.sd.H, D = A.sd.D;
+    const int lane = threadIdx.x, S = A.sd.S, s = blockIdx.x % S, j = blockIdx.x / S;
+    const int w = A.sd.W, h = A.sd.H, D = A.sd.D, B = A.L + 1;
     const int y = s * 32 + lane;
     const bool row = y < h;
     const int steps = w + 31;  // diagonals of one strip per sweep
     const double scale = A.scale;
     // diag of the reference: scale added once per existing neighbour, in order
-    const double d2 = scale + scale, d3 = d2 + scale, d4 = d3 + scale;
-    const double *rs = A.r + (size_t)s * D * 32 + lane;
-    const size_t own = (size_t)s * D * 32 + lane;
-    // lane 31 of strip s-1 at diagonal x + 31, lane 0 of strip s+1 at diagonal x
-    const size_t below = s > 0 ? ((size_t)(s - 1) * D + 31) * 32 + 31 : 0;
-    const size_t above = s + 1 < S ? (size_t)(s + 1) * D * 32 : 0;
-    const bool top_row = 32 * s + 31 < h - 1;  // lane 31 has an upper neighbour
+    Divisor d2, d3, d4;
+    d2.set(scale + scale);
+    d3.set((scale + scale) + scale);
+    d4.set(((scale + scale) + scale) + scale);
+    const unsigned ed = biased_exponent(d2.d);
+    const bool plain = ed < 1023u - 98u || ed > 1023u + 98u || !(scale > 0.0);  // divisors out of range: divide
+    const size_t own = (size_t)s * D * 32 + lane, cells = A.sd.total();
+    const bool below = s > 0, above = s + 1 < S;
+    // lane 0 reads the row below and hands the first row up's way; lane 31 the row above and the last row
+    const bool edge = (lane == 0 && below) || (lane == 31 && above);
     const int nsweeps = A.pinned >= 0 ? min(A.limit, A.pinned) : A.limit;
+    const int around = 2 + (y > 0) + (y < h - 1);  // neighbours of an inner column
 
-    int final_sweeps = -1, status = 2;
-    for (int it = 0; it < nsweeps; it++) {
-        if (A.pinned < 0 && it >= 2) {  // the convergence test of sweep it - 2
-            gs_wait_all(A, (unsigned long long)(it - 1) * steps);
-            if (gs_sweep_max(A, it - 2) < kGsTol) {
-                final_sweeps = it - 1;
-                status = 0;
-                break;
-            }
+    // the initial p is sweep -1, buffer 0
+    for (int d = j; d < steps && nsweeps > 0; d += A.J) {
+        const int x = d - lane;
+        if (!row || x < 0 || x >= w) continue;
+        const double v = A.p[own + (size_t)d * 32];
+        st_entry(A.ring + own + (size_t)d * 32, v, 1ull);
+        if (lane == 0 && below) st_entry(A.up + (size_t)s * w + x, fma(-scale, v, 0.0), 1ull);
+    }
+
+    int stop = 0;  // first converged sweep + 1
+    bool dead = false;
+    for (int k = j; k < nsweeps; k += A.J) {
+        if (k >= A.L) {
+            stop = (int)__double_as_longlong(gs_wait(A, A.verdict + (k - A.L) % B, (unsigned long long)(k - A.L) + 2));
+            if (stop != 0) break;
         }
-        if (__any_sync(0xffffffffu, gs_aborted(A))) break;
-        const double *oldb = A.buf[it & 1];
-        double *newb = A.buf[(it + 1) & 1];
-        const double *ps_old = oldb + own;
-        double *ps_new = newb + own;
-        const unsigned long long base = (unsigned long long)it * steps;
-        unsigned long long seen_below = 0, seen_above = 0;
-        double lmax = 0.0, prev = 0.0;
-        // operands of step d, loaded one step ahead (previous-sweep values of
-        // this strip's own cells)
-        double pold = 0.0, rr = 0.0, right = 0.0, up = 0.0;
+        dead = __any_sync(FULL, gs_aborted(A));
+        if (dead) break;
+        const unsigned long long tag = (unsigned long long)k + 2;  // this sweep's; the previous sweep's is tag - 1
+        const int b_old = k % B, b_new = (k + 1) % B;
+        const Entry *old_own = A.ring + (size_t)b_old * cells + own;
+        Entry *new_own = A.ring + (size_t)b_new * cells + own;
+        // the row that lane 0 / lane 31 reads: column d / d - 31 at step d
+        const Entry *halo = lane == 0 ? A.down + ((size_t)b_new * S + (below ? s - 1 : 0)) * w
+                                      : A.up + ((size_t)b_old * S + (above ? s + 1 : 0)) * w - 31;
+        Entry *hand = lane == 0 ? A.up + ((size_t)b_new * S + s) * w : A.down + ((size_t)b_new * S + s) * w - 31;
+        const bool gives = (lane == 0 && below) || (lane == 31 && above);
+        const unsigned long long halo_tag = lane == 0 ? tag : tag - 1;
+        unsigned long long mx = 0ull;  // bits of the largest change
+        double ql = 0.0;               // -scale * (this lane's previous value)
+        double pold = 0.0;             // the previous sweep's value of the cell
+        Entry R, Hw;                   // the previous sweep's right value; the edge lane's neighbour row
+        double rr = 0.0;
         auto load = [&](int d) {
             const int x = d - lane;
+            R.v = 0.0;
+            R.tag = tag - 1;
+            Hw.v = 0.0;
+            Hw.tag = halo_tag;
+            if (row && x + 1 >= 0 && x + 1 < w) R = ld_entry(old_own + (size_t)(d + 1) * 32);
             if (row && x >= 0 && x < w) {
-                const size_t k = (size_t)d * 32;
-                pold = ps_old[k];
-                rr = rs[k];
-                right = x < w - 1 ? ps_old[k + 32] : 0.0;
-                if (y < h - 1 && lane < 31) up = ps_old[k + 33];  // lane 31: the block's prefetch
+                rr = A.r[own + (size_t)d * 32];
+                if (edge) Hw = ld_entry(halo + d);
             }
         };
+        // the entries of step d, loaded again until they are there
+        auto settle = [&](int d) {
+            long long spins = 0;
+            while (__any_sync(FULL, R.tag != tag - 1 || Hw.tag != halo_tag)) {
+                if (++spins > A.spin_limit) gs_abort(A);
+                if ((spins & 15) == 0 || spins > A.spin_limit) {
+                    if (__any_sync(FULL, gs_aborted(A))) return false;
+                }
+                if (R.tag != tag - 1) R = ld_entry(old_own + (size_t)(d + 1) * 32);
+                if (Hw.tag != halo_tag) Hw = ld_entry(halo + d);
+            }
+            return true;
+        };
+        load(-1);
+        dead = !settle(-1);
+        if (dead) break;
+        pold = R.v;
         load(0);
-        for (int d0 = 0; d0 < steps; d0 += kGB) {
-            // Neighbour-strip values for the kGB steps of this block, fetched
-            // once per block by lanes 0..kGB-1: the lower row's values of this
-            // sweep (the strip below must have finished diagonal x + 31) and
-            // the upper row's values of the previous sweep (the strip above
-            // must have passed column x in that sweep; in sweep 0 they are the
-            // initial p, which no sweep 0 writes).
-            double dv = 0.0, uv = 0.0;
-            if (lane == 0) {
-                if (s > 0 && d0 < w) gs_wait(A, s - 1, base + min(d0 + kGB - 1, w - 1) + 32, seen_below);
-                const int xu_hi = min(d0 + kGB - 1 - 31, w - 1);
-                if (s + 1 < S && top_row && it > 0 && xu_hi >= 0)
-                    gs_wait(A, s + 1, base - steps + xu_hi + 1, seen_above);
-            }
-            __syncwarp();
-            __threadfence();
-            if (s > 0 && lane < kGB && d0 + lane < w) dv = __ldcg(newb + below + (size_t)(d0 + lane) * 32);
-            if (s + 1 < S && top_row && lane < kGB) {
-                const int xu = d0 + lane - 31;  // lane 31's column at step d0 + lane
-                if (xu >= 0 && xu < w) uv = __ldcg(oldb + above + (size_t)xu * 32);
-            }
-            if (__any_sync(0xffffffffu, gs_aborted(A))) break;
-            const int dend = min(d0 + kGB, steps);
-            for (int d = d0; d < dend; d++) {
-                const int x = d - lane;
-                const bool act = row && x >= 0 && x < w;
-                double down = __shfl_up_sync(0xffffffffu, prev, 1);
-                const double d_blk = __shfl_sync(0xffffffffu, dv, d - d0);
-                const double u_blk = __shfl_sync(0xffffffffu, uv, d - d0);
-                if (lane == 0) down = d_blk;
-                const double c_pold = pold, c_rr = rr, c_right = right;
-                const double c_up = lane == 31 ? u_blk : up;
-                if (d + 1 < steps) load(d + 1);
-                if (act) {
-                    const int nb = (x > 0) + (y > 0) + (x < w - 1) + (y < h - 1);
-                    const double diag = nb == 4 ? d4 : nb == 3 ? d3 : d2;
-                    double off = 0.0;
-                    if (x > 0) off -= scale * prev;
-                    if (y > 0) off -= scale * down;
-                    if (x < w - 1) off -= scale * c_right;
-                    if (y < h - 1) off -= scale * c_up;
-                    const double np = (c_rr - off) / diag;
-                    lmax = smax(lmax, fabs(c_pold - np));
-                    ps_new[(size_t)d * 32] = np;
-                    prev = np;
-                }
-                const bool last = d + 1 == steps;
-                if (last) {  // this strip's maximum change, before the sweep's last publication
-                    double m = lmax;
-                    for (int o = 16; o > 0; o >>= 1) m = smax(m, __shfl_xor_sync(0xffffffffu, m, o));
-                    if (lane == 0) *(volatile double *)(A.smax + (size_t)(it % kMaxSlots) * S + s) = m;
-                }
-                // publish every 4 diagonals and at the end of the sweep: a
-                // device-scope fence per diagonal would lengthen every step
-                // (every lane's stores fenced, since the strips above and below
-                // read this strip's last and first rows)
-                if (((d + 1) & 3) == 0 || last) {
-                    __threadfence();
-                    __syncwarp();
-                    if (lane == 0) *(volatile unsigned long long *)(A.prog + s) = base + d + 1;
-                }
-            }
-        }
-    }
-    const bool aborted = __any_sync(0xffffffffu, gs_aborted(A));
-    double maxDelta = 0.0;
-    if (final_sweeps < 0) {  // no early stop: the tests of the last sweeps are still open
-        final_sweeps = nsweeps;
-        if (nsweeps > 0 && !aborted) {
-            gs_wait_all(A, (unsigned long long)nsweeps * steps);
-            maxDelta = gs_sweep_max(A, nsweeps - 1);
-            status = 2;
-            if (A.pinned < 0) {
-                if (nsweeps >= 2 && gs_sweep_max(A, nsweeps - 2) < kGsTol) {
-                    final_sweeps = nsweeps - 1;
-                    maxDelta = gs_sweep_max(A, nsweeps - 2);
-                    status = 0;
-                } else if (maxDelta < kGsTol) {
-                    status = 0;
-                }
-            }
-        }
-    } else {
-        maxDelta = gs_sweep_max(A, final_sweeps - 1);
-    }
-    if (aborted) status = 2;
-    // the result is in buf[final & 1]; move it to p (this strip's own cells,
-    // after this strip's last sweep, so nothing of this strip writes them later)
-    if ((final_sweeps & 1) && !aborted) {
         for (int d = 0; d < steps; d++) {
+            dead = !settle(d);
+            if (dead) break;
             const int x = d - lane;
-            if (row && x >= 0 && x < w) A.buf[0][own + (size_t)d * 32] = A.buf[1][own + (size_t)d * 32];
+            const bool act = row && x >= 0 && x < w;
+            const double right = R.v, side = Hw.v, rhs = rr;
+            if (d + 1 < steps) load(d + 1);
+            // 0 - scale * value, as the reference's first subtraction leaves it; 0 for a
+            // neighbour that does not exist (subtracting scale * value and adding this
+            // give the same bits: the running sum is never -0)
+            const double qr = fma(-scale, right, 0.0);
+            double qd = __shfl_up_sync(FULL, ql, 1);
+            double qu = __shfl_down_sync(FULL, qr, 1);
+            if (lane == 0) qd = side;
+            if (lane == 31) qu = side;
+            const double num = rhs - (((ql + qd) + qr) + qu);
+            const int nb = around - (x == 0) - (x == w - 1);
+            const double dv = nb == 4 ? d4.d : nb == 3 ? d3.d : d2.d, zh = nb == 4 ? d4.zh : nb == 3 ? d3.zh : d2.zh,
+                         zl = nb == 4 ? d4.zl : nb == 3 ? d3.zl : d2.zl;
+            const double q = fma(num, zh, num * zl);
+            double np = fma(fma(-q, dv, num), zh, q);
+            if (is_zero(num)) np = num;
+            const bool range = biased_exponent(num) - (1023u - 800u) < 1600u || is_zero(num);
+            if (__any_sync(FULL, act && (plain || !range))) np = num / dv;
+            const unsigned long long c = (unsigned long long)__double_as_longlong(pold - np) & 0x7fffffffffffffffull;
+            const double qn = fma(-scale, np, 0.0);
+            // maxDelta = std::max(maxDelta, |change|): a NaN is skipped
+            if (act && c <= 0x7ff0000000000000ull && c > mx) mx = c;
+            if (act) {
+                st_entry(new_own + (size_t)d * 32, np, tag);
+                if (gives) st_entry(hand + d, qn, tag);
+            }
+            ql = act ? qn : 0.0;
+            pold = right;
+        }
+        if (dead) break;
+        // the sweep's largest change up to this strip; the last strip decides
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(FULL, mx, o);
+            mx = other > mx ? other : mx;
+        }
+        const int b = k % B;
+        if (below) {
+            const unsigned long long m = (unsigned long long)__double_as_longlong(gs_wait(A, A.change + (size_t)b * S + s - 1, tag));
+            mx = m > mx ? m : mx;
+        }
+        const double change = __longlong_as_double((long long)mx);
+        gs_publish(A.change + (size_t)b * S + s, change, tag);
+        if (!above) {
+            int v = k > 0 ? (int)__double_as_longlong(gs_wait(A, A.verdict + (k - 1) % B, tag - 1)) : 0;
+            if (v == 0 && A.pinned < 0 && change < kGsTol) v = k + 1;
+            gs_publish(A.verdict + b, __longlong_as_double((long long)v), tag);
         }
     }
-    if (s == 0 && lane == 0) {
+    int final_sweeps = nsweeps;
+    double maxDelta = 0.0;
+    if (nsweeps > 0 && !dead) {
+        if (stop == 0)
+            stop = (int)__double_as_longlong(gs_wait(A, A.verdict + (nsweeps - 1) % B, (unsigned long long)nsweeps + 1));
+        if (stop != 0) final_sweeps = stop;
+        maxDelta = gs_wait(A, A.change + (size_t)((final_sweeps - 1) % B) * S + S - 1, (unsigned long long)final_sweeps + 1);
+        dead = __any_sync(FULL, gs_aborted(A));
+    }
+    // the result is in buffer `final`; move it to p (this strip's own cells)
+    for (int d = j; d < steps && final_sweeps > 0 && !dead; d += A.J) {
+        const int x = d - lane;
+        if (row && x >= 0 && x < w)
+            A.p[own + (size_t)d * 32] = ld_entry(A.ring + (size_t)(final_sweeps % B) * cells + own + (size_t)d * 32).v;
+    }
+    if (s == 0 && j == 0 && lane == 0) {
         A.out->iterations = final_sweeps;
-        A.out->status = status;
+        A.out->status = stop != 0 && !dead ? 0 : 2;
         A.out->max_error = maxDelta;
         atomicAdd(A.iter_total, (unsigned long long)final_sweeps);
     }
 }
 
-constexpr int kSpreadBytes = 120 * 1024;  // one such CTA per SM
+size_t ring_words(const SDIdx &sd, int L) {
+    return (size_t)(L + 1) * (sd.total() + 2 * (size_t)sd.S * sd.W + sd.S + 1) * 2 + 2;
+}
+
+// Sweeps in flight (J) and the lead over the verdict (L).  A sweep follows the one
+// before it by about four steps (two of dependence, two of hand-over), so more than
+// steps / 4 sweeps of a strip do not help, nor more than four workers per SM: an
+// FP64 instruction takes 64 cycles of a warp with one worker on an SM and 76 with
+// four.  The verdict of a sweep comes after the last strip's last step (36 steps
+// per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes, with
+// fewer sweeps in flight.
+constexpr size_t kRingBytes = (size_t)256 << 20;
+void gs_plan(const SDIdx &sd, int sms, int *J, int *L) {
+    const long steps = sd.W + 31, until = steps + 36L * (sd.S - 1) + 8;
+    *J = (int)std::max(1L, std::min(4L * sms / sd.S, (steps + 3) / 4));
+    auto lead = [&](int n) { return (int)((n * until + steps - 1) / steps) + 2; };
+    *L = lead(*J);
+    while (*J > 1 && ring_words(sd, *L) * 8 > kRingBytes) *L = lead(--*J);
+    while (*L > 2 && ring_words(sd, *L) * 8 > kRingBytes) --*L;
+}
 
 }  // namespace
 
 int gs_max_rows() { return 32 * 4096; }
 
+size_t gs_words(const SDIdx &sd, int sms) {
+    int J, L;
+    gs_plan(sd, sms, &J, &L);
+    return ring_words(sd, L);
+}
+
 template <typename F>
 cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int limit, int pinned, cudaStream_t st,
                       long long wait_limit) {
-    const int strips = S.sd.S;
-    int dev = 0, sms = 0, per_sm = 0;
+    const SDIdx &sd = S.sd;
+    int dev = 0, sms = 0, per_sm = 0, optin = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    int smem = strips <= sms ? kSpreadBytes : 0;
+    GsArgs A;
+    gs_plan(sd, sms, &A.J, &A.L);
+    // as many workers per SM as it takes to seat them all, and no more
+    const int share = (sd.S * A.J + sms - 1) / sms;
+    const int smem = share > 4 ? 0 : std::min(optin, 220 * 1024 / share - 2048);
     if (smem) {
         e = cudaFuncSetAttribute(gs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs_kernel, 32, smem);
     if (e != cudaSuccess) return e;
-    if ((long)per_sm * sms < strips) return cudaErrorCooperativeLaunchTooLarge;
-    GsArgs A;
+    if ((long)per_sm * sms < (long)sd.S * A.J) A.J = (int)((long)per_sm * sms / sd.S);
+    if (A.J < 1) return cudaErrorCooperativeLaunchTooLarge;
     A.r = S.r;
-    A.buf[0] = S.p;
-    A.buf[1] = S.as;  // A*s is not used by the Gauss-Seidel steps
-    A.sd = S.sd;
+    A.p = S.p;
+    A.sd = sd;
     A.scale = dt / (S.rho_air * S.hx * S.hx);
     A.limit = limit;
     A.pinned = pinned;
@@ -280,12 +365,18 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     A.out = X.out;
     A.flags = S.flags;
     A.iter_total = X.iter_total;
-    A.prog = X.halo;      // strips + 1 words (halo holds 2 x S x D)
-    A.smax = X.partials;  // kMaxSlots x strips doubles (partials hold 4 x S x D / 16)
-    e = cudaMemsetAsync(A.prog, 0, sizeof(unsigned long long) * (strips + 1), st);
+    const size_t rows = (size_t)(A.L + 1) * sd.S * sd.W;
+    A.ring = (Entry *)X.gs;
+    A.down = A.ring + (size_t)(A.L + 1) * sd.total();
+    A.up = A.down + rows;
+    A.change = A.up + rows;
+    A.verdict = A.change + (size_t)(A.L + 1) * sd.S;
+    A.abort = (unsigned long long *)(A.verdict + A.L + 1);
+    // every tag back to `empty`: the whole of it, 24 MB at 128 x 128 (5 us)
+    e = cudaMemsetAsync(X.gs, 0, ring_words(sd, A.L) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     void *args[] = {&A};
-    return cudaLaunchCooperativeKernel((const void *)gs_kernel, dim3(strips), dim3(32), args, (size_t)smem, st);
+    return cudaLaunchCooperativeKernel((const void *)gs_kernel, dim3(sd.S * A.J), dim3(32), args, (size_t)smem, st);
 }
 
 template cudaError_t launch_gs<double>(const Scene<double> &, const PcgScratch &, double, int, int, cudaStream_t,

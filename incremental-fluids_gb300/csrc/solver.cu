@@ -562,6 +562,8 @@ class SolverImpl final : public SolverBase {
         scratch_.halo = c.take<unsigned long long>(base, pcg_halo_words(S_.sd));
         scratch_.out = c.take<PcgOut>(base, 2);
         scratch_.iter_total = c.take<unsigned long long>(base, 1);
+        scratch_.gs = nullptr;
+        if (prm_.variant <= IFL_GS) scratch_.gs = c.take<unsigned long long>(base, gs_words(S_.sd, max_blocks_ / 2));
     }
 
     int upload_bodies() {
