@@ -21,10 +21,13 @@
 // upper one from strip s + 1's worker of the previous sweep.
 //
 // Hand-over: sweep k writes ring buffer (k + 1) mod B.  An entry is 16 bytes, the
-// value and the sweep's tag, stored and loaded as one: a reader that finds its
-// tag has the value, with no counter or fence behind it.  A worker loads the
-// entries of a step one step ahead (a step is about the L2's latency) and loads
-// again those that had not come.
+// value and the value xor the sweep's tag.  A reader that finds its tag in the two
+// words has the value, with no counter or fence behind it, even if the words of
+// the entry before and of this one came mixed: with this sweep's check word the
+// tag comes out only for this sweep's value, and an older check word can only
+// give it by chance beside this sweep's value.  A worker loads the entries of a
+// step one step ahead (a step is about the L2's latency) and loads again those
+// that had not come.
 //
 // Convergence: the strips of a sweep pass its largest change on, the last strip
 // decides (`verdict`: the first converged sweep so far), and sweep k starts once
@@ -47,11 +50,13 @@ namespace ifl {
 namespace {
 
 constexpr double kGsTol = 1e-5;
+constexpr int kBlockWarps = 4;  // workers per block at most: one for each quarter of an SM
 constexpr unsigned FULL = 0xffffffffu;
 
+// A value and its check word, the value's bits xor the sweep's tag (sweep + 2; the
+// initial p counts as sweep -1; an empty entry has tag 0).
 struct __align__(16) Entry {
-    double v;
-    unsigned long long tag;  // sweep + 2 (the initial p counts as sweep -1); 0: empty
+    unsigned long long v, check;
 };
 
 struct GsArgs {
@@ -75,19 +80,18 @@ struct GsArgs {
 // ------------------------------------------------------------- hand-over
 __device__ __forceinline__ Entry ld_entry(const Entry *e) {
     Entry r;
-    unsigned long long v;
-    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
-                 : "=l"(v), "=l"(r.tag)
-                 : "l"(e)
-                 : "memory");
-    r.v = __longlong_as_double((long long)v);
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(r.v), "=l"(r.check) : "l"(e) : "memory");
     return r;
 }
-__device__ __forceinline__ void st_entry(Entry *e, double v, unsigned long long tag) {
-    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(e),
-                 "l"(__double_as_longlong(v)), "l"(tag)
+__device__ __forceinline__ void st_entry_if(Entry *e, double v, unsigned long long tag, bool p) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %3, 0;\n @q st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n}\n" ::"l"(e),
+                 "l"(b), "l"(b ^ tag), "r"((unsigned)p)
                  : "memory");
 }
+__device__ __forceinline__ void st_entry(Entry *e, double v, unsigned long long tag) { st_entry_if(e, v, tag, true); }
+__device__ __forceinline__ double value_of(const Entry &e) { return __longlong_as_double((long long)e.v); }
+__device__ __forceinline__ unsigned long long tag_of(const Entry &e) { return e.v ^ e.check; }
 __device__ __forceinline__ bool gs_aborted(const GsArgs &A) {
     return *(const volatile unsigned long long *)A.abort != 0ull;
 }
@@ -99,13 +103,13 @@ __device__ __forceinline__ void gs_abort(const GsArgs &A) {
 __device__ __forceinline__ double gs_wait(const GsArgs &A, const Entry *e, unsigned long long tag) {
     Entry c = ld_entry(e);
     long long spins = 0;
-    while (__any_sync(FULL, c.tag != tag)) {
+    while (__any_sync(FULL, tag_of(c) != tag)) {
         if (++spins > A.spin_limit) gs_abort(A);
         if (gs_aborted(A)) break;
         c = ld_entry(e);
     }
     __threadfence();
-    return __shfl_sync(FULL, c.v, 0);
+    return __shfl_sync(FULL, value_of(c), 0);
 }
 // Whole warp, after its loads and stores: hands an entry on with them (release).
 __device__ __forceinline__ void gs_publish(Entry *e, double v, unsigned long long tag) {
@@ -139,10 +143,15 @@ struct Divisor {
 __device__ __forceinline__ unsigned biased_exponent(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
 __device__ __forceinline__ bool is_zero(double x) { return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) == 0u; }
 
-__global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
+// Out of line: inline, the compiler divides first and selects after.
+__device__ __noinline__ double divide(double x, double d) { return x / d; }
+
+__global__ void __launch_bounds__(32 * kBlockWarps) gs_kernel(GsArgs A) {
     extern __shared__ unsigned char spread[];  // spreads the workers over the SMs; never touched
     (void)spread;
-    const int lane = threadIdx.x, S = A.sd.S, s = blockIdx.x % S, j = blockIdx.x / S;
+    const int lane = threadIdx.x & 31, worker = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int S = A.sd.S, s = worker % S, j = worker / S;
+    if (j >= A.J) return;
     const int w = A.sd.W, h = A.sd.H, D = A.sd.D, B = A.L + 1;
     const int y = s * 32 + lane;
     const bool row = y < h;
@@ -157,10 +166,15 @@ __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
     const bool plain = ed < 1023u - 98u || ed > 1023u + 98u || !(scale > 0.0);  // divisors out of range: divide
     const size_t own = (size_t)s * D * 32 + lane, cells = A.sd.total();
     const bool below = s > 0, above = s + 1 < S;
-    // lane 0 reads the row below and hands the first row up's way; lane 31 the row above and the last row
+    // lane 0 reads the last row of the strip below and hands its own up, lane 31 the
+    // first row of the strip above and hands its own down
     const bool edge = (lane == 0 && below) || (lane == 31 && above);
     const int nsweeps = A.pinned >= 0 ? min(A.limit, A.pinned) : A.limit;
-    const int around = 2 + (y > 0) + (y < h - 1);  // neighbours of an inner column
+    // divisors of an inner column and of the first and last one, which in a grid of
+    // one column are the same one
+    const int around = 2 + (y > 0) + (y < h - 1), fewer = around - (w > 1 ? 1 : 2);
+    const Divisor inner = around == 4 ? d4 : around == 3 ? d3 : d2, at_side = fewer == 4 ? d4 : fewer == 3 ? d3 : d2;
+    const unsigned columns = row ? (unsigned)w : 0u;
 
     // the initial p is sweep -1, buffer 0
     for (int d = j; d < steps && nsweeps > 0; d += A.J) {
@@ -182,56 +196,53 @@ __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
         if (dead) break;
         const unsigned long long tag = (unsigned long long)k + 2;  // this sweep's; the previous sweep's is tag - 1
         const int b_old = k % B, b_new = (k + 1) % B;
-        const Entry *old_own = A.ring + (size_t)b_old * cells + own;
-        Entry *new_own = A.ring + (size_t)b_new * cells + own;
-        // the row that lane 0 / lane 31 reads: column d / d - 31 at step d
-        const Entry *halo = lane == 0 ? A.down + ((size_t)b_new * S + (below ? s - 1 : 0)) * w
-                                      : A.up + ((size_t)b_old * S + (above ? s + 1 : 0)) * w - 31;
+        // Operands of a step: the previous sweep's right value, the edge lane's neighbour
+        // row and the right-hand side.  Lanes at a column outside the grid load what lies
+        // there and ignore it.  Two sets in turn, pointers that move on by two steps.
+        struct Operands {
+            Entry right, side;
+            double rr;
+        } two[2] = {};
+        const Entry *old_right = A.ring + (size_t)b_old * cells + own + 32;  // column of the step + 1
+        // the row that lane 0 / lane 31 reads (column d / d - 31 at step d), and hands on
+        const Entry *halo = lane == 0 && below  ? A.down + ((size_t)b_new * S + s - 1) * w
+                            : lane == 31 && above ? A.up + ((size_t)b_old * S + s + 1) * w - 31
+                                                  : A.ring + 1;
         Entry *hand = lane == 0 ? A.up + ((size_t)b_new * S + s) * w : A.down + ((size_t)b_new * S + s) * w - 31;
-        const bool gives = (lane == 0 && below) || (lane == 31 && above);
+        Entry *result = A.ring + (size_t)b_new * cells + own;
+        const double *rhs = A.r + own;
         const unsigned long long halo_tag = lane == 0 ? tag : tag - 1;
         unsigned long long mx = 0ull;  // bits of the largest change
         double ql = 0.0;               // -scale * (this lane's previous value)
         double pold = 0.0;             // the previous sweep's value of the cell
-        Entry R, Hw;                   // the previous sweep's right value; the edge lane's neighbour row
-        double rr = 0.0;
-        auto load = [&](int d) {
-            const int x = d - lane;
-            R.v = 0.0;
-            R.tag = tag - 1;
-            Hw.v = 0.0;
-            Hw.tag = halo_tag;
-            if (row && x + 1 >= 0 && x + 1 < w) R = ld_entry(old_own + (size_t)(d + 1) * 32);
-            if (row && x >= 0 && x < w) {
-                rr = A.r[own + (size_t)d * 32];
-                if (edge) Hw = ld_entry(halo + d);
-            }
+        int x = -lane;                 // column of an even step
+        // operands of step u after the even step that the pointers are at
+        auto load = [&](Operands &o, int u) {
+            o.right = ld_entry(old_right + u * 32);
+            o.side = ld_entry(halo + u);
+            o.rr = *((unsigned)(x + u) < columns ? rhs + u * 32 : A.r + own + (size_t)lane * 32);
         };
-        // the entries of step d, loaded again until they are there
-        auto settle = [&](int d) {
+        // the entries of that step, loaded again until they are there
+        auto settle = [&](Operands &o, int u) {
+            const bool need = (unsigned)(x + u + 1) < columns, needs = edge && (unsigned)(x + u) < columns;
             long long spins = 0;
-            while (__any_sync(FULL, R.tag != tag - 1 || Hw.tag != halo_tag)) {
+            while (__any_sync(FULL, (need && tag_of(o.right) != tag - 1) || (needs && tag_of(o.side) != halo_tag))) {
                 if (++spins > A.spin_limit) gs_abort(A);
                 if ((spins & 15) == 0 || spins > A.spin_limit) {
                     if (__any_sync(FULL, gs_aborted(A))) return false;
                 }
-                if (R.tag != tag - 1) R = ld_entry(old_own + (size_t)(d + 1) * 32);
-                if (Hw.tag != halo_tag) Hw = ld_entry(halo + d);
+                if (need && tag_of(o.right) != tag - 1) o.right = ld_entry(old_right + u * 32);
+                if (needs && tag_of(o.side) != halo_tag) o.side = ld_entry(halo + u);
             }
             return true;
         };
-        load(-1);
-        dead = !settle(-1);
-        if (dead) break;
-        pold = R.v;
-        load(0);
-        for (int d = 0; d < steps; d++) {
-            dead = !settle(d);
-            if (dead) break;
-            const int x = d - lane;
-            const bool act = row && x >= 0 && x < w;
-            const double right = R.v, side = Hw.v, rhs = rr;
-            if (d + 1 < steps) load(d + 1);
+        auto step = [&](Operands &o, Operands &next, int u) {
+            if (!settle(o, u)) return false;
+            const int col = x + u;
+            const bool act = (unsigned)col < columns;
+            const double right = (unsigned)(col + 1) < columns ? value_of(o.right) : 0.0;
+            const double side = act && edge ? value_of(o.side) : 0.0, rr = o.rr;
+            load(next, u + 1);
             // 0 - scale * value, as the reference's first subtraction leaves it; 0 for a
             // neighbour that does not exist (subtracting scale * value and adding this
             // give the same bits: the running sum is never -0)
@@ -240,25 +251,39 @@ __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
             double qu = __shfl_down_sync(FULL, qr, 1);
             if (lane == 0) qd = side;
             if (lane == 31) qu = side;
-            const double num = rhs - (((ql + qd) + qr) + qu);
-            const int nb = around - (x == 0) - (x == w - 1);
-            const double dv = nb == 4 ? d4.d : nb == 3 ? d3.d : d2.d, zh = nb == 4 ? d4.zh : nb == 3 ? d3.zh : d2.zh,
-                         zl = nb == 4 ? d4.zl : nb == 3 ? d3.zl : d2.zl;
+            const double num = rr - (((ql + qd) + qr) + qu);
+            const bool side_col = col == 0 || col == w - 1;
+            const double dv = side_col ? at_side.d : inner.d, zh = side_col ? at_side.zh : inner.zh,
+                         zl = side_col ? at_side.zl : inner.zl;
             const double q = fma(num, zh, num * zl);
             double np = fma(fma(-q, dv, num), zh, q);
             if (is_zero(num)) np = num;
             const bool range = biased_exponent(num) - (1023u - 800u) < 1600u || is_zero(num);
-            if (__any_sync(FULL, act && (plain || !range))) np = num / dv;
+            if (__any_sync(FULL, act && (plain || !range))) np = divide(num, dv);
             const unsigned long long c = (unsigned long long)__double_as_longlong(pold - np) & 0x7fffffffffffffffull;
             const double qn = fma(-scale, np, 0.0);
             // maxDelta = std::max(maxDelta, |change|): a NaN is skipped
             if (act && c <= 0x7ff0000000000000ull && c > mx) mx = c;
-            if (act) {
-                st_entry(new_own + (size_t)d * 32, np, tag);
-                if (gives) st_entry(hand + d, qn, tag);
-            }
+            st_entry_if(result + u * 32, np, tag, act);
+            st_entry_if(hand + u, qn, tag, act && edge);
             ql = act ? qn : 0.0;
             pold = right;
+            return true;
+        };
+        two[1].right = ld_entry(old_right - 32);  // column 0, lane 0
+        dead = !settle(two[1], -1);
+        if (dead) break;
+        pold = lane == 0 && row ? value_of(two[1].right) : 0.0;
+        load(two[0], 0);
+        for (int d = 0; d < steps && !dead; d += 2) {
+            dead = !step(two[0], two[1], 0);
+            if (!dead && d + 1 < steps) dead = !step(two[1], two[0], 1);
+            old_right += 64;
+            halo += 2;
+            rhs += 64;
+            result += 64;
+            hand += 2;
+            x += 2;
         }
         if (dead) break;
         // the sweep's largest change up to this strip; the last strip decides
@@ -292,7 +317,7 @@ __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
     for (int d = j; d < steps && final_sweeps > 0 && !dead; d += A.J) {
         const int x = d - lane;
         if (row && x >= 0 && x < w)
-            A.p[own + (size_t)d * 32] = ld_entry(A.ring + (size_t)(final_sweeps % B) * cells + own + (size_t)d * 32).v;
+            A.p[own + (size_t)d * 32] = value_of(ld_entry(A.ring + (size_t)(final_sweeps % B) * cells + own + (size_t)d * 32));
     }
     if (s == 0 && j == 0 && lane == 0) {
         A.out->iterations = final_sweeps;
@@ -303,20 +328,23 @@ __global__ void __launch_bounds__(32) gs_kernel(GsArgs A) {
 }
 
 size_t ring_words(const SDIdx &sd, int L) {
-    return (size_t)(L + 1) * (sd.total() + 2 * (size_t)sd.S * sd.W + sd.S + 1) * 2 + 2;
+    // (64 entries more: loads beyond a row's or a strip's last column, which are ignored)
+    return ((size_t)(L + 1) * (sd.total() + 2 * (size_t)sd.S * sd.W + sd.S + 1) + 64) * 2 + 2;
 }
 
 // Sweeps in flight (J) and the lead over the verdict (L).  A sweep follows the one
-// before it by about four steps (two of dependence, two of hand-over), so more than
-// steps / 4 sweeps of a strip do not help, nor more than four workers per SM: an
-// FP64 instruction takes 64 cycles of a warp with one worker on an SM and 76 with
-// four.  The verdict of a sweep comes after the last strip's last step (36 steps
-// per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes, with
-// fewer sweeps in flight.
-constexpr size_t kRingBytes = (size_t)256 << 20;
+// before it by three to four steps (one of dependence, one of loading ahead, the
+// hand-over): at 128 x 128, with 159 steps of about 1500 cycles, 600 sweeps took
+// 4.4 million cycles with 40 sweeps in flight per strip, 3.9 with 56, 3.5 with 76
+// and 3.2 with 120, so half as many as steps; and no more than four workers per SM:
+// an FP64 instruction takes 64 cycles of a warp with one worker on an SM and 76
+// with four.  The verdict of a sweep comes after the last strip's last step (36
+// steps per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes,
+// with fewer sweeps in flight.
+constexpr size_t kRingBytes = (size_t)512 << 20;
 void gs_plan(const SDIdx &sd, int sms, int *J, int *L) {
     const long steps = sd.W + 31, until = steps + 36L * (sd.S - 1) + 8;
-    *J = (int)std::max(1L, std::min(4L * sms / sd.S, (steps + 3) / 4));
+    *J = (int)std::max(1L, std::min(4L * sms / sd.S, (steps + 1) / 2));
     auto lead = [&](int n) { return (int)((n * until + steps - 1) / steps) + 2; };
     *L = lead(*J);
     while (*J > 1 && ring_words(sd, *L) * 8 > kRingBytes) *L = lead(--*J);
@@ -344,16 +372,18 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     if (e != cudaSuccess) return e;
     GsArgs A;
     gs_plan(sd, sms, &A.J, &A.L);
-    // as many workers per SM as it takes to seat them all, and no more
+    // blocks of as many workers as seat them all with one block per SM, up to one
+    // for each of its quarters (single-warp blocks share a quarter: 1.6 times the
+    // time per step with two workers on an SM)
     const int share = (sd.S * A.J + sms - 1) / sms;
-    const int smem = share > 4 ? 0 : std::min(optin, 220 * 1024 / share - 2048);
+    const int warps = std::min(share, kBlockWarps), smem = share > kBlockWarps ? 0 : std::min(optin, 120 * 1024);
     if (smem) {
         e = cudaFuncSetAttribute(gs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs_kernel, 32, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs_kernel, 32 * warps, smem);
     if (e != cudaSuccess) return e;
-    if ((long)per_sm * sms < (long)sd.S * A.J) A.J = (int)((long)per_sm * sms / sd.S);
+    if ((long)per_sm * sms * warps < (long)sd.S * A.J) A.J = (int)((long)per_sm * sms * warps / sd.S);
     if (A.J < 1) return cudaErrorCooperativeLaunchTooLarge;
     A.r = S.r;
     A.p = S.p;
@@ -371,12 +401,12 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     A.up = A.down + rows;
     A.change = A.up + rows;
     A.verdict = A.change + (size_t)(A.L + 1) * sd.S;
-    A.abort = (unsigned long long *)(A.verdict + A.L + 1);
-    // every tag back to `empty`: the whole of it, 24 MB at 128 x 128 (5 us)
+    A.abort = (unsigned long long *)(A.verdict + A.L + 1 + 64);
+    // every tag back to `empty`: the whole of it, 47 MB at 128 x 128 (10 us)
     e = cudaMemsetAsync(X.gs, 0, ring_words(sd, A.L) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     void *args[] = {&A};
-    return cudaLaunchCooperativeKernel((const void *)gs_kernel, dim3(sd.S * A.J), dim3(32), args, (size_t)smem, st);
+    return cudaLaunchCooperativeKernel((const void *)gs_kernel, dim3((sd.S * A.J + warps - 1) / warps), dim3(32 * warps), args, (size_t)smem, st);
 }
 
 template cudaError_t launch_gs<double>(const Scene<double> &, const PcgScratch &, double, int, int, cudaStream_t,
