@@ -88,7 +88,7 @@ __device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
 // The preparer's part of one backward strip: y becomes dd y, and sigma = z.r =
 // sum of dd y^2 (see pcg_job) is added up: sums of two fused FP32 products per
 // row of the tiles and step, over a block, then FP64.
-__device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<float> &ring) {
+__device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<float> &ring, bool in) {
     Ring<float> R = ring;
     const Flags flags = A.fl;
     const int lane = threadIdx.x & 31, nblk = A.sd.D / kT;
@@ -107,7 +107,10 @@ __device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<
             qs = fma4(q1, y1, fma4(q0, y0, qs));
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(R.bar(Ring<float>::READY, R.st));
+        if (lane == 0) {
+            mbar_arrive(R.bar(Ring<float>::PREPARED, R.st));
+            if (!in) mbar_arrive(R.bar(Ring<float>::READY, R.st));  // else the loader's, with the halo words
+        }
         qq += to_f64((qs.x + qs.y) + (qs.z + qs.w));
         R.next();
     }
@@ -121,9 +124,9 @@ __device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<
 
 // One strip of a sweep.  At step t lane l works on tile diagonal t (backward:
 // D-1-t), one tile behind lane l-1 (l+1), whose boundary row arrives by two
-// shuffles; lane 0 (31) takes it from the block's halo words (IN: whether the
-// strip has a neighbour to take from), and lane 31 (0) hands this strip's on
-// through `out` as soon as it is formed: a word of two floats per tile column X,
+// shuffles; lane 0 (31) has its neighbour strip's folded into its operands
+// (put_halo), and lane 31 (0) hands this strip's on through `out` as soon as it is
+// formed: a word of two floats per tile column X,
 // at X + 32 of the row (forward; the lane starts at X = -31) or at X (backward).
 // Words of columns that no step waits for are written along and never read.
 // Functions of their own: inlined, the solve's registers spill into their steps.
@@ -136,7 +139,7 @@ __device__ __noinline__ void sweep_strip(const PcgArgs<float> &A, int s, Ring<fl
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     const int nblk = sd.D / kT;
-    const bool edge = lane == (BWD ? 31 : 0), hands = out.valid && lane == (BWD ? 0 : 31);
+    const bool hands = out.valid && lane == (BWD ? 0 : 31);
     float4 *zp = (float4 *)A.z + ((size_t)s * sd.D + (BWD ? sd.D - kT : 0)) * 64 + lane;
     unsigned long long *op = out.row + (BWD ? sd.D - 1 : 1);  // word of this lane's first step
     float4 o0[kDepth][3], o1[kDepth][3];  // operands of kDepth steps, columns 0 and 1
@@ -155,22 +158,19 @@ __device__ __noinline__ void sweep_strip(const PcgArgs<float> &A, int s, Ring<fl
     };
     float4 n = zero4();        // the previous tile's column next to this one
     float g0 = 0.f, g1 = 0.f;  // boundary row of the previous lane (columns 0, 1)
+    bool next_ready = false;
     for (int blk = 0; blk < nblk; blk++) {
-        ring_wait(R, R.bar(Ring<float>::READY, R.st), R.parity, flags);
+        ring_wait_lane(R, R.bar(Ring<float>::READY, R.st), R.parity, next_ready, flags);
         g = g_smem + R.stage(R.st) + lane * 16;
 #pragma unroll
         for (int j = 0; j < kDepth; j++) load(j);
-        float2 halo[kT];  // all of the block's halo words at once: no step waits for its own
-        if constexpr (IN) {
-            const float2 *h = (const float2 *)(g - lane * 16 + kHaloAt<float>);
-#pragma unroll
-            for (int j = 0; j < kT; j++) halo[j] = h[j];
-        }
 #pragma unroll
         for (int j = 0; j < kT; j++) {
-            if constexpr (IN) {
-                g0 = edge ? halo[j].x : g0;
-                g1 = edge ? halo[j].y : g1;
+            // asked for two steps ahead: waiting for a barrier that is complete takes 90 cycles too
+            if (j == kT - 2) {
+                Ring<float> N = R;
+                N.next();
+                next_ready = mbar_test(N.bar(Ring<float>::READY, N.st), N.parity);
             }
             const int i = j % kDepth;
             float4 v0, v1;

@@ -38,7 +38,7 @@ __device__ __forceinline__ double madd(double a, double b, double c) {
 
 // The preparer's part of one backward strip: y becomes dd y, and sigma = z.r =
 // sum of dd y^2 (see pcg_job) is added up.
-__device__ __noinline__ void prepare_strip(const PcgArgs<double> &A, int s, Ring<double> &ring) {
+__device__ __noinline__ void prepare_strip(const PcgArgs<double> &A, int s, Ring<double> &ring, bool in) {
     Ring<double> R = ring;
     const Flags flags = A.fl;
     const int lane = threadIdx.x & 31, nblk = A.sd.D / kT;
@@ -54,7 +54,10 @@ __device__ __noinline__ void prepare_strip(const PcgArgs<double> &A, int s, Ring
             qq = fma(q, y0, qq);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(R.bar(Ring<double>::READY, R.st));
+        if (lane == 0) {
+            mbar_arrive(R.bar(Ring<double>::PREPARED, R.st));
+            if (!in) mbar_arrive(R.bar(Ring<double>::READY, R.st));  // else the loader's, with the halo words
+        }
         R.next();
     }
     qq = warp_sum(qq);
@@ -86,8 +89,9 @@ __device__ __noinline__ void sweep_strip(const PcgArgs<double> &A, int s, Ring<d
     double *zp = A.z + ((size_t)s * sd.D + (BWD ? sd.D - kT : 0)) * 32 + lane;
     unsigned long long *op = out.row + (BWD ? sd.D - 1 : 1);  // word of this lane's first step
     double n = 0.0, h = 0.0;  // this lane's previous value, the previous lane's
+    bool next_ready = false;
     for (int blk = 0; blk < nblk; blk++) {
-        ring_wait(R, R.bar(Ring<double>::READY, R.st), R.parity, flags);
+        ring_wait_lane(R, R.bar(Ring<double>::READY, R.st), R.parity, next_ready, flags);
         const char *g = g_smem + R.stage(R.st);
         double o[kT][kO], halo[kT];
 #pragma unroll
@@ -107,6 +111,11 @@ __device__ __noinline__ void sweep_strip(const PcgArgs<double> &A, int s, Ring<d
         }
 #pragma unroll
         for (int j = 0; j < kT; j++) {
+            if (j == kT - 2) {
+                Ring<double> N = R;
+                N.next();
+                next_ready = mbar_test(N.bar(Ring<double>::READY, N.st), N.parity);
+            }
             const double t = REF ? o[j][0] - o[j][1] * n : fma(o[j][1], n, o[j][0]);
             if constexpr (IN) h = edge ? halo[j] : h;
             if constexpr (REF) n = (t - o[j][2] * h) * o[j][3];

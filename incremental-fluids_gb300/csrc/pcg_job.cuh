@@ -18,7 +18,7 @@ __host__ __device__ __forceinline__ unsigned ring_offset(int K, int D) {
 }
 
 // Sweep of all strips of this block: warps 0..K-1 sweep, K..2K-1 load for them,
-// 2K..3K-1 prepare.  The team's T.size*K sweeping warps take the strips
+// 2K..3K-1 prepare, 3K..4K-1 take the halo words.  The team's T.size*K sweeping warps take the strips
 // round-robin: warp `base` sweeps strips base, base + P, base + 2P,
 // ... (P = T.size*K), in increasing order for the forward solve and in
 // decreasing order for the backward solve, so that every strip waits only on a
@@ -58,13 +58,15 @@ __device__ void sweep_all(const PcgArgs<F> &A, const Team &T, Ring<F> &R) {
             if (s > 0) out = (one_round && w > 0) ? smem_row(w - 1) : glob_row(down + (size_t)s * row);
         }
         if (role == 0) {
-            if (in.valid) sweep_strip<REF, BWD, true>(A, s, R, out);
+            // FP32: the halo words are folded into the operands (put_halo)
+            if (sizeof(F) == 8 && in.valid) sweep_strip<REF, BWD, sizeof(F) == 8>(A, s, R, out);
             else sweep_strip<REF, BWD, false>(A, s, R, out);
         } else if (role == 1) {
-            if (in.valid) load_strip<F, REF, BWD, true>(A, s, R, in);
-            else load_strip<F, REF, BWD, false>(A, s, R, in);
-        } else if (BWD && !REF) {
-            prepare_strip(A, s, R);
+            load_strip<F, REF, BWD>(A, s, R, in.valid);
+        } else if (role == 2 && BWD && !REF) {
+            prepare_strip(A, s, R, in.valid);
+        } else if (role == 3 && in.valid) {
+            take_strip<F, REF, BWD>(A, R, in);
         } else {
             R.skip(sd.D / Lay<F>::kSteps);
         }
@@ -207,7 +209,8 @@ __device__ void ring_init(Ring<F> &R, int K, int stages) {
     if (lane == 0 && warp < K) {
         for (int k = 0; k < stages; k++) {
             mbar_init(R.bar(Ring<F>::COPIED, k), 1);
-            mbar_init(R.bar(Ring<F>::READY, k), 2);
+            mbar_init(R.bar(Ring<F>::PREPARED, k), 1);
+            mbar_init(R.bar(Ring<F>::READY, k), 1);
             mbar_init(R.bar(Ring<F>::FREE, k), 1);
         }
         fence_mbar_init();
@@ -254,13 +257,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     }
 }
 
-constexpr int kSingleThreads = 256, kSingleStages = 6;
+constexpr int kSingleThreads = 256, kSingleStages = 8;
 
 template <typename F>
 size_t pcg_smem(int K, int D, int stages) { return ring_offset(K, D) + (size_t)K * stages * kStageBytes<F>; }
 
 // What a shape {threads, strips per block, stages} comes to: at least a strip's
-// three warps per strip, as many strips and stages as threads and shared memory
+// four warps per strip, as many strips and stages as threads and shared memory
 // allow (smem: bytes of a block).
 template <typename F>
 void pcg_shape(int threads, int D, size_t smem_max, int *block, int *K, int *stages) {

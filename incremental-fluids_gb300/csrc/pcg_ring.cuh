@@ -46,7 +46,7 @@ template <typename F> constexpr unsigned kHaloAt = 4u * kVecBytes<F>;       // i
 template <typename F> constexpr unsigned kStageBytes = kHaloAt<F> + 128u;   // a ring stage
 constexpr int kMaxStages = 8;
 constexpr int kMaxThreads = 384;  // of a block (168 registers per thread)
-constexpr int kRoles = 3;   // warps that work on one strip: sweep, load, prepare
+constexpr int kRoles = 4;   // warps that work on one strip: sweep, load, prepare, take
 constexpr int kSums = 16;   // partial sums of a reduction (see total_of)
 
 // ---------------------------------------------------------- conversions
@@ -103,14 +103,15 @@ __device__ __forceinline__ F *coef(const PcgArgs<F> &A, size_t k, int arr) {
 // A strip's ring in shared memory: `stages` buffers of kSteps diagonals,
 //   [r][al, bd per diagonal] (forward) or [y][dd, a, b per diagonal] (backward),
 //   then the halo words of the block's steps.
-// Three warps share it, each with its own running position (stage, mbarrier
+// Four warps share it, each with its own running position (stage, mbarrier
 // parity):
-//  * the loader waits for a free stage, starts two bulk copies into it, takes the
-//    block's halo words as they arrive and puts them behind the operands;
-//  * the preparer (backward, L D L^T form) waits for the copies, multiplies y by dd in place and
-//    adds up sigma;
-//  * the sweeping warp waits for both (`ready`), stores its results and hands its
-//    boundary row on, and frees the stage.
+//  * the loader waits for a free stage and starts two bulk copies into it;
+//  * the preparer (backward, L D L^T form) waits for the copies, multiplies y by
+//    dd in place and adds up sigma;
+//  * the taker (where the strip has a neighbour to take from) puts the halo words
+//    to the operands as they arrive;
+//  * the sweeping warp waits until all that is done (`ready`), stores its results
+//    and hands its boundary row on, and frees the stage.
 // Every wait is bounded.  A timeout elsewhere in the launch does not shorten the
 // mbarrier waits: the copies were issued from this GPU's memory and complete,
 // and the loader's halo polls give up by themselves, so a timed-out sweep still
@@ -124,7 +125,7 @@ struct Ring {
     int stages, st;
     unsigned parity;
     bool dead;
-    enum { COPIED = 0, READY = 1, FREE = 2, KINDS = 3 };
+    enum { COPIED = 0, PREPARED = 1, READY = 2, FREE = 3, KINDS = 4 };
     __device__ __forceinline__ uint64_t *bar(int kind, int at) const {
         return (uint64_t *)(g_smem + bars) + kind * kMaxStages + at;
     }
@@ -151,6 +152,18 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
                  : "memory");
     return ok != 0;
 }
+// This lane: phase `parity` of a barrier, tested earlier with the result `done`.
+template <typename F>
+__device__ __forceinline__ void ring_wait_lane(Ring<F> &R, uint64_t *bar, unsigned parity, bool done, const Flags &flags) {
+    if (done) return;
+    long long n = 0;
+    while (!R.dead && !mbar_try_wait(bar, parity)) {
+        if (++n > kMbarWaitLimit + flags.limit) {
+            set_timeout(flags);
+            R.dead = true;
+        }
+    }
+}
 // Whole warp: the phase `parity` of a barrier.
 template <typename F>
 __device__ __forceinline__ void ring_wait(Ring<F> &R, uint64_t *bar, unsigned parity, const Flags &flags) {
@@ -165,89 +178,120 @@ __device__ __forceinline__ void ring_wait(Ring<F> &R, uint64_t *bar, unsigned pa
     }
 }
 
-// The loader's part of one strip.  Halo words: at step t the waiting lane needs
-// the boundary value of one column (a double, or the two floats of a tile's
-// columns) in one 8-byte word of the neighbour's row (t <= D - 32; beyond, the
-// coefficient is zero).  Lane i polls the word of the i-th step from the first block that waits
-// for words, so one round of loads (about 700 cycles) serves up to eight blocks.
-template <typename F, bool REF, bool BWD, bool IN>
-__device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &ring, const Chan in) {
+// The halo word of step j of a block, into its stage.  FP64: behind the operands,
+// as the reference's order of operations is kept (k_pcg64.cu).  FP32: folded into
+// the edge lane's operands, r (or dd y) += b * word, and b = 0, so that the sweep
+// needs no word of its own (reading and selecting it took 6 cycles per step).
+template <typename F, bool BWD>
+__device__ __forceinline__ void put_halo(char *stage, int j, unsigned long long w) {
+    if constexpr (sizeof(F) == 8) {
+        *(volatile unsigned long long *)(stage + kHaloAt<F> + 8 * j) = w;
+    } else {
+        constexpr int kC = kCoefs<false, BWD>, kEdge = BWD ? 31 * 16 + 12 : 0;  // element w of lane 31, x of lane 0
+        const int jj = BWD ? Lay<F>::kSteps - 1 - j : j;
+        float *r = (float *)(stage + jj * 1024 + kEdge);
+        float *b = (float *)(stage + kVecBytes<F> + (jj * kC + kC - 1) * 1024 + kEdge);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {  // the tile's columns, 512 bytes apart
+            r[128 * e] = fmaf(b[128 * e], __uint_as_float((unsigned)(w >> (32 * e))), r[128 * e]);
+            b[128 * e] = 0.f;
+        }
+    }
+}
+
+// The loader's part of one strip: the bulk copies, as stages become free.
+template <typename F, bool REF, bool BWD>
+__device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &ring, bool in) {
     constexpr int kC = kCoefs<REF, BWD>;  // coefficient arrays
     constexpr bool kPrepared = BWD && !REF;  // the preparer stands between the copies and the sweep
     constexpr int kT = Lay<F>::kSteps, kCells = Lay<F>::kCells;
     constexpr unsigned kVec = kVecBytes<F>;
     Ring<F> R = ring;
     const Flags flags = A.fl;
-    const int lane = threadIdx.x & 31;
     const int D = A.sd.D, nblk = D / kT;
     const size_t row0 = (size_t)s * D + (BWD ? D - kT : 0);  // first diagonal of the first block
     const F *vec = (BWD ? A.z : A.rf) + row0 * kCells;
     const F *cf = coef<REF, BWD>(A, row0 * kCells, 0);
     fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
-    int issued = 0, ready = 0;   // blocks whose copies are started, whose halo words are in place
-    int rst = R.st;              // stage of block `ready`
+    for (int blk = 0; blk < nblk; blk++) {
+        ring_wait(R, R.bar(Ring<F>::FREE, R.st), R.parity ^ 1u, flags);
+        if ((threadIdx.x & 31) == 0) {
+            // without preparer and halo words the sweeping warp itself waits for the
+            // copies; the barriers that nobody waits for keep pace
+            uint64_t *ready = R.bar(Ring<F>::READY, R.st), *copied = R.bar(Ring<F>::COPIED, R.st);
+            uint64_t *tx = kPrepared || in ? copied : ready;
+            char *dst = g_smem + R.stage(R.st);
+            fence_proxy_async_shared();  // what was written into the stage by hand -> bulk copies
+            mbar_expect_tx(tx, (1u + kC) * kVec);
+            bulk_g2s(dst, vec, kVec, tx);
+            bulk_g2s(dst + kVec, cf, kC * kVec, tx);
+            if (!kPrepared) mbar_arrive(R.bar(Ring<F>::PREPARED, R.st));
+            if (!kPrepared && !in) mbar_arrive(copied);
+        }
+        vec += BWD ? -kT * kCells : kT * kCells;
+        cf += (BWD ? -kT * kCells : kT * kCells) * kC;
+        R.next();
+    }
+    ring = R;
+    __syncwarp();
+}
+
+// The taker's part of one strip: the halo words.  At step t the edge lane needs the
+// boundary value of one column (a double, or the two floats of a tile's columns)
+// in one 8-byte word of the neighbour's row (t <= D - 32; beyond, the coefficient
+// is zero).  Lane i polls the word of the i-th step from the first block that
+// waits for words, so one round of loads (about 700 cycles) serves up to eight
+// blocks.  A warp of its own: with the copies in the same loop a round served
+// little more than a block in the time that the sweep takes for one (640 cycles),
+// and every strip behind another fell back further at every block.
+template <typename F, bool REF, bool BWD>
+__device__ __noinline__ void take_strip(const PcgArgs<F> &A, Ring<F> &ring, const Chan in) {
+    constexpr bool kPrepared = BWD && !REF;
+    constexpr int kT = Lay<F>::kSteps;
+    Ring<F> R = ring;
+    const Flags flags = A.fl;
+    const int lane = threadIdx.x & 31, D = A.sd.D, nblk = D / kT;
     unsigned long long w = kSentinel;
     bool given_up = false;
     long long polls = 0;
-    while (ready < nblk) {
-        // start copies into free stages; wait for one only when there is nothing else to do
-        while (issued < nblk && issued < ready + R.stages) {
-            uint64_t *fr = R.bar(Ring<F>::FREE, R.st);
-            if (!__all_sync(FULL, R.dead || mbar_test(fr, R.parity ^ 1u))) {
-                if (issued > ready) break;
-                ring_wait(R, fr, R.parity ^ 1u, flags);
-            }
-            if (lane == 0) {
-                // without a preparer the sweeping warp itself waits for the copies; `copied` keeps pace
-                uint64_t *ready_bar = R.bar(Ring<F>::READY, R.st), *copied = R.bar(Ring<F>::COPIED, R.st);
-                uint64_t *tx = kPrepared ? copied : ready_bar;
-                char *dst = g_smem + R.stage(R.st);
-                mbar_expect_tx(tx, (1u + kC) * kVec);
-                bulk_g2s(dst, vec, kVec, tx);
-                bulk_g2s(dst + kVec, cf, kC * kVec, tx);
-                if (!kPrepared) mbar_arrive(copied);
-                if (!IN) mbar_arrive(ready_bar);
-            }
-            vec += BWD ? -kT * kCells : kT * kCells;
-            cf += (BWD ? -kT * kCells : kT * kCells) * kC;
-            R.next();
-            issued++;
-            if (!IN) ready++;
+    for (int ready = 0; ready < nblk;) {  // blocks whose words are in place
+        const int t = ready * kT + lane;
+        const bool need = t <= D - 32;
+        unsigned long long *word = in.row + (BWD ? D - 32 - t : t + 32);
+        // poll when the next block lacks a word, for all that are missing
+        const bool missing = need && w == kSentinel && !given_up;
+        if ((__ballot_sync(FULL, missing) & ((1u << kT) - 1u)) != 0u && missing) {
+            asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(w) : "l"(word));
+            if (w != kSentinel) asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(word), "l"(kSentinel));
         }
-        if constexpr (IN) {
-            const int t = ready * kT + lane;
-            const bool need = t <= D - 32;
-            unsigned long long *word = in.row + (BWD ? D - 32 - t : t + 32);
-            if (need && w == kSentinel && !given_up) {
-                asm volatile("ld.relaxed.gpu.u64 %0, [%1];" : "=l"(w) : "l"(word));
-                if (w != kSentinel) asm volatile("st.relaxed.gpu.u64 [%0], %1;" ::"l"(word), "l"(kSentinel));
+        if (!need) w = 0ull;
+        // the operands, which the words are put behind or folded into, of the blocks that fit the ring
+        const int q = lane / kT;
+        const bool wrapped = R.st + q >= R.stages;
+        const int st = R.st + q - (wrapped ? R.stages : 0);
+        bool there = (w != kSentinel || given_up) && q < R.stages;
+        if (there)
+            there = R.dead || mbar_test(R.bar(kPrepared ? Ring<F>::PREPARED : Ring<F>::COPIED, st), R.parity ^ (wrapped ? 1u : 0u));
+        const unsigned have = __ballot_sync(FULL, there);
+        // blocks that have all they need
+        const int k = min((have == FULL ? 32 : __ffs(~have) - 1) / kT, nblk - ready);
+        if (k > 0) {
+            polls = 0;
+            if (q < k) put_halo<F, BWD>(g_smem + R.stage(st), lane % kT, given_up && w == kSentinel ? 0ull : w);
+            __syncwarp();
+            if (lane < k) {
+                int at = R.st + lane;
+                at -= at >= R.stages ? R.stages : 0;
+                mbar_arrive(R.bar(Ring<F>::READY, at));
             }
-            if (!need) w = 0ull;
-            const unsigned have = __ballot_sync(FULL, w != kSentinel || given_up);
-            // blocks from `ready` on whose words are all there
-            int k = min(__ffs(~have) - 1 < 0 ? 32 : __ffs(~have) - 1, (issued - ready) * kT) / kT;
-            if (k > 0) {
-                polls = 0;
-                const int q = lane / kT;
-                int st = rst + q;
-                st -= st >= R.stages ? R.stages : 0;
-                if (q < k)
-                    *(volatile unsigned long long *)(g_smem + R.stage(st) + kHaloAt<F> + 8 * (lane % kT)) = given_up && w == kSentinel ? 0ull : w;
-                __syncwarp();
-                if (lane < k) {
-                    int at = rst + lane;
-                    at -= at >= R.stages ? R.stages : 0;
-                    mbar_arrive(R.bar(Ring<F>::READY, at));
-                }
-                w = __shfl_down_sync(FULL, w, k * kT);
-                if (lane >= 32 - k * kT) w = kSentinel;
-                ready += k;
-                rst += k;
-                rst -= rst >= R.stages ? R.stages : 0;
-            } else if (++polls > flags.limit || ((polls & 15) == 0 && __any_sync(FULL, timed_out(flags)))) {
-                if (!given_up) set_timeout(flags);
-                given_up = true;
-            }
+            w = __shfl_down_sync(FULL, w, (k * kT) & 31);
+            if (lane >= 32 - k * kT) w = kSentinel;
+            ready += k;
+            R.skip(k);
+        } else if (++polls > flags.limit || ((polls & 15) == 0 && __any_sync(FULL, timed_out(flags)))) {
+            if (!given_up) set_timeout(flags);
+            given_up = true;
+            R.dead = polls > kMbarWaitLimit + flags.limit;
         }
     }
     ring = R;
