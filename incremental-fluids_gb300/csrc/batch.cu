@@ -52,8 +52,8 @@ constexpr double kHomeMargin = 0.05;
 template <typename F>
 std::vector<PcgShape> candidate_shapes() {
     if (sizeof(F) == 4)
-        return {{128, 1, 4}, {128, 1, 3}, {64, 1, 3}, {64, 1, 4}, {256, 1, 4}, {256, 2, 3}, {128, 2, 2}};
-    return {{128, 1, 4}, {128, 1, 3}, {64, 1, 4}, {256, 1, 4}, {256, 2, 4}, {128, 2, 3}};
+        return {{256, 2, 3}, {128, 1, 3}, {128, 1, 4}, {256, 1, 4}};
+    return {{128, 1, 4}, {128, 1, 3}, {256, 1, 4}, {256, 2, 4}};
 }
 
 template <typename F>
@@ -358,35 +358,25 @@ class BatchImpl final : public BatchBase {
                    : IFL_OK;
     }
 
-    // Estimated PCG time of each scene: iterations x (two wavefront sweeps,
-    // D + lag per strip steps each; the elementwise passes over its team).
-    // Estimated time (microseconds) of scene i's solve on a team of g blocks:
-    // per PCG iteration a forward and a backward sweep, the elementwise passes
-    // and the team barriers.  A sweep of S strips by P = g*K warps (strips taken
+    // Estimated time (microseconds) of scene i's solve on a team of g blocks: per
+    // PCG iteration a forward and a backward sweep, the elementwise passes and the
+    // team barriers.  A sweep of S strips by P = g*K warps (strips taken
     // round-robin) finishes after
     //   max((S-1)*lag + D*tau, (S-1)/P * D*tau + ((S-1) mod P)*lag + D*tau):
     // strip s starts a hand-over (lag) after strip s-1 and not before its warp
-    // finished strip s-P.  The elementwise passes cost a fixed time per cell
-    // and warp; a team of more than one block adds its barriers, which grow
-    // with its size.  Constants fitted to per-phase timers in the batched
-    // kernel on GB300 (512-scene batch, FP32 form, 64-thread blocks, teams of
-    // 1 to 64 blocks): tau = 0.11 us per wavefront step, lag = 6.4 us per
-    // strip, 27.4 ns per cell per two-warp block for three elementwise passes,
-    // barriers 15 + 6 log2(g) us for five team barriers per iteration; the
-    // sigma pass (about an eighth of the elementwise time) and one barrier have
-    // since moved into the forward sweep, leaving 24 ns and 12 + 4.8 log2(g).
-    // The step time is flat around these values: with the faster matvec that
-    // followed, 17, 20 or 30 ns per cell and a lag of 8 us changed the
-    // 512-scene step by less than its step-to-step spread.
+    // finished strip s-P.  The elementwise passes cost a fixed time per cell and
+    // warp; the totals and, for a team of more than one block, its barriers a fixed
+    // time.  Constants from per-phase timers in the batched kernel on GB300
+    // (512-scene batch, 128-thread blocks, three to an SM).
     double plan_cost(int i, int g) const {
         constexpr bool f32 = sizeof(F) == 4;
-        constexpr double kTau = f32 ? 0.085 : 0.075, kLag = f32 ? 6.5 : 4.1, kElemNs = f32 ? 6.0 : 8.0;
+        constexpr double kTau = f32 ? 0.14 : 0.11, kLag = f32 ? 6.0 : 6.0, kElemNs = f32 ? 7.7 : 10.0;
         const Scene<F> &S = scene(i);
         const int P = g * shape_.K, Sn = S.sd.S;
         const double Dt = S.sd.D * kTau;
         const double sweep = std::max((Sn - 1) * kLag + Dt, ((Sn - 1) / P) * Dt + ((Sn - 1) % P) * kLag + Dt);
-        const double elem = 1e-3 * kElemNs * (double)S.w * S.h / g * (128.0 / shape_.threads);
-        return iters_[i] * (2.0 * sweep + elem + (g == 1 ? 6.0 : 12.0));
+        const double elem = 1e-3 * kElemNs * (double)S.w * S.h / g * (128.0 / pcg_batch_block(plan_));
+        return iters_[i] * (2.0 * sweep + elem + (g == 1 ? 8.0 : 16.0));
     }
 
     int schedule() {

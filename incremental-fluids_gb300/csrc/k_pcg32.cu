@@ -230,6 +230,14 @@ struct Tiles {
     __device__ __forceinline__ size_t at(int d) const { return base + (size_t)d * 64; }
 };
 
+// The operands of this warp's next chunk on their way from HBM to L2: the scenes of
+// a batch do not fit there together, and a warp has no more loads in flight than
+// its registers hold.
+template <typename T>
+__device__ __forceinline__ void prefetch_chunk(const T *p, int c, int c_end, int kc) {
+    if (c < c_end && (threadIdx.x & 31) == 0) prefetch_l2(p + (size_t)c * kc * 256, kc * 256 * sizeof(T));
+}
+
 // s = z + beta*s (first iteration: s = z), then z' = A s and z'.s over this
 // warp's chunks (3-conjugate-gradients/Fluid.cpp:361-362, 375, 315-332).  A lane
 // forms the new s of its tile, of the column left of it and of the column right
@@ -256,6 +264,10 @@ __device__ __noinline__ void matvec(const PcgArgs<float> &A, int iter, float bet
     for (int c = c_begin; c < c_end; c += c_step) {
         const int s = (c * kc) / D, d0 = c * kc - s * D;  // a chunk lies inside one strip
         const Tiles T(sd, s, lane);
+        prefetch_chunk(A.z, c + c_step, c_end, kc);
+        prefetch_chunk(so, c + c_step, c_end, kc);
+        prefetch_chunk(A.ax, c + c_step, c_end, kc);
+        prefetch_chunk(A.ay, c + c_step, c_end, kc);
         double dacc = 0.0;
         for (int u = 0; u < kc; u++) {
             const int d = d0 + u;
@@ -412,6 +424,11 @@ __device__ __noinline__ void axpy(const PcgArgs<float> &A, int iter, double alph
     for (int c = c_begin; c < c_end; c += c_step) {
         const int s = (c * kc) / D, d0 = c * kc - s * D;
         const Tiles T(sd, s, lane);
+        prefetch_chunk((const float *)sp, c + c_step, c_end, kc);
+        if (ROWSUM) prefetch_chunk((const float *)A.as, c + c_step, c_end, kc);
+        else prefetch_chunk(A.as, c + c_step, c_end, kc);
+        prefetch_chunk(A.p, c + c_step, c_end, kc);
+        prefetch_chunk(A.r, c + c_step, c_end, kc);
         unsigned long long mx = 0ull;  // bits of the largest |r| so far
         for (int u = 0; u < kc; u++) {
             const int d = d0 + u;

@@ -45,7 +45,10 @@ template <typename F> constexpr unsigned kVecBytes = Lay<F>::kSteps * Lay<F>::kC
 template <typename F> constexpr unsigned kHaloAt = 4u * kVecBytes<F>;       // its halo words, behind four arrays
 template <typename F> constexpr unsigned kStageBytes = kHaloAt<F> + 128u;   // a ring stage
 constexpr int kMaxStages = 8;
-constexpr int kMaxThreads = 384;  // of a block (168 registers per thread)
+// Threads of a block: the FP32 form's batched passes are bound by what 128-thread
+// blocks an SM holds (three at 160 registers, four at 128: 512 scenes of 64^2 to
+// 768^2 in 316 instead of 381 ms), the FP64 form spills below 168.
+template <typename F> constexpr int kMaxThreads = sizeof(F) == 4 ? 512 : 384;
 constexpr int kRoles = 4;   // warps that work on one strip: sweep, load, prepare, take
 constexpr int kSums = 16;   // partial sums of a reduction (see total_of)
 
