@@ -374,11 +374,11 @@ __device__ __noinline__ void factor_rows(const PcgArgs<F> &A, int q, const Chan 
     }
 }
 
-// Sum (or maximum) of n partials in a fixed order that depends on n alone:
+// Sum of n partials in a fixed order that depends on n alone:
 // virtual warp v < kSums adds the partials v*32 + lane + 512 k in order of k,
 // its lanes follow a fixed shuffle tree, and so do the kSums results.  Every
 // block forms the same bits, whatever its number of warps.
-__device__ __forceinline__ double total_of(const double *pt, int n, bool is_max, double *sm) {
+__device__ __forceinline__ double total_of(const double *pt, int n, double *sm) {
     const int warps = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (n <= 32) {  // every warp for itself
@@ -386,7 +386,7 @@ __device__ __forceinline__ double total_of(const double *pt, int n, bool is_max,
         for (int o = 16; o > 0; o >>= 1) {
             if (o >= n) continue;
             const double w = __shfl_down_sync(FULL, acc, o);
-            acc = is_max ? smax(acc, w) : acc + w;
+            acc = acc + w;
         }
         return __shfl_sync(FULL, acc, 0);
     }
@@ -399,9 +399,9 @@ __device__ __forceinline__ double total_of(const double *pt, int n, bool is_max,
                 for (int j = 0; j < 4; j++) w[j] = i0 + j * 32 * kSums < n ? __ldcg(pt + i0 + j * 32 * kSums) : 0.0;
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    if (i0 + j * 32 * kSums < n) acc = is_max ? smax(acc, w[j]) : acc + w[j];
+                    if (i0 + j * 32 * kSums < n) acc = acc + w[j];
             }
-            acc = is_max ? warp_max(acc) : warp_sum(acc);
+            acc = warp_sum(acc);
         }
         if (lane == 0) sm[v] = acc;
     }
@@ -411,7 +411,7 @@ __device__ __forceinline__ double total_of(const double *pt, int n, bool is_max,
     for (int o = kSums / 2; o > 0; o >>= 1) {
         if (o >= used) continue;
         const double w = __shfl_xor_sync(FULL, acc, o);
-        acc = is_max ? smax(acc, w) : acc + w;
+        acc = acc + w;
     }
     return __shfl_sync(FULL, acc, 0);
 }
@@ -428,6 +428,20 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v
         v = w > v ? w : v;
     }
     return v;
+}
+
+// Maximum of n partials that max_bits formed, by one warp, into sm[0].
+__device__ __forceinline__ void max_of(const double *pt, int n, double *sm) {
+    unsigned long long mx = 0ull;
+    for (int c0 = threadIdx.x & 31; c0 < n; c0 += 32 * 8) {
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = c0 + 32 * j < n ? __ldcg(pt + c0 + 32 * j) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) max_bits(mx, v[j]);
+    }
+    mx = warp_max_bits(mx);
+    if ((threadIdx.x & 31) == 0) sm[0] = __longlong_as_double((long long)mx);
 }
 
 }  // namespace
