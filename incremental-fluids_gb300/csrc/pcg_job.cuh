@@ -107,10 +107,11 @@ __device__ void pcg_job(const PcgArgs<F> &A, Team &T, Ring<F> &R, double *sm) {
         const int nq = (sd.H + 31) / 32;
         for (int q = warp * T.size + T.rank; q < nq; q += nwarps) {
             const Chan in{A.halo + (size_t)(q > 0 ? q - 1 : 0) * sd.W, q > 0}, out{A.halo + (size_t)q * sd.W, q + 1 < nq};
-            if (q > 0) factor_rows<F, REF, true>(A, q, in, out);
-            else factor_rows<F, REF, false>(A, q, in, out);
+            if (q > 0) factor_rows<F, true>(A, q, in, out);
+            else factor_rows<F, false>(A, q, in, out);
         }
         team_barrier(T, A.fl);
+        coefs<F, REF>(A, c_begin, c_end, nwarps, kc);  // used after start()'s barrier
     }
     if (!(A.mode & PCG_SOLVE)) return;
 

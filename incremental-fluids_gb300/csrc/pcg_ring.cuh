@@ -304,20 +304,21 @@ __device__ __noinline__ void take_strip(const PcgArgs<F> &A, Ring<F> &ring, cons
 // --------------------------------------------------------------- factor
 // buildPreconditioner (3-conjugate-gradients/Fluid.cpp:253-269): FP64
 // arithmetic in the reference's order (the factor is bit-identical), so the
-// step's ~35 FP64 instructions at 64 cycles each (one warp of an SM quarter)
-// are what it costs: rows, not tiles, are spread over the warps - lane l of a
-// warp walks row 32 q + l, one column behind lane l - 1 - and the scattered
-// accesses to the tile layout hide behind them.  A cell forms the terms that
-// its right and upper neighbours subtract from their diagonals (the same
-// products the reference forms there) and writes their al and bd.  The upper
+// step's FP64 instructions at 64 cycles each (one warp of an SM quarter), most of
+// them in the square root and the division, are what it costs: rows, not tiles,
+// are spread over the warps - lane l of a warp walks row 32 q + l, one column
+// behind lane l - 1 - and the step does nothing that need not be in the chain: the
+// sweeps' coefficients are formed from the factor afterwards (coefs), everywhere
+// at once.  A cell forms the terms that its right and upper neighbours subtract
+// from their diagonals (the same products the reference forms there).  The upper
 // term of row 32 q - 1 arrives through a halo row of W words.
-template <typename F, bool REF, bool IN>
+template <typename F, bool IN>
 __device__ __noinline__ void factor_rows(const PcgArgs<F> &A, int q, const Chan in, const Chan out) {
     const int lane = threadIdx.x & 31;
     const SDIdx sd = A.sd;
     const int W = sd.W, H = sd.H, y = 32 * q + lane;
     const bool rowok = y < H;
-    const size_t base = sd.slot(0, rowok ? y : 0), above = sd.slot(0, y + 1 < H ? y + 1 : 0);
+    const size_t base = sd.slot(0, rowok ? y : 0);
     auto at = [](size_t row, int x) { return sizeof(F) == 8 ? row + (size_t)x * 32 : row + (size_t)(x >> 1) * 256 + (x & 1) * 128; };
     // operands of the step after the current one
     F ndiag = F(0), nax = F(0), nay = F(0);
@@ -356,21 +357,36 @@ __device__ __noinline__ void factor_rows(const PcgArgs<F> &A, int q, const Chan 
         const double px = ax * pcv, py = ay * pcv, txy = kTau * px * py;
         left = px * px + txy;
         upper = py * py + txy;
-        const bool self = b & NB_SELF;
-        const double p2 = !self ? 0.0 : REF ? pcv : pcv * pcv;
-        const F va = from_f64<F>(ax * p2), vb = from_f64<F>(ay * p2);
-        if (active) {
-            const size_t k = at(base, x);
-            const F dd = from_f64<F>(p2), sign = REF ? F(1) : F(-1);
-            if (self) A.pc[k] = pcv;
-            *coef<REF, true>(A, k, REF ? R_RIGHT : C_RIGHT) = sign * va;
-            *coef<REF, true>(A, k, REF ? R_UP : C_UP) = sign * vb;
+        if (b & NB_SELF) A.pc[at(base, x)] = pcv;
+        hstore_if(out, x, henc(upper), out.valid && lane == 31 && active);
+    }
+}
+
+// The sweeps' coefficients of this warp's chunks, from the factor.  A cell writes
+// its own backward ones and the forward ones of its right and upper neighbours.
+template <typename F, bool REF>
+__device__ __noinline__ void coefs(const PcgArgs<F> &A, int c_begin, int c_end, int c_step, int kc) {
+    const int lane = threadIdx.x & 31;
+    const SDIdx sd = A.sd;
+    for (int row = c_begin * kc; row < c_end * kc; row += (row + 1) % kc ? 1 : (c_step - 1) * kc + 1) {
+        const int s = row / sd.D, d = row - s * sd.D;
+#pragma unroll
+        for (int i = 0; i < Lay<F>::kCells / 32; i++) {
+            const int idx = 32 * i + lane, l = sizeof(F) == 8 ? idx : (idx >> 2) & 31;
+            const int x = sizeof(F) == 8 ? d - l : 2 * (d - l) + (idx >> 7);
+            const int y = sizeof(F) == 8 ? 32 * s + l : 4 * (32 * s + l) + (idx & 3);
+            if (x < 0 || x >= sd.W || y >= sd.H) continue;
+            const size_t k = (size_t)row * Lay<F>::kCells + idx;
+            const double pcv = A.pc[k], p2 = !(A.nb[k] & NB_SELF) ? 0.0 : REF ? pcv : pcv * pcv;
+            const F sign = REF ? F(1) : F(-1), dd = from_f64<F>(p2);
+            const F va = sign * from_f64<F>(to_f64(A.ax[k]) * p2), vb = sign * from_f64<F>(to_f64(A.ay[k]) * p2);
+            *coef<REF, true>(A, k, REF ? R_RIGHT : C_RIGHT) = va;
+            *coef<REF, true>(A, k, REF ? R_UP : C_UP) = vb;
             *coef<REF, true>(A, k, REF ? R_PC : C_DD) = dd;
             if (REF) *coef<REF, false>(A, k, R_PC) = dd;
-            if (x + 1 < W) *coef<REF, false>(A, at(base, x + 1), C_LEFT) = sign * va;
-            if (y + 1 < H) *coef<REF, false>(A, at(above, x), C_DOWN) = sign * vb;
+            if (x + 1 < sd.W) *coef<REF, false>(A, sd.slot(x + 1, y), C_LEFT) = va;
+            if (y + 1 < sd.H) *coef<REF, false>(A, sd.slot(x, y + 1), C_DOWN) = vb;
         }
-        hstore_if(out, x, henc(upper), out.valid && lane == 31 && active);
     }
 }
 
