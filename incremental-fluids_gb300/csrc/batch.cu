@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <numeric>
 #include <vector>
 
 #include "solver.h"
@@ -44,15 +45,17 @@ int pow2ceil(int v) {
 
 // The home shape (the first candidate) is kept unless another one is more than
 // kHomeMargin faster in the trial: a trial of a few pinned iterations of the
-// first system cannot separate shapes within a few percent (on GB300 the
-// 512-scene batch ran its steps 19 % faster on 64 x 1 x 2 than on 32 x 1 x 2,
-// which had won such a trial by 1.4 %).
+// first system cannot separate shapes within a few percent.
 constexpr double kHomeMargin = 0.05;
 
+// PCG milliseconds per step of 24 scenes (64^2 to 256^2) and 512 scenes (to 768^2)
+// on GB300, FP32 form: {256,1,4} 6.4 and 275, {128,1,3} 6.9 and 306, {256,2,3} 6.8
+// and 314, {128,1,4} 6.4 and 376, {256,1,3} 6.6 and 289: sixteen warps to an SM for
+// the elementwise passes, a strip's copies far enough ahead.
 template <typename F>
 std::vector<PcgShape> candidate_shapes() {
     if (sizeof(F) == 4)
-        return {{256, 2, 3}, {128, 1, 3}, {128, 1, 4}, {256, 1, 4}};
+        return {{256, 1, 4}, {128, 1, 3}, {256, 2, 3}};
     return {{128, 1, 4}, {128, 1, 3}, {256, 1, 4}, {256, 2, 4}};
 }
 
@@ -597,8 +600,8 @@ class BatchImpl final : public BatchBase {
         return check(cudaGetLastError(), "tile autotune") ? IFL_ERR_CUDA : IFL_OK;
     }
 
-    // Each candidate shape solves the first step's real system with a pinned
-    // iteration count (twice; the faster run counts).  The phases before the
+    // Each candidate shape solves the first step's real system with pinned
+    // iteration counts (twice; the faster run counts).  The phases before the
     // first solve are idempotent, so the real step repeats them unchanged.
     int autotune(double dt) {
         const int iters = opt_.tune_iterations > 0 ? opt_.tune_iterations : 8;
@@ -606,6 +609,14 @@ class BatchImpl final : public BatchBase {
         record_head(dt);
         double best = std::numeric_limits<double>::infinity();
         PcgShape best_sh{};
+        // each scene's share of the iterations, as the plan expects them: with the
+        // same count for all, the largest scenes do not hold up a trial as they do a step
+        const std::vector<int4> ctl(h_ctl_, h_ctl_ + n_);
+        const double mean = std::accumulate(iters_.begin(), iters_.end(), 0.0) / n_;
+        for (int i = 0; i < n_; i++) {
+            const int k = std::max(1, (int)std::lround(iters * iters_[i] / mean));
+            h_ctl_[i] = make_int4(k, k, ctl[i].z, ctl[i].w);
+        }
         trial_ms_.clear();
         for (const PcgShape &sh : candidate_shapes<F>()) {
             if (make_plan(sh) != IFL_OK) {
@@ -615,8 +626,10 @@ class BatchImpl final : public BatchBase {
             if (int e = schedule()) return e;
             if (int e = upload_ctl()) return e;
             double t = std::numeric_limits<double>::infinity();
-            for (int rep = 0; rep < 2; rep++) {
-                PcgConfig cfg{PCG_FACTOR | PCG_SOLVE, 0, iters, heat};
+            for (int rep = 0; rep < 3; rep++) {
+                // the factor, once and untimed, then solves alone: it weighs as much as
+                // 15 iterations, of a hundred and more in a step's solve
+                PcgConfig cfg{rep == 0 ? PCG_FACTOR | PCG_SOLVE : PCG_SOLVE, 0, rep == 0 ? 1 : -2, heat};
                 if (check(cudaEventRecord(ev_trial0_, st_), "event") ||
                     check(launch_pcg_batch<F>(plan_, cfg, st_), "autotune launch") ||
                     check(cudaEventRecord(ev_trial1_, st_), "event") ||
@@ -625,7 +638,7 @@ class BatchImpl final : public BatchBase {
                 launches_++;
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, ev_trial0_, ev_trial1_);
-                t = std::min(t, (double)ms);
+                if (rep > 0) t = std::min(t, (double)ms);
             }
             trial_ms_.push_back(t);
             if (t < best) {
@@ -633,6 +646,7 @@ class BatchImpl final : public BatchBase {
                 best_sh = sh;
             }
         }
+        std::copy(ctl.begin(), ctl.end(), h_ctl_);
         if (!(best < std::numeric_limits<double>::infinity())) {
             err_ = "no batched PCG shape fits this batch";
             return IFL_ERR_UNSUPPORTED;
