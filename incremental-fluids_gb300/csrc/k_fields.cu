@@ -556,36 +556,70 @@ __global__ void __launch_bounds__(1024)
     extrap_solve_body(S, qmask, counters, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsigned qmask, const int *empties) {
-    const int qi = blockIdx.x;
-    if (!((qmask >> qi) & 1u) || empties[qi] == 0) return;
-    const Quant<double> Q = S.q[qi];
+// What the walk knows of a cell, in a byte: its type (an outer-ring cell that is
+// not fluid is never touched: kInert), the reference's _mask, and the signs of its
+// normal.
+constexpr unsigned kInert = 3u;
+__device__ __forceinline__ unsigned walk_sign(double v) { return v > 0.0 ? 1u : v < 0.0 ? 2u : 0u; }
+__device__ __forceinline__ unsigned walk_type(unsigned b) { return b & 3u; }
+__device__ __forceinline__ unsigned walk_mask(unsigned b) { return b >> 2 & 3u; }
+__device__ __forceinline__ unsigned walk_nx(unsigned b) { return b >> 4 & 3u; }
+__device__ __forceinline__ unsigned walk_ny(unsigned b) { return b >> 6; }
+
+// sum / k for k = 1..4 (0: NaN), as the division rounds it: by powers of two the
+// product is the same, and for 3 the remainder of sum * RN(1/3) corrects the
+// product to the nearest (P. Markstein, IBM J. Res. Dev. 34, 1990; |3 RN(1/3) - 1| =
+// 2^-54 keeps the product within an ulp), away from underflow and overflow.
+__device__ __forceinline__ double walk_average(double sum, int k) {
+    if (k == 3) {
+        const unsigned e = ((unsigned)__double2hiint(sum) >> 20) & 0x7ffu;
+        if (e - 100u >= 1900u && sum != 0.0) return sum / 3.0;
+        const double y = 1.0 / 3.0, q = sum * y;
+        return fma(fma(-3.0, q, sum), y, q);
+    }
+    return k == 4 ? sum * 0.25 : k == 2 ? sum * 0.5 : k == 1 ? sum : sum / 0.0;
+}
+
+// One thread replays the stack: a chain of a few thousand pops, each waiting for
+// its loads, and for its sum and division.  So the cells' bytes and the stack's
+// first kWalkStack entries lie in shared memory (SHARED; grids whose bytes do not
+// fit keep them in Q.ready), src is read into L1 before, and an average takes no
+// division: 128 x 128 with four quantities 2.14 ms with everything in global
+// memory, two byte arrays, six loads of normals and a division per pop.
+constexpr int kWalkStack = 8192, kWalkBytes = 160 * 1024;
+template <bool SHARED>
+__device__ __forceinline__ void extrap_walk(const Scene<double> &S, const Quant<double> &Q) {
+    extern __shared__ __align__(16) unsigned char walk_smem[];
     const int w = Q.w, h = Q.h, P = S.P;
-    uint8_t *c = Q.cell, *m = Q.ready;  // `ready` holds the reference's _mask here
+    uint8_t *c = Q.cell, *info = SHARED ? (uint8_t *)(walk_smem + 4 * kWalkStack) : Q.ready;
+    int *near_stack = (int *)walk_smem, *stack = Q.list;
     double *src = Q.src;
     const double *nx = Q.nx, *ny = Q.ny;
-    int *stack = Q.list;
     const long stack_cap = 2L * P * (S.h + 2);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    auto entry = [&](long t) -> int * { return SHARED && t < kWalkStack ? near_stack + t : stack + t; };
 
-    // fillSolidMask: outer ring 0xFF; solid cells wait for non-fluid upwind
-    // neighbours; empty cells with no fluid neighbour wait for any neighbour.
+    // fillSolidMask: the outer ring is never freed; solid cells wait for non-fluid
+    // upwind neighbours; empty cells with no fluid neighbour wait for any neighbour.
+    unsigned long long touched = 0ull;
     for (int i = tid; i < w * h; i += blockDim.x) {
         const int x = i % w, y = i / w;
         const long idx = x + (long)y * P;
-        uint8_t mv = 0;
+        const double ax = nx[idx], ay = ny[idx];
+        unsigned type = c[idx], mv = 0;
+        touched ^= (unsigned long long)__double_as_longlong(src[idx]);
         if (x == 0 || y == 0 || x == w - 1 || y == h - 1) {
-            mv = 0xFF;
-        } else if (c[idx] == CELL_SOLID) {
-            const double ax = nx[idx], ay = ny[idx];
+            if (type != CELL_FLUID) type = kInert;
+        } else if (type == CELL_SOLID) {
             if (ax != 0.0 && c[idx + sgn(ax)] != CELL_FLUID) mv |= 1;
             if (ay != 0.0 && c[idx + (long)sgn(ay) * P] != CELL_FLUID) mv |= 2;
-        } else if (c[idx] == CELL_EMPTY) {
+        } else if (type == CELL_EMPTY) {
             mv = c[idx - 1] != CELL_FLUID && c[idx + 1] != CELL_FLUID && c[idx - P] != CELL_FLUID &&
                  c[idx + P] != CELL_FLUID;
         }
-        m[idx] = mv;
+        info[idx] = (uint8_t)(type | mv << 2 | walk_sign(ax) << 4 | walk_sign(ay) << 6);
     }
+    asm volatile("" ::"l"(touched));  // the loads stay
     __syncthreads();
 
     // Initial stack: interior cells in row-major order (ordered compaction).
@@ -600,7 +634,8 @@ __global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsi
         bool f = false;
         if (i < ni) {
             idx = 1 + i % iw + (long)(1 + i / iw) * P;
-            f = c[idx] != CELL_FLUID && m[idx] == 0;
+            const unsigned b = info[idx];
+            f = walk_type(b) != CELL_FLUID && walk_mask(b) == 0;
         }
         const unsigned bal = __ballot_sync(0xffffffffu, f);
         if (lane == 0) s_warp[warp] = __popc(bal);
@@ -616,7 +651,7 @@ __global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsi
         }
         __syncthreads();
         const int total = s_total;
-        if (f) stack[s_base + s_warp[warp] + __popc(bal & ((1u << lane) - 1u))] = (int)idx;
+        if (f) *entry(s_base + s_warp[warp] + __popc(bal & ((1u << lane) - 1u))) = (int)idx;
         __syncthreads();
         if (tid == 0) s_base += total;
         __syncthreads();
@@ -626,60 +661,76 @@ __global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsi
         long top = s_base, guard = 0;
         const long limit = 8L * w * h + 64;
         bool bad = false;
-        auto push = [&](long v) {
+        auto push = [&](int v) {
             if (top >= stack_cap) bad = true;
-            else stack[top++] = (int)v;
+            else *entry(top++) = v;
         };
         while (top > 0 && !bad) {
             if (++guard > limit) {
                 bad = true;
                 break;
             }
-            const long idx = stack[--top];
-            if (c[idx] == CELL_EMPTY) {  // extrapolateAverage
+            const int idx = *entry(--top);
+            const int nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
+            const unsigned me = info[idx];
+            unsigned n[4];
+            double v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                n[j] = info[nb[j]];
+                v[j] = src[nb[j]];
+            }
+            if (walk_type(me) == CELL_EMPTY) {  // extrapolateAverage
                 double sum = 0.0;
                 int k = 0;
-                const long nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
+#pragma unroll
                 for (int j = 0; j < 4; j++)
-                    if (c[nb[j]] == CELL_FLUID) {
-                        sum += src[nb[j]];
+                    if (walk_type(n[j]) == CELL_FLUID) {
+                        sum += v[j];
                         k++;
                     }
-                src[idx] = sum / k;
-                c[idx] = CELL_FLUID;
+                src[idx] = walk_average(sum, k);
+                info[idx] = (uint8_t)((me & ~3u) | CELL_FLUID);
             } else {  // extrapolateNormal
                 const double ax = nx[idx], ay = ny[idx];
-                src[idx] = (fabs(ax) * src[idx + sgn(ax)] + fabs(ay) * src[idx + (long)sgn(ay) * P]) /
-                           (fabs(ax) + fabs(ay));
+                src[idx] = (fabs(ax) * src[idx + sgn(ax)] + fabs(ay) * src[idx + sgn(ay) * P]) / (fabs(ax) + fabs(ay));
             }
             // freeSolidNeighbour: a solid neighbour whose normal points here
-            const long sn[4] = {idx - 1, idx + 1, idx - P, idx + P};
-            const bool toward[4] = {nx[idx - 1] > 0.0, nx[idx + 1] < 0.0, ny[idx - P] > 0.0, ny[idx + P] < 0.0};
+            const bool toward[4] = {walk_nx(n[0]) == 1u, walk_nx(n[1]) == 2u, walk_ny(n[2]) == 1u, walk_ny(n[3]) == 2u};
+#pragma unroll
             for (int j = 0; j < 4; j++) {
-                if (!toward[j] || c[sn[j]] != CELL_SOLID) continue;
-                m[sn[j]] &= (uint8_t)~(j < 2 ? 1 : 2);
-                if (m[sn[j]] == 0) push(sn[j]);
+                if (!toward[j] || walk_type(n[j]) != CELL_SOLID) continue;
+                const unsigned b = n[j] & ~(j < 2 ? 4u : 8u);
+                info[nb[j]] = (uint8_t)b;
+                if (walk_mask(b) == 0) push(nb[j]);
             }
             // freeEmptyNeighbour
+#pragma unroll
             for (int j = 0; j < 4; j++)
-                if (c[sn[j]] == CELL_EMPTY && m[sn[j]] == 1) {
-                    m[sn[j]] = 0;
-                    push(sn[j]);
+                if (walk_type(n[j]) == CELL_EMPTY && walk_mask(n[j]) == 1u) {
+                    info[nb[j]] = (uint8_t)(n[j] & ~12u);
+                    push(nb[j]);
                 }
         }
         if (bad) atomicOr(S.flags, FLAG_FLIP_STACK);
-        // extrapolateEmptyBorders: ring cells copy the inward neighbour,
-        // corners average two ring cells.
-        for (int x = 1; x < w - 1; x++) {
-            const long t = x, b = x + (long)(h - 1) * P;
-            if (c[t] == CELL_EMPTY) src[t] = src[t + P];
-            if (c[b] == CELL_EMPTY) src[b] = src[b - P];
-        }
-        for (int y = 1; y < h - 1; y++) {
-            const long l = (long)y * P, r = (long)y * P + w - 1;
-            if (c[l] == CELL_EMPTY) src[l] = src[l + 1];
-            if (c[r] == CELL_EMPTY) src[r] = src[r - 1];
-        }
+    }
+    __syncthreads();
+    // extrapolateEmptyBorders: ring cells copy the inward neighbour (an interior
+    // cell; in a grid without any the reference's order counts), corners average
+    // two ring cells.
+    const bool serial = w < 3 || h < 3;
+    for (int x = serial ? (tid == 0 ? 1 : w) : 1 + tid; x < w - 1; x += serial ? 1 : blockDim.x) {
+        const long t = x, b = x + (long)(h - 1) * P;
+        if (c[t] == CELL_EMPTY) src[t] = src[t + P];
+        if (c[b] == CELL_EMPTY) src[b] = src[b - P];
+    }
+    for (int y = serial ? (tid == 0 ? 1 : h) : 1 + tid; y < h - 1; y += serial ? 1 : blockDim.x) {
+        const long l = (long)y * P, r = (long)y * P + w - 1;
+        if (c[l] == CELL_EMPTY) src[l] = src[l + 1];
+        if (c[r] == CELL_EMPTY) src[r] = src[r - 1];
+    }
+    __syncthreads();
+    if (tid == 0) {
         const long tl = 0, tr = w - 1, bl = (long)(h - 1) * P, br = (long)(h - 1) * P + w - 1;
         if (c[tl] == CELL_EMPTY) src[tl] = 0.5 * (src[tl + 1] + src[tl + P]);
         if (c[tr] == CELL_EMPTY) src[tr] = 0.5 * (src[tr - 1] + src[tr + P]);
@@ -691,6 +742,12 @@ __global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsi
         const long idx = i % w + (long)(i / w) * P;
         if (c[idx] == CELL_EMPTY) c[idx] = CELL_FLUID;
     }
+}
+__global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsigned qmask, const int *empties, int shared) {
+    const int qi = blockIdx.x;
+    if (!((qmask >> qi) & 1u) || empties[qi] == 0) return;
+    if (shared) extrap_walk<true>(S, S.q[qi]);
+    else extrap_walk<false>(S, S.q[qi]);
 }
 
 // -------------------------------------------------------------- advection
@@ -928,7 +985,11 @@ void launch_extrapolate_guarded(const Scene<double> &S, unsigned qmask, const in
     dim3 b(32, 8);
     extrap_mask_guard_kernel<double><<<grid2(S.w + 1, S.h + 1, 4, b), b, 0, st>>>(S, qmask, counters, empty_counts);
     extrap_solve_guard_kernel<double><<<4, 1024, 0, st>>>(S, qmask, counters, empty_counts);
-    extrap_lifo_kernel<<<4, 1024, 0, st>>>(S, qmask, empty_counts);
+    const int bytes = S.P * (S.h + 1);  // a byte per cell of the largest quantity
+    const bool shared = bytes <= kWalkBytes;
+    const int smem = shared ? 4 * kWalkStack + bytes : 0;
+    cudaFuncSetAttribute(extrap_lifo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kWalkStack + kWalkBytes);
+    extrap_lifo_kernel<<<4, 1024, smem, st>>>(S, qmask, empty_counts, shared ? 1 : 0);
 }
 
 template <typename F>
