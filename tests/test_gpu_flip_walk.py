@@ -1,7 +1,8 @@
-"""The order-exact extrapolation of step 8 (k_fields.cu, extrap_walk) in both places
-that its bytes can lie: shared memory, and global memory for grids above 160 KB of
-them.  Bit for bit the oracle's, from the crafted particle state with empty cells.  (Sizes
-with h <= w + 2: step 7-8 index v-face densities with the u width.)
+"""The order-exact extrapolation of step 8 (k_fields.cu, extrap_lifo_kernel) in each of
+its forms: values after the walk (small grids), value by value with the cells' bytes
+in shared memory (larger ones, and small ones with more than 4096 pops), and in
+global memory (more than 160 KB of bytes).  Bit for bit the oracle's, from the
+crafted particle state with empty cells.
 """
 import pytest
 
@@ -10,12 +11,13 @@ from oracle import oracle as O
 from test_gpu_flip import _fields_equal, _pair, _particles_equal, _random_fields
 
 pytestmark = pytest.mark.gpu
+BLOCK = (0, 0.5, 0.5, 0.7, 0.7, 0.3, 0.0, 0.0, 0.0)
 
 
-@pytest.mark.parametrize("size", [(64, 50), (128, 128), (400, 390), (410, 405)], ids=lambda s: "%dx%d" % s)
-def test_transfer_with_empty_cells(ifl, size):
-    w, h = size
-    o, g, _ = _pair(ifl, w, h, [FC.BOX])
+@pytest.mark.parametrize("w,h,body", [(64, 50, FC.BOX), (128, 128, FC.BOX), (160, 150, BLOCK), (400, 390, FC.BOX),
+                                      (410, 405, FC.BOX)])
+def test_transfer_with_empty_cells(ifl, w, h, body):
+    o, g, _ = _pair(ifl, w, h, [body])
     o.flip_init()
     g.flip_init()
     arrays = FC.crafted(w, h, o.particles(O.P_X).copy(), o.particles(O.P_Y).copy())
