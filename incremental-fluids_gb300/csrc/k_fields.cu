@@ -541,8 +541,8 @@ __global__ void __launch_bounds__(1024) extrap_solve_kernel(Scene<F> S, unsigned
 // CELL_EMPTY cells it is the DAG above (the outer ring is never extrapolated
 // in either form).  With empty cells the result depends on the reference's
 // LIFO order - an empty cell averages the neighbours that are fluid when it is
-// popped - so one thread per quantity replays the stack exactly; the other
-// threads of the CTA build the masks and the initial stack
+// popped - so one warp per quantity replays the stack exactly; all threads of the
+// CTA build the masks and the initial stack, and compute the values
 // (8-flip/Fluid.cpp:478-653).
 template <typename F>
 __global__ void extrap_mask_guard_kernel(Scene<F> S, unsigned qmask, int *counters, const int *skip) {
@@ -580,22 +580,23 @@ __device__ __forceinline__ double walk_average(double sum, int k) {
     return k == 4 ? sum * 0.25 : k == 2 ? sum * 0.5 : k == 1 ? sum : sum / 0.0;
 }
 
-// The walk's order is one thread's, a pop after a pop; so everything it needs lies in
-// shared memory if it fits: the cells' bytes (else in Q.ready), the stack's first
-// entries, and, up to kEvents pops, what a pop leaves behind: its cell, the pops (or
-// original values) it takes its neighbours' values from, and its depth.  The values
-// follow afterwards, depth by depth, on all threads: on the walking thread a pop's
-// loads, products and division took 1700 cycles, 128 x 128 with four quantities
-// (1830 pops each) 1.58 ms, and 2.14 ms with the bytes in global memory too.
+// The walk's order is a single one, a pop after a pop; so everything it needs lies in
+// shared memory if it fits: the cells' bytes (else in Q.ready) and the stack's first
+// entries.  Up to kEvents pops, the walk leaves nothing but the order; a neighbour's
+// value in it is the one of its own pop if that came before, and the original one
+// if not.  The values follow afterwards on all threads, each waiting for those it
+// takes.  128 x 128 with four quantities (1830 pops each): 2.14 ms by one thread in
+// global memory, 1.58 with bytes and stack in shared memory, 0.45 with the values
+// (1700 cycles per pop for loads, products and a division) left for afterwards and a
+// lane for each neighbour.
 constexpr int kWalkStack = 4096, kWalkBytes = 160 * 1024, kEvents = 4096;
-constexpr int kNoInput = -2, kOriginal = -1;
 enum { WALK_GLOBAL = 0, WALK_SHARED = 1, WALK_EVENTS = 2 };
 __host__ __device__ __forceinline__ int walk_pad(int bytes) { return (bytes + 15) / 16 * 16; }
 // Shared memory of a mode, for `cells` bytes.
 inline int walk_smem_bytes(int mode, int cells) {
     if (mode == WALK_GLOBAL) return 0;
     const int b = 4 * kWalkStack + walk_pad(cells);
-    return mode == WALK_SHARED ? b : b + walk_pad(2 * cells) + kEvents * (4 + 8 + 8 + 2);
+    return mode == WALK_SHARED ? b : b + walk_pad(2 * cells) + kEvents * (8 + 4 + 2);
 }
 
 struct Walk {
@@ -666,47 +667,40 @@ __device__ __forceinline__ int walk_setup(const Quant<double> &Q, const Walk &W)
     return s_base;
 }
 
-// One thread: the walk from a stack of height `top`.  pop(idx, byte of the cell,
-// bytes of its neighbours) sets or records the cell's value; false ends the walk.
-// Returns whether the stack outgrew `cap` or the walk did not end.
-template <typename Pop>
+// One warp: the walk from a stack of height `top`; lane j < 4 is at the popped cell's
+// neighbour j (left, right, lower, upper).  pop(idx, byte of the cell, byte of the
+// lane's neighbour, its offset) sets or records the cell's value; false ends the
+// walk.  Returns whether the stack outgrew `cap` or the walk did not end.
+// SHARED: bytes and stack in shared memory as a whole.
+template <bool SHARED, typename Pop>
 __device__ __forceinline__ bool walk_run(const Walk &W, long top, long cap, Pop pop) {
-    const int P = W.P;
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    uint8_t *info = SHARED ? (uint8_t *)(walk_smem + 4 * kWalkStack) : W.info;
+    auto entry = [&](long t) -> int * { return SHARED ? (int *)walk_smem + t : W.entry(t); };
+    const int lane = threadIdx.x & 31, off = lane == 0 ? -1 : lane == 1 ? 1 : lane == 2 ? -W.P : lane == 3 ? W.P : 0;
+    const unsigned below = (1u << lane) - 1u;
     const long limit = 8L * W.w * W.h + 64;
     long guard = 0;
-    bool bad = false;
-    auto push = [&](int v) {
-        if (top >= cap) bad = true;
-        else *W.entry(top++) = v;
-    };
-    while (top > 0 && !bad) {
+    while (top > 0) {
         if (++guard > limit) return true;
-        const int idx = *W.entry(--top);
-        const int nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
-        const unsigned me = W.info[idx];
-        unsigned n[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) n[j] = W.info[nb[j]];
-        if (!pop(idx, me, n)) return true;
-        if (walk_type(me) == CELL_EMPTY) W.info[idx] = (uint8_t)((me & ~3u) | CELL_FLUID);
-        // freeSolidNeighbour: a solid neighbour whose normal points here
-        const bool toward[4] = {walk_nx(n[0]) == 1u, walk_nx(n[1]) == 2u, walk_ny(n[2]) == 1u, walk_ny(n[3]) == 2u};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (!toward[j] || walk_type(n[j]) != CELL_SOLID) continue;
-            const unsigned b = n[j] & ~(j < 2 ? 4u : 8u);
-            W.info[nb[j]] = (uint8_t)b;
-            if (walk_mask(b) == 0) push(nb[j]);
-        }
-        // freeEmptyNeighbour
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (walk_type(n[j]) == CELL_EMPTY && walk_mask(n[j]) == 1u) {
-                W.info[nb[j]] = (uint8_t)(n[j] & ~12u);
-                push(nb[j]);
-            }
+        const int idx = *entry(--top);
+        const unsigned me = info[idx], n = lane < 4 ? info[idx + off] : kInert;
+        if (!pop(idx, me, n, off)) return true;
+        if (lane == 0 && walk_type(me) == CELL_EMPTY) info[idx] = (uint8_t)((me & ~3u) | CELL_FLUID);
+        // freeSolidNeighbour, a solid neighbour whose normal points here, for all four,
+        // then freeEmptyNeighbour for all four
+        const unsigned sign = lane < 2 ? walk_nx(n) : walk_ny(n), b = n & ~(lane < 2 ? 4u : 8u);
+        const bool solid = walk_type(n) == CELL_SOLID && sign == ((lane & 1) ? 2u : 1u);
+        const bool empty = walk_type(n) == CELL_EMPTY && walk_mask(n) == 1u;
+        if (solid || empty) info[idx + off] = (uint8_t)(solid ? b : n & ~12u);
+        const unsigned ps = __ballot_sync(0xffffffffu, solid && walk_mask(b) == 0), pe = __ballot_sync(0xffffffffu, empty);
+        if (top + __popc(ps | pe) > cap) return true;
+        if (ps >> lane & 1u) *entry(top + __popc(ps & below)) = idx + off;
+        if (pe >> lane & 1u) *entry(top + __popc(ps) + __popc(pe & below)) = idx + off;
+        top += __popc(ps) + __popc(pe);
+        __syncwarp();
     }
-    return bad;
+    return false;
 }
 
 // extrapolateAverage over the neighbours that are fluid, extrapolateNormal.
@@ -725,103 +719,86 @@ __device__ __forceinline__ double walk_empty(const bool fluid[4], Value value) {
 __device__ __forceinline__ double walk_normal(double ax, double ay, double sx, double sy) {
     return (fabs(ax) * sx + fabs(ay) * sy) / (fabs(ax) + fabs(ay));
 }
-__device__ __forceinline__ int walk_step(unsigned sign) { return sign == 1u ? 1 : sign == 2u ? -1 : 0; }
 
-// The walk with its values left for afterwards.  False: more than kEvents pops or a
-// stack above kWalkStack; nothing but the bytes and the stack has changed then.
-__device__ __forceinline__ bool walk_events(const Quant<double> &Q, const Walk &W, int top, unsigned char *mem, int cells) {
+// The walk with its values left for afterwards.  False: more than kEvents pops, a cell
+// popped twice, or a stack above kWalkStack; nothing but the bytes and the stack has
+// changed then.
+__device__ __forceinline__ bool walk_events(const Quant<double> &Q, const Walk &W, int top, unsigned char *mem, int cells,
+                                            unsigned *flags) {
     double *val = (double *)mem;
     int *cell = (int *)(val + kEvents);
-    short *in = (short *)(cell + kEvents), *lev = in + 4 * kEvents, *last = lev + kEvents;
+    short *done = (short *)(cell + kEvents), *when = done + kEvents;
     const int tid = threadIdx.x, P = W.P;
-    __shared__ int s_n, s_levels, s_ok;
-    for (int i = tid; i < cells; i += blockDim.x) last[i] = kOriginal;
+    __shared__ int s_n, s_ok;
+    for (int i = tid; i < cells; i += blockDim.x) when[i] = -1;
+    for (int i = tid; i < kEvents; i += blockDim.x) done[i] = 0;
     __syncthreads();
-    if (tid == 0) {
-        int n = 0, levels = 0;
-        const bool stopped = top > kWalkStack || walk_run(W, top, kWalkStack, [&](int idx, unsigned me, const unsigned b[4]) {
+    if (tid < 32) {
+        int n = 0;
+        bool twice = false;
+        const bool stopped = top > kWalkStack || walk_run<true>(W, top, kWalkStack, [&](int idx, unsigned, unsigned, int) {
             if (n >= kEvents) return false;
-            int from[4] = {kNoInput, kNoInput, kNoInput, kNoInput};
-            if (walk_type(me) == CELL_EMPTY) {
-                const int nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (walk_type(b[j]) == CELL_FLUID) from[j] = last[nb[j]];
+            if (tid == 0) {
+                twice |= when[idx] >= 0;
+                when[idx] = (short)n;
                 cell[n] = idx;
-            } else {
-                from[0] = last[idx + walk_step(walk_nx(me))];
-                from[1] = last[idx + walk_step(walk_ny(me)) * P];
-                cell[n] = ~idx;
             }
-            int level = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                in[4 * n + j] = (short)from[j];
-                if (from[j] >= 0) level = max(level, lev[from[j]] + 1);
-            }
-            lev[n] = (short)level;
-            levels = max(levels, level + 1);
-            last[idx] = (short)n;
             n++;
             return true;
         });
-        s_n = n;
-        s_levels = levels;
-        s_ok = !stopped;
+        if (tid == 0) {
+            s_n = n;
+            s_ok = !stopped && !twice;
+        }
     }
     __syncthreads();
     if (!s_ok) return false;
-    const int n = s_n, levels = s_levels;
-    // the pops by depth: counts and starts in the stack's place, the order in the bytes'
-    int *start = W.near_stack;
-    unsigned short *order = (unsigned short *)W.info;  // n <= cells / 2 is checked below
-    const bool sorted = 2 * n <= cells && levels < kWalkStack;
-    if (sorted) {
-        for (int i = tid; i <= levels; i += blockDim.x) start[i] = 0;
-        __syncthreads();
-        for (int e = tid; e < n; e += blockDim.x) atomicAdd(start + lev[e], 1);
-        __syncthreads();
-        if (tid < 32) {  // exclusive prefix
-            int base = 0;
-            for (int l0 = 0; l0 <= levels; l0 += 32) {
-                const int v = l0 + tid <= levels ? start[l0 + tid] : 0;
-                int incl = v;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (tid >= o) incl += t;
-                }
-                if (l0 + tid <= levels) start[l0 + tid] = base + incl - v;
-                base += __shfl_sync(0xffffffffu, incl, 31);
+    // every pop takes values of earlier ones only, so the waiting ends
+    const int n = s_n;
+    for (int e0 = tid & ~31; e0 < n; e0 += blockDim.x) {
+        const int e = e0 + (tid & 31);
+        bool open = e < n, average = false;
+        int from[4] = {-1, -1, -1, -1};  // earlier pops; -1: the value in v
+        bool takes[4] = {false, false, false, false};
+        double v[4] = {0.0, 0.0, 0.0, 0.0}, ax = 0.0, ay = 0.0;
+        if (open) {
+            const int idx = cell[e];
+            average = Q.cell[idx] == CELL_EMPTY;
+            ax = Q.nx[idx];
+            ay = Q.ny[idx];
+            const int nb[4] = {average ? idx - 1 : idx + sgn(ax), average ? idx + 1 : idx + sgn(ay) * P, idx - P, idx + P};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int at = when[nb[j]];
+                if (at >= 0 && at < e) from[j] = at;
+                takes[j] = average ? Q.cell[nb[j]] == CELL_FLUID || (Q.cell[nb[j]] == CELL_EMPTY && from[j] >= 0) : j < 2;
+                if (!takes[j]) from[j] = -1;
+                v[j] = Q.src[nb[j]];
             }
         }
-        __syncthreads();
-        for (int e = tid; e < n; e += blockDim.x) order[atomicAdd(start + lev[e], 1)] = (unsigned short)e;
-        __syncthreads();  // start[l] is now the end of depth l
-    }
-    for (int l = 0; l < levels; l++) {
-        const int lo = sorted ? (l > 0 ? start[l - 1] : 0) : 0, hi = sorted ? start[l] : n;
-        for (int i = lo + tid; i < hi; i += blockDim.x) {
-            const int e = sorted ? order[i] : i;
-            if (lev[e] != l) continue;
-            const bool normal = cell[e] < 0;
-            const int idx = normal ? ~cell[e] : cell[e];
-            const short *from = in + 4 * e;
-            if (normal) {
-                const double ax = Q.nx[idx], ay = Q.ny[idx];
-                const int jx = idx + sgn(ax), jy = idx + sgn(ay) * P;
-                val[e] = walk_normal(ax, ay, from[0] >= 0 ? val[from[0]] : Q.src[jx], from[1] >= 0 ? val[from[1]] : Q.src[jy]);
-            } else {
-                const int nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
-                const bool fluid[4] = {from[0] != kNoInput, from[1] != kNoInput, from[2] != kNoInput, from[3] != kNoInput};
-                val[e] = walk_empty(fluid, [&](int j) { return from[j] >= 0 ? val[from[j]] : Q.src[nb[j]]; });
+        for (int spins = 0; __any_sync(0xffffffffu, open); spins++) {
+            bool ready = open;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (open && from[j] >= 0) ready = ready && *(volatile short *)(done + from[j]) != 0;
+            __threadfence_block();
+            if (ready) {
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (from[j] >= 0) v[j] = *(volatile double *)(val + from[j]);
+                *(volatile double *)(val + e) = average ? walk_empty(takes, [&](int j) { return v[j]; }) : walk_normal(ax, ay, v[0], v[1]);
+                __threadfence_block();
+                *(volatile short *)(done + e) = 1;
+                open = false;
+            }
+            if (spins > (1 << 22)) {  // cannot be
+                if (open) atomicOr(flags, FLAG_FLIP_STACK);
+                break;
             }
         }
-        __syncthreads();
     }
-    for (int e = tid; e < n; e += blockDim.x) {
-        const int idx = cell[e] < 0 ? ~cell[e] : cell[e];
-        if (last[idx] == e) Q.src[idx] = val[e];
-    }
+    __syncthreads();
+    for (int e = tid; e < n; e += blockDim.x) Q.src[cell[e]] = val[e];
     __syncthreads();
     return true;
 }
@@ -837,26 +814,31 @@ __global__ void __launch_bounds__(1024) extrap_lifo_kernel(Scene<double> S, unsi
     const Walk W{w, h, P, mode ? (uint8_t *)(walk_smem + 4 * kWalkStack) : Q.ready, (int *)walk_smem, Q.list,
                  mode ? kWalkStack : 0};
     int top = walk_setup(Q, W);
-    const bool done = mode == WALK_EVENTS && walk_events(Q, W, top, walk_smem + 4 * kWalkStack + walk_pad(cells), cells);
+    const bool done = mode == WALK_EVENTS && walk_events(Q, W, top, walk_smem + 4 * kWalkStack + walk_pad(cells), cells, S.flags);
     if (!done) {
         if (mode == WALK_EVENTS) {  // too many pops: from the start, value by value
             __syncthreads();
             top = walk_setup(Q, W);
         }
-        if (tid == 0) {
-            const bool bad = walk_run(W, top, 2L * P * (S.h + 2), [&](int idx, unsigned me, const unsigned b[4]) {
+        if (tid < 32) {
+            const bool bad = walk_run<false>(W, top, 2L * P * (S.h + 2), [&](int idx, unsigned me, unsigned b, int off) {
+                double out;
                 if (walk_type(me) == CELL_EMPTY) {
-                    const int nb[4] = {idx - 1, idx + 1, idx - P, idx + P};
-                    const bool fluid[4] = {walk_type(b[0]) == CELL_FLUID, walk_type(b[1]) == CELL_FLUID,
-                                           walk_type(b[2]) == CELL_FLUID, walk_type(b[3]) == CELL_FLUID};
-                    src[idx] = walk_empty(fluid, [&](int j) { return src[nb[j]]; });
+                    const unsigned fl = __ballot_sync(0xffffffffu, tid < 4 && walk_type(b) == CELL_FLUID);
+                    const double v = src[idx + off];
+                    const bool fluid[4] = {(fl & 1u) != 0, (fl & 2u) != 0, (fl & 4u) != 0, (fl & 8u) != 0};
+                    const double vs[4] = {__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1),
+                                          __shfl_sync(0xffffffffu, v, 2), __shfl_sync(0xffffffffu, v, 3)};
+                    out = walk_empty(fluid, [&](int j) { return vs[j]; });
                 } else {
                     const double ax = Q.nx[idx], ay = Q.ny[idx];
-                    src[idx] = walk_normal(ax, ay, src[idx + sgn(ax)], src[idx + sgn(ay) * P]);
+                    out = walk_normal(ax, ay, src[idx + sgn(ax)], src[idx + sgn(ay) * P]);
                 }
+                __syncwarp();
+                if (tid == 0) src[idx] = out;
                 return true;
             });
-            if (bad) atomicOr(S.flags, FLAG_FLIP_STACK);
+            if (bad && tid == 0) atomicOr(S.flags, FLAG_FLIP_STACK);
         }
         __syncthreads();
     }
