@@ -271,7 +271,7 @@ int ifl_get_timing(ifl_solver *s, ifl_timing *out);
  * synchronised.
  *
  * Every intermediate array lives in one fixed device array inside the
- * library (about 8.4 MB, held by every GPU that loads the library until the
+ * library (about 9.1 MB, held by every GPU that loads the library until the
  * process exits).  Limit: the grid must fit 2304 strip-diagonals, i.e.
  * ceil(h/32) * round_up(w + 31, 16) <= 2304 (for example 256 x 256); larger
  * grids return IFL_ERR_UNSUPPORTED without touching the GPU.  It calls no
@@ -313,11 +313,12 @@ typedef struct {
 
 typedef struct {
     /* Shape of the batched PCG launch: threads per block (32, 64, 128 or 256),
-     * strips per block, bulk-copy ring stages.  threads = 0: autotune at the
-     * first update (each candidate shape runs a few pinned PCG iterations of
-     * the real system; the fastest is kept, unless the home shape, the first
-     * candidate, is within 5 % of it: such a short trial cannot separate
-     * closer shapes). */
+     * strips per block, bulk-copy ring stages (a request: a block gets at
+     * least 128 threads per strip, and fewer strips or stages where threads or
+     * shared memory do not hold more).  threads = 0: autotune at the first
+     * update (each candidate shape runs a few pinned PCG iterations of the real
+     * system; the fastest is kept, unless the home shape, the first candidate,
+     * is within 5 % of it: such a short trial cannot separate closer shapes). */
     int32_t threads, strips_per_block, stages;
     int32_t use_graph;        /* 1: replay each step as one CUDA graph (default) */
     int32_t tune_iterations;  /* PCG iterations per autotuning trial (default 8) */

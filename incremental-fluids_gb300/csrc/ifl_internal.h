@@ -171,11 +171,12 @@ struct PcgConfig {
     long long wait_limit = 0;  // polls of one device-side wait before it gives up; 0: about a second
 };
 
-// Launch shape of the batched PCG kernel (chosen by the batch autotuner).
+// Launch shape of the batched PCG kernel (chosen by the batch autotuner); a request
+// that pcg_shape (pcg_job.cuh) fits to threads and shared memory.
 struct PcgShape {
     int threads;  // 32, 64, 128 or 256 threads per block
     int K;        // strips (sweeping warps) per block, <= threads / 32
-    int stages;   // bulk-copy ring stages per sweeping warp, 2..4
+    int stages;   // ring stages per strip, 2..4
 };
 
 // Launchers (stream-ordered, no host synchronisation).
