@@ -309,8 +309,13 @@ cudaError_t launch_single(PcgArgs<F> A, const PcgScratch &X, const PcgConfig &cf
     if (e == cudaSuccess)
         e = cudaMemsetAsync(X.halo, 0xff, pcg_halo_words(sd) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
+    // FP32 grids with more chunks than the warps of 256-thread blocks (above about
+    // 550^2): twice the warps for the elementwise passes.  Cycles per iteration of
+    // matvec and AXPYs, without their barriers, 256 and 512 threads: 768^2 33K and 28K,
+    // 1536^2 88K and 58K; smaller grids only have more warps at the barriers.
+    const int threads = sizeof(F) == 4 && pcg_chunks(sd) > (size_t)sms * kSingleThreads / 32 ? kMaxThreads<F> : kSingleThreads;
     void *args[] = {&A};
-    return cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kSingleThreads), args, smem, st);
+    return cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), args, smem, st);
 }
 
 }  // namespace
