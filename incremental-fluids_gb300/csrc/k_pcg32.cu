@@ -31,10 +31,10 @@
 // four cycles for every instruction, beside a dependency chain per wavefront
 // step of a shuffle (25 cycles) and six fused multiply-adds (5 each).  So a step
 // does eight cells of every lane, nothing in it depends on the position in the
-// grid (the padding is computed along), and two more warps per strip take from
+// grid (the padding is computed along), and three more warps per strip take from
 // the sweeping warp what is not on the chain: a loader fills a ring in shared
-// memory and takes the neighbouring strip's boundary row, and in the backward
-// sweep a preparer forms dd y and sigma.  What is left per step is 6 loads of 16
+// memory, a taker folds the neighbouring strip's boundary row into the operands,
+// and in the backward sweep a preparer forms dd y and sigma.  What is left per step is 6 loads of 16
 // bytes from shared memory, 16 fused multiply-adds, two shuffles and three
 // stores: 150 cycles, of which the multiply-adds are 63, the loads 45, the
 // stores 30 (timed with each left out).
