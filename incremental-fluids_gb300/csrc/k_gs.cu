@@ -146,10 +146,7 @@ __device__ __forceinline__ bool is_zero(double x) { return (((unsigned)__double2
 // Out of line: inline, the compiler divides first and selects after.
 __device__ __noinline__ double divide(double x, double d) { return x / d; }
 
-// BLOCKS: blocks that an SM has to hold at least; 1 leaves the compiler the registers
-// it likes (96), 7 seats a worker for each of 4096 strips (72, with spills).
-template <int BLOCKS>
-__global__ void __launch_bounds__(32 * kBlockWarps, BLOCKS) gs_kernel(GsArgs A) {
+__global__ void __launch_bounds__(32 * kBlockWarps) gs_kernel(GsArgs A) {
     extern __shared__ unsigned char spread[];  // spreads the workers over the SMs; never touched
     (void)spread;
     const int lane = threadIdx.x & 31, worker = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -380,16 +377,11 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     // time per step with two workers on an SM)
     const int share = (sd.S * A.J + sms - 1) / sms;
     const int warps = std::min(share, kBlockWarps), smem = share > kBlockWarps ? 0 : std::min(optin, 120 * 1024);
-    auto kernel = gs_kernel<1>;
     if (smem) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = cudaFuncSetAttribute(gs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * warps, smem);
-    if (e == cudaSuccess && (long)per_sm * sms * warps < sd.S) {
-        kernel = gs_kernel<7>;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * warps, smem);
-    }
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gs_kernel, 32 * warps, smem);
     if (e != cudaSuccess) return e;
     if ((long)per_sm * sms * warps < (long)sd.S * A.J) A.J = (int)((long)per_sm * sms * warps / sd.S);
     if (A.J < 1) return cudaErrorCooperativeLaunchTooLarge;
@@ -414,7 +406,7 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     e = cudaMemsetAsync(X.gs, 0, ring_words(sd, A.L) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     void *args[] = {&A};
-    return cudaLaunchCooperativeKernel((const void *)kernel, dim3((sd.S * A.J + warps - 1) / warps), dim3(32 * warps), args, (size_t)smem, st);
+    return cudaLaunchCooperativeKernel((const void *)gs_kernel, dim3((sd.S * A.J + warps - 1) / warps), dim3(32 * warps), args, (size_t)smem, st);
 }
 
 template cudaError_t launch_gs<double>(const Scene<double> &, const PcgScratch &, double, int, int, cudaStream_t,

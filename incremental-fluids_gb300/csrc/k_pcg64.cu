@@ -230,16 +230,29 @@ __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double b
 
 // ---- the reference's arithmetic, with sums over chunks of kRefChunk diagonals
 
-// Dot product of two operands by the chunk: the warps of a block form a chunk's
-// products, a diagonal each in turn, and leave them in shared memory; one warp
-// then adds them in order.  (A warp per chunk, start to end, takes four times as
-// long: 16 diagonals of up to 21 FP64 instructions, one after the other.)
+// Dot product of two operands by the chunk.  Where every warp of the team has one, a
+// warp takes its chunks start to end.  Otherwise the warps of a block form a chunk's
+// products, a diagonal each in turn, and leave them in shared memory, and one warp
+// adds them in order: a quarter of the time for a team with warps to spare (203x150
+// alone: 11.6K instead of 20.0K cycles for the matvec), but the others wait for the
+// sum (512 scenes in a batch: a third more time).
 template <typename Product>
 __device__ __forceinline__ void ref_dot(const PcgArgs<double> &A, const Team &T, double *partials, Product product) {
     __shared__ double prod[kRefChunk][32];
     const SDIdx sd = A.sd;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int c = T.rank; c < ref_chunks(sd); c += T.size) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, n = ref_chunks(sd);
+    if (n >= T.size * warps) {
+        for (int c = warp * T.size + T.rank; c < n; c += T.size * warps) {
+            const int s = c * kRefChunk / sd.D, d0 = c * kRefChunk - s * sd.D;
+            const Cells C(sd, s, lane);
+            double acc = 0.0;
+            for (int u = 0; u < kRefChunk; u++) acc = acc + product(C, s, d0 + u);
+            acc = warp_sum(acc);
+            if (lane == 0) partials[c] = acc;
+        }
+        return;
+    }
+    for (int c = T.rank; c < n; c += T.size) {
         const int s = c * kRefChunk / sd.D, d0 = c * kRefChunk - s * sd.D;  // a chunk lies inside one strip
         const Cells C(sd, s, lane);
         for (int u = warp; u < kRefChunk; u += warps) prod[u][lane] = product(C, s, d0 + u);

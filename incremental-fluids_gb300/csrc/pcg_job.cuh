@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kMaxThreads<F>, 1) pcg_kernel(PcgArgs<F> A) {
 
 // Many independent scenes in one cooperative launch (see BatchTeams).
 template <typename F>
-__global__ void __launch_bounds__(kMaxThreads<F>, 1)
+__global__ void __launch_bounds__(kBatchThreads, 1)
     pcg_batch_kernel(const PcgArgs<F> *jobs, BatchTeams B, int mode, int heat, int pinned, int K, int stages) {
     __shared__ double sm[3 * kSums];
     __shared__ PcgArgs<F> sA;
@@ -274,7 +274,7 @@ size_t pcg_smem(int K, int D, int stages) { return ring_offset(K, D) + (size_t)K
 // allow (smem: bytes of a block).
 template <typename F>
 void pcg_shape(int threads, int D, size_t smem_max, int *block, int *K, int *stages) {
-    *K = std::min(*K, kMaxThreads<F> / (32 * kRoles));
+    *K = std::min(*K, kBatchThreads / (32 * kRoles));
     while (*stages > 2 && pcg_smem<F>(*K, D, *stages) > smem_max) (*stages)--;
     while (*K > 1 && pcg_smem<F>(*K, D, *stages) > smem_max) (*K)--;
     *block = std::max(threads, 32 * kRoles * *K);

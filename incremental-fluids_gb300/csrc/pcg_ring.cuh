@@ -45,9 +45,11 @@ template <typename F> constexpr unsigned kVecBytes = Lay<F>::kSteps * Lay<F>::kC
 template <typename F> constexpr unsigned kHaloAt = 4u * kVecBytes<F>;       // its halo words, behind four arrays
 template <typename F> constexpr unsigned kStageBytes = kHaloAt<F> + 128u;   // a ring stage
 constexpr int kMaxStages = 8;
-// Threads of a block: the FP32 form's batched passes are bound by what 128-thread
-// blocks an SM holds (three at 160 registers, four at 128: 512 scenes of 64^2 to
-// 768^2 in 316 instead of 381 ms), the FP64 form spills below 168.
+// Threads of a block at most.  The batched passes are bound by how many 128-thread
+// blocks an SM holds, three at 160 registers and four at 128 (512 FP32 scenes of 64^2
+// to 768^2: 381 and 316 ms; 256 FP64 scenes to 512^2: 427 and 375 ms); the FP64
+// form's single solves have a block per SM and would only spill.
+constexpr int kBatchThreads = 512;
 template <typename F> constexpr int kMaxThreads = sizeof(F) == 4 ? 512 : 384;
 constexpr int kRoles = 4;   // warps that work on one strip: sweep, load, prepare, take
 constexpr int kSums = 16;   // partial sums of a reduction (see total_of)
