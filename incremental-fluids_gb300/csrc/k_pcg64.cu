@@ -235,7 +235,7 @@ __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double b
 // products, a diagonal each in turn, and leave them in shared memory, and one warp
 // adds them in order: a quarter of the time for a team with warps to spare (203x150
 // alone: 11.6K instead of 20.0K cycles for the matvec), but the others wait for the
-// sum (512 scenes in a batch: a third more time).
+// sum.
 template <typename Product>
 __device__ __forceinline__ void ref_dot(const PcgArgs<double> &A, const Team &T, double *partials, Product product) {
     __shared__ double prod[kRefChunk][32];
