@@ -381,13 +381,17 @@ __device__ __noinline__ void coefs(const PcgArgs<F> &A, int c_begin, int c_end, 
             const size_t k = (size_t)row * Lay<F>::kCells + idx;
             const double pcv = A.pc[k], p2 = !(A.nb[k] & NB_SELF) ? 0.0 : REF ? pcv : pcv * pcv;
             const F sign = REF ? F(1) : F(-1), dd = from_f64<F>(p2);
-            const F va = sign * from_f64<F>(to_f64(A.ax[k]) * p2), vb = sign * from_f64<F>(to_f64(A.ay[k]) * p2);
+            // A neighbour that does not exist has a zero coefficient, whatever the matrix
+            // holds there: lane 31 (0) of a strip without one sees its own previous value.
+            const bool right = x + 1 < sd.W, upper = y + 1 < sd.H;
+            const F va = sign * from_f64<F>(right ? to_f64(A.ax[k]) * p2 : 0.0),
+                    vb = sign * from_f64<F>(upper ? to_f64(A.ay[k]) * p2 : 0.0);
             *coef<REF, true>(A, k, REF ? R_RIGHT : C_RIGHT) = va;
             *coef<REF, true>(A, k, REF ? R_UP : C_UP) = vb;
             *coef<REF, true>(A, k, REF ? R_PC : C_DD) = dd;
             if (REF) *coef<REF, false>(A, k, R_PC) = dd;
-            if (x + 1 < sd.W) *coef<REF, false>(A, sd.slot(x + 1, y), C_LEFT) = va;
-            if (y + 1 < sd.H) *coef<REF, false>(A, sd.slot(x, y + 1), C_DOWN) = vb;
+            if (right) *coef<REF, false>(A, sd.slot(x + 1, y), C_LEFT) = va;
+            if (upper) *coef<REF, false>(A, sd.slot(x, y + 1), C_DOWN) = vb;
         }
     }
 }
