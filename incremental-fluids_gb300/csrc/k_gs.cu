@@ -34,7 +34,9 @@
 // the verdict of sweep k - L is in and open.  So up to L - 1 sweeps run ahead of
 // the decision; their buffers are dropped.  B = L + 1 buffers: sweep k + B starts
 // after sweep k + 1 is complete (nobody reads sweep k any more) and found not
-// converged (sweep k is not the result).
+// converged (sweep k is not the result).  A worker that has no sweep left to ask
+// before waits for an entry of its own (`decided`): the last sweeps, and with
+// them their verdicts, do not exist if an earlier one converged.
 //
 // 600 sweeps at 128 x 128: 2.2 ms; 116 ms with one sweep and the head of the next in
 // flight, a hand-over with a fence every four diagonals and a division per cell.
@@ -74,6 +76,7 @@ struct GsArgs {
     Entry *down, *up;      // -scale p of every strip's last and first row, by buffer, strip and column
     Entry *change;         // L + 1 x S: largest change of a sweep up to strip s
     Entry *verdict;        // L + 1: first converged sweep + 1, or 0 (as bits of v)
+    Entry *decided;        // the same for the whole solve, written once
     unsigned long long *abort;
 };
 
@@ -300,15 +303,16 @@ __global__ void __launch_bounds__(32 * kBlockWarps) gs_kernel(GsArgs A) {
         gs_publish(A.change + (size_t)b * S + s, change, tag);
         if (!above) {
             int v = k > 0 ? (int)__double_as_longlong(gs_wait(A, A.verdict + (k - 1) % B, tag - 1)) : 0;
-            if (v == 0 && A.pinned < 0 && change < kGsTol) v = k + 1;
+            const bool open = v == 0;
+            if (open && A.pinned < 0 && change < kGsTol) v = k + 1;
+            if (open && (v != 0 || k == nsweeps - 1)) gs_publish(A.decided, __longlong_as_double((long long)v), 1ull);
             gs_publish(A.verdict + b, __longlong_as_double((long long)v), tag);
         }
     }
     int final_sweeps = nsweeps;
     double maxDelta = 0.0;
     if (nsweeps > 0 && !dead) {
-        if (stop == 0)
-            stop = (int)__double_as_longlong(gs_wait(A, A.verdict + (nsweeps - 1) % B, (unsigned long long)nsweeps + 1));
+        if (stop == 0) stop = (int)__double_as_longlong(gs_wait(A, A.decided, 1ull));
         if (stop != 0) final_sweeps = stop;
         maxDelta = gs_wait(A, A.change + (size_t)((final_sweeps - 1) % B) * S + S - 1, (unsigned long long)final_sweeps + 1);
         dead = __any_sync(FULL, gs_aborted(A));
@@ -328,8 +332,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps) gs_kernel(GsArgs A) {
 }
 
 size_t ring_words(const SDIdx &sd, int L) {
-    // (64 entries more: loads beyond a row's or a strip's last column, which are ignored)
-    return ((size_t)(L + 1) * (sd.total() + 2 * (size_t)sd.S * sd.W + sd.S + 1) + 64) * 2 + 2;
+    // (64 entries more: loads beyond a row's or a strip's last column, which are ignored; `decided`, `abort`)
+    return ((size_t)(L + 1) * (sd.total() + 2 * (size_t)sd.S * sd.W + sd.S + 1) + 64 + 1) * 2 + 2;
 }
 
 // Sweeps in flight (J) and the lead over the verdict (L).  A sweep follows the one
@@ -401,7 +405,8 @@ cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int lim
     A.up = A.down + rows;
     A.change = A.up + rows;
     A.verdict = A.change + (size_t)(A.L + 1) * sd.S;
-    A.abort = (unsigned long long *)(A.verdict + A.L + 1 + 64);
+    A.decided = A.verdict + A.L + 1 + 64;
+    A.abort = (unsigned long long *)(A.decided + 1);
     // every tag back to `empty`: the whole of it, 47 MB at 128 x 128 (10 us)
     e = cudaMemsetAsync(X.gs, 0, ring_words(sd, A.L) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
