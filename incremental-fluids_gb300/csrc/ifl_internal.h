@@ -106,7 +106,7 @@ struct Scene {
     F *rf;             // r in storage precision for the substitutions (aliases r for FP64)
     F *z, *sa, *sb;
     F *adiag, *ax, *ay;
-    F *mic;            // MIC(0) apply operands, five values per slot (pcg_ring.cuh)
+    F *mic;            // MIC(0) apply operands, five or six values per slot (pcg_ring.cuh)
     double *pc;        // MIC(0) factor, FP64
     uint8_t *nb;
     F *udens, *vdens;

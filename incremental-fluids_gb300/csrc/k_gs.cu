@@ -343,8 +343,10 @@ size_t ring_words(const SDIdx &sd, int L) {
 // and 3.2 with 120, so half as many as steps; and no more than four workers per SM:
 // an FP64 instruction takes 64 cycles of a warp with one worker on an SM and 76
 // with four.  The verdict of a sweep comes after the last strip's last step (36
-// steps per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes,
-// with fewer sweeps in flight.
+// steps per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes
+// with fewer sweeps in flight, but not below the three buffers of 16-byte entries
+// that one sweep and its successor need: 0.8 GB at 4096^2, 52 GB at 32768^2, where
+// a handle has fewer arrays for it (solver.cu).
 constexpr size_t kRingBytes = (size_t)512 << 20;
 void gs_plan(const SDIdx &sd, int sms, int *J, int *L) {
     const long steps = sd.W + 31, until = steps + 36L * (sd.S - 1) + 8;

@@ -46,7 +46,7 @@ struct PcgArgs {
     SDIdx sd;
     const F *adiag, *ax, *ay;
     double *pc;
-    F *mic;  // MIC(0) apply operands, five values per slot (pcg_ring.cuh)
+    F *mic;  // MIC(0) apply operands, five or six values per slot (pcg_ring.cuh)
     const uint8_t *nb;
     double *r, *p, *as;
     F *rf;  // r in storage precision for the substitutions (== r when F is double)

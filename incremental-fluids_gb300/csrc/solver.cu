@@ -502,14 +502,19 @@ class SolverImpl final : public SolverBase {
         S_.p = c.take<double>(base, NS);
         S_.z = c.take<F>(base, NS);
         S_.sa = c.take<F>(base, NS);
-        S_.sb = c.take<F>(base, NS);
-        S_.as = c.take<double>(base, NS);
+        // Work arrays that no field names exist where a solve uses them: not beside the
+        // Gauss-Seidel solve's ring, and the MIC(0) operands as many as its form has
+        // (pcg_ring.cuh: five values per slot in L D L^T form, six in the reference's own).
+        const bool pcg = prm_.variant > IFL_GS;
+        const int mic = sizeof(F) == 8 && prm_.variant >= IFL_SOLID ? 6 : 5;
+        S_.sb = pcg && !f32_solves_ ? c.take<F>(base, NS) : nullptr;
+        S_.as = pcg ? c.take<double>(base, NS) : nullptr;
         if (sizeof(F) == 8) S_.rf = (F *)S_.r;
-        else S_.rf = c.take<F>(base, NS);
+        else S_.rf = pcg ? c.take<F>(base, NS) : nullptr;
         S_.adiag = c.take<F>(base, NS);
         S_.ax = c.take<F>(base, NS);
         S_.ay = c.take<F>(base, NS);
-        S_.mic = c.take<F>(base, (sizeof(F) == 8 ? 6 : 5) * NS);
+        S_.mic = pcg && !f32_solves_ ? c.take<F>(base, mic * NS) : nullptr;
         S_.pc = c.take<double>(base, NS);
         S_.nb = c.take<uint8_t>(base, NS);
         if (prm_.variant >= IFL_VARDENS) {
