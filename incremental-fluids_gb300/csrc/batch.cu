@@ -389,12 +389,19 @@ class BatchImpl final : public BatchBase {
         // smaller, round-robin teams for the step time the grid could hold
         // spent fewer block-microseconds but packed worse on GB300: 1.12-1.24 s
         // against 1.00 s per step of the 512-scene batch.)
+        // A grid too small for a team of every class leaves out the largest.
+        const int K = shape_.K;
         std::vector<int> cls(n_);
-        for (int i = 0; i < n_; i++) {
-            const int cover = pow2ceil((scene(i).sd.S + shape_.K - 1) / shape_.K);
-            int c = 0;
-            while ((1 << c) < cover && (1 << c) < 128) c++;
-            cls[i] = c;
+        for (int most = 7, need = 0; most >= 0; most--) {
+            for (int i = 0; i < n_; i++) {
+                const int cover = pow2ceil((scene(i).sd.S + K - 1) / K);
+                int c = 0;
+                while ((1 << c) < cover && c < most) c++;
+                cls[i] = c;
+                need |= 1 << c;
+            }
+            if (need <= pcg_batch_grid(plan_)) break;
+            need = 0;
         }
         const PlanWork work = [this](int i, int g) { return plan_cost(i, g); };
         if (pcg_batch_schedule(plan_, cls.data(), work, st_) != 0) {
