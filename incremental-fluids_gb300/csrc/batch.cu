@@ -373,9 +373,9 @@ class BatchImpl final : public BatchBase {
     // (512-scene batch, 128-thread blocks, three to an SM).
     double plan_cost(int i, int g) const {
         constexpr bool f32 = sizeof(F) == 4;
-        constexpr double kTau = f32 ? 0.14 : 0.11, kLag = f32 ? 6.0 : 6.0, kElemNs = f32 ? 7.7 : 10.0;
+        constexpr double kTau = f32 ? 0.14 : 0.11, kLag = 6.0, kElemNs = f32 ? 7.7 : 10.0;
         const Scene<F> &S = scene(i);
-        const int P = g * shape_.K, Sn = S.sd.S;
+        const int P = g * pcg_batch_strips(plan_), Sn = S.sd.S;
         const double Dt = S.sd.D * kTau;
         const double sweep = std::max((Sn - 1) * kLag + Dt, ((Sn - 1) / P) * Dt + ((Sn - 1) % P) * kLag + Dt);
         const double elem = 1e-3 * kElemNs * (double)S.w * S.h / g * (128.0 / pcg_batch_block(plan_));
@@ -389,8 +389,10 @@ class BatchImpl final : public BatchBase {
         // smaller, round-robin teams for the step time the grid could hold
         // spent fewer block-microseconds but packed worse on GB300: 1.12-1.24 s
         // against 1.00 s per step of the 512-scene batch.)
-        // A grid too small for a team of every class leaves out the largest.
-        const int K = shape_.K;
+        // Strips per block as the launch has them, not as the shape was requested
+        // (eight become four).  A grid too small for a team of every class leaves
+        // out the largest.
+        const int K = pcg_batch_strips(plan_);
         std::vector<int> cls(n_);
         for (int most = 7, need = 0; most >= 0; most--) {
             for (int i = 0; i < n_; i++) {

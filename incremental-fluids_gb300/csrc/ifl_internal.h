@@ -221,6 +221,7 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
 void pcg_batch_destroy(PcgBatchPlan *P);
 int pcg_batch_grid(const PcgBatchPlan *P);
 int pcg_batch_block(const PcgBatchPlan *P);  // threads of a block of its launch
+int pcg_batch_strips(const PcgBatchPlan *P);  // strips a block sweeps at a time
 size_t pcg_batch_table_bytes(const PcgBatchPlan *P);  // team/queue tables uploaded per schedule
 // Estimated time of scene i's solves on a team of g blocks (planner cost model).
 using PlanWork = std::function<double(int i, int g)>;

@@ -334,6 +334,7 @@ void pcg_batch_destroy(PcgBatchPlan *P) {
 
 int pcg_batch_grid(const PcgBatchPlan *P) { return P->grid; }
 int pcg_batch_block(const PcgBatchPlan *P) { return P->block; }
+int pcg_batch_strips(const PcgBatchPlan *P) { return P->K; }
 size_t pcg_batch_table_bytes(const PcgBatchPlan *P) { return P->tab_bytes; }
 void pcg_batch_set_max_team(PcgBatchPlan *P, int blocks) { P->max_team = blocks > 0 ? blocks : 128; }
 
