@@ -150,12 +150,17 @@ __device__ __forceinline__ double cubic_pulse(double x) {
 
 template <typename F> __device__ __forceinline__ F lerp1(F a, F b, F x) { return a * (F(1.0) - x) + b * x; }
 
+// The cell of a sample position that is clamped to [0, n - 1.001].  A NaN passes
+// the clamp and converts to the lowest integer (FP64) or zero (FP32): cell 0 then,
+// and its offset from there, still NaN, makes the sample NaN.
+template <typename F> __device__ __forceinline__ int sample_cell(F x) { return max((int)x, 0); }
+
 // FluidQuantity::lerp (3-conjugate-gradients/Fluid.cpp:121-133) on a pitched grid.
 template <typename F>
 __device__ __forceinline__ F q_lerp(const F *__restrict__ src, int P, int w, int h, F ox, F oy, F x, F y) {
     x = smin(smax(x - ox, F(0.0)), F(w) - F(1.001));
     y = smin(smax(y - oy, F(0.0)), F(h) - F(1.001));
-    int ix = (int)x, iy = (int)y;
+    int ix = sample_cell(x), iy = sample_cell(y);
     x -= F(ix);
     y -= F(iy);
     const F *r0 = src + ix + (size_t)iy * P;

@@ -899,7 +899,7 @@ template <typename F>
 __device__ __forceinline__ F q_cerp(const F *__restrict__ src, int P, int w, int h, F ox, F oy, F x, F y) {
     x = smin(smax(x - ox, F(0.0)), F(w) - F(1.001));
     y = smin(smax(y - oy, F(0.0)), F(h) - F(1.001));
-    int ix = (int)x, iy = (int)y;
+    int ix = sample_cell(x), iy = sample_cell(y);
     x -= F(ix);
     y -= F(iy);
     int x0 = max(ix - 1, 0), x1 = ix, x2 = ix + 1, x3 = min(ix + 2, w - 1);
