@@ -204,7 +204,8 @@ __device__ __forceinline__ KindGeo kind_geo(const Scene<double> &S, const FlipSt
     return g;
 }
 // fromParticles' clamped sample position relative to the grid
-// (8-flip/Fluid.cpp:669-673): max(0.5, min(w - 1.5, p - o)).
+// (8-flip/Fluid.cpp:669-673): max(0.5, min(w - 1.5, p - o)); a NaN becomes n - 1.5,
+// as in the reference.
 __device__ __forceinline__ double clamp_sample(double p, double o, int n) {
     return smax(0.5, smin(n - 1.5, p - o));
 }
@@ -458,7 +459,7 @@ __device__ __forceinline__ double lerp_diff(const Scene<double> &S, int t, doubl
     const Quant<double> &Q = S.q[t];
     x = smin(smax(x - Q.ox, 0.0), Q.w - 1.001);
     y = smin(smax(y - Q.oy, 0.0), Q.h - 1.001);
-    const int ix = (int)x, iy = (int)y;
+    const int ix = sample_cell(x), iy = sample_cell(y);
     x -= ix;
     y -= iy;
     const long i0 = ix + (long)iy * S.P, i1 = i0 + S.P;

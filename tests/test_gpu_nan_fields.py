@@ -51,3 +51,34 @@ def test_nan_velocity(ifl, variant, precision):
         # the cells whose backtrace reads the face, a few rows and columns around it
         assert bad.any() and bad[:12, :13].sum() == bad.sum()
         assert np.array_equal(a[~bad], b[~bad])
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32-solves"])
+def test_flip_scene_that_goes_nan(ifl, precision):
+    g = ifl.FluidSolver(W, H, 0.1, 0.25, 0.01, [ifl.SolidBox(*BODY)], variant=ifl.FLIP, precision=precision)
+    g.flip_init()
+    a = [g.particles(k).copy() for k in range(6)]
+    a[4][7] = np.nan  # one particle's velocity: the pressure solve spreads it
+    g.set_particles(a)
+    for _ in range(3):
+        g.update(DT)
+    assert g.stats()[2] & 1 == 0
+    assert np.isnan(g.particles(0)).any() and g.particle_count() <= 12 * W * H
+
+
+def test_particle_at_a_nan_position(ifl):
+    """Grid to particles and the advection: that particle's values and position become NaN, no other's."""
+    out = []
+    for nan in (False, True):
+        g = ifl.FluidSolver(W, H, 0.1, 0.25, 0.01, [ifl.SolidBox(*BODY)], variant=ifl.FLIP)
+        g.flip_init()
+        a = [g.particles(k).copy() for k in range(6)]
+        if nan:
+            a[0][9] = np.nan
+        g.set_particles(a)
+        _fields(g, False)
+        for ph in (ifl.PH_FLIP_COPY, ifl.PH_G2P, ifl.PH_PADVECT):
+            g.run_phase(ph, DT)
+        out.append([g.particles(k) for k in range(6)])
+    for a, b in zip(*out):
+        assert np.isnan(b[9]) and np.array_equal(np.delete(a, 9), np.delete(b, 9))
