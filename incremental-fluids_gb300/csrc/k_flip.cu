@@ -209,15 +209,18 @@ __device__ __forceinline__ KindGeo kind_geo(const Scene<double> &S, const FlipSt
 __device__ __forceinline__ double clamp_sample(double p, double o, int n) {
     return smax(0.5, smin(n - 1.5, p - o));
 }
+// Base node of a particle in the buckets.
+__device__ __forceinline__ int base_node(const KindGeo &g, double px, double py) {
+    const int bx = (int)clamp_sample(px, g.ox, g.w), by = (int)clamp_sample(py, g.oy, g.h);
+    return g.off + bx + by * g.w;
+}
 
 __global__ void p2g_bucket_kernel(Scene<double> S, FlipState X) {
     const int N = X.ctl[FC_COUNT];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const double px = X.px[i], py = X.py[i];
         for (int k = 0; k < 3; k++) {
-            const KindGeo g = kind_geo(S, X, k);
-            const int bx = (int)clamp_sample(px, g.ox, g.w), by = (int)clamp_sample(py, g.oy, g.h);
-            const int key = g.off + bx + by * g.w;
+            const int key = base_node(kind_geo(S, X, k), px, py);
             X.brank[(long)k * X.cap + i] = (int)atomicAdd(&X.bcount[key], 1ull);
         }
     }
@@ -228,28 +231,57 @@ __global__ void p2g_scatter_kernel(Scene<double> S, FlipState X) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const double px = X.px[i], py = X.py[i];
         for (int k = 0; k < 3; k++) {
-            const KindGeo g = kind_geo(S, X, k);
-            const int bx = (int)clamp_sample(px, g.ox, g.w), by = (int)clamp_sample(py, g.oy, g.h);
-            const int key = g.off + bx + by * g.w;
+            const int key = base_node(kind_geo(S, X, k), px, py);
             X.blist[X.bstart[key] + X.brank[(long)k * X.cap + i]] = i;
         }
     }
 }
 
-// Buckets hold a few particles each: insertion sort by particle index.
-__global__ void p2g_sort_kernel(FlipState X) {
-    const int key = blockIdx.x * blockDim.x + threadIdx.x;
-    if (key >= X.node_off[3]) return;
-    int *b = X.blist + X.bstart[key];
-    const int n = (int)(X.bstart[key + 1] - X.bstart[key]);
-    for (int i = 1; i < n; i++) {
-        const int v = b[i];
-        int j = i - 1;
-        while (j >= 0 && b[j] > v) {
-            b[j + 1] = b[j];
-            j--;
+// Buckets hold a few particles each: insertion sort by particle index.  Infinite or
+// NaN velocities leave all particles in a few buckets, where that would take the
+// square of their number: above kSortedAlone the block lists such a bucket's
+// particles anew, in order, from all particles.
+constexpr int kSortThreads = 256, kSortedAlone = 256;
+__global__ void __launch_bounds__(kSortThreads) p2g_sort_kernel(Scene<double> S, FlipState X) {
+    __shared__ int s_big[kSortThreads], s_nbig, s_count[kSortThreads / 32];
+    const int key = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_nbig = 0;
+    __syncthreads();
+    if (key < X.node_off[3]) {
+        int *b = X.blist + X.bstart[key];
+        const int n = (int)(X.bstart[key + 1] - X.bstart[key]);
+        if (n > kSortedAlone) s_big[atomicAdd(&s_nbig, 1)] = key;
+        for (int i = 1; i < (n > kSortedAlone ? 0 : n); i++) {
+            const int v = b[i];
+            int j = i - 1;
+            while (j >= 0 && b[j] > v) {
+                b[j + 1] = b[j];
+                j--;
+            }
+            b[j + 1] = v;
         }
-        b[j + 1] = v;
+    }
+    __syncthreads();
+    const int N = X.ctl[FC_COUNT];
+    for (int k = 0; k < s_nbig; k++) {
+        const int big = s_big[k];
+        const KindGeo g = kind_geo(S, X, big < X.node_off[1] ? 0 : big < X.node_off[2] ? 1 : 2);
+        int *b = X.blist + X.bstart[big];
+        for (int i0 = 0; i0 < N; i0 += kSortThreads) {
+            const int i = i0 + threadIdx.x;
+            const bool mine = i < N && base_node(g, X.px[i], X.py[i]) == big;
+            const unsigned bal = __ballot_sync(0xffffffffu, mine);
+            if (lane == 0) s_count[warp] = __popc(bal);
+            __syncthreads();
+            int before = __popc(bal & ((1u << lane) - 1u)), all = 0;
+            for (int j = 0; j < kSortThreads / 32; j++) {
+                before += j < warp ? s_count[j] : 0;
+                all += s_count[j];
+            }
+            if (mine) b[before] = i;
+            b += all;
+            __syncthreads();
+        }
     }
 }
 
@@ -566,7 +598,7 @@ void launch_flip_p2g(const Scene<double> &S, const FlipState &X, cudaStream_t st
     p2g_bucket_kernel<<<pb, 256, 0, st>>>(S, X);
     scan_u64(X.bcount, X.bstart, X.scan_tmp, nodes, st);
     p2g_scatter_kernel<<<pb, 256, 0, st>>>(S, X);
-    p2g_sort_kernel<<<blocks_for(nodes, 256), 256, 0, st>>>(X);
+    p2g_sort_kernel<<<blocks_for(nodes, kSortThreads), kSortThreads, 0, st>>>(S, X);
     const int gmax = (S.w + 1) * (S.h + 1);
     p2g_gather_kernel<<<dim3(blocks_for(gmax, 256), 3), 256, 0, st>>>(S, X);
     launch_extrapolate_guarded(S, 0xFu, X.ctl + FC_EMPTY, st);
