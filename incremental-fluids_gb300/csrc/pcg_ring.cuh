@@ -220,7 +220,7 @@ __device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &rin
     fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
     for (int blk = 0; blk < nblk; blk++) {
         ring_wait(R, R.bar(Ring<F>::FREE, R.st), R.parity ^ 1u, flags);
-        if ((threadIdx.x & 31) == 0) {
+        if ((threadIdx.x & 31) == 0 && !R.dead) {
             // without preparer and halo words the sweeping warp itself waits for the
             // copies; the barriers that nobody waits for keep pace
             uint64_t *ready = R.bar(Ring<F>::READY, R.st), *copied = R.bar(Ring<F>::COPIED, R.st);
