@@ -211,6 +211,7 @@ __device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &rin
     constexpr bool kPrepared = BWD && !REF;  // the preparer stands between the copies and the sweep
     constexpr int kT = Lay<F>::kSteps, kCells = Lay<F>::kCells;
     constexpr unsigned kVec = kVecBytes<F>;
+    if (ring.dead) return;
     Ring<F> R = ring;
     const Flags flags = A.fl;
     const int D = A.sd.D, nblk = D / kT;
@@ -219,8 +220,11 @@ __device__ __noinline__ void load_strip(const PcgArgs<F> &A, int s, Ring<F> &rin
     const F *cf = coef<REF, BWD>(A, row0 * kCells, 0);
     fence_proxy_async_global();  // generic-proxy writes before this sweep -> bulk copies
     for (int blk = 0; blk < nblk; blk++) {
-        ring_wait(R, R.bar(Ring<F>::FREE, R.st), R.parity ^ 1u, flags);
-        if ((threadIdx.x & 31) == 0 && !R.dead) {
+        if (!__all_sync(FULL, mbar_try_wait(R.bar(Ring<F>::FREE, R.st), R.parity ^ 1u))) {
+            ring_wait(R, R.bar(Ring<F>::FREE, R.st), R.parity ^ 1u, flags);
+            if (R.dead) break;
+        }
+        if ((threadIdx.x & 31) == 0) {
             // without preparer and halo words the sweeping warp itself waits for the
             // copies; the barriers that nobody waits for keep pace
             uint64_t *ready = R.bar(Ring<F>::READY, R.st), *copied = R.bar(Ring<F>::COPIED, R.st);
