@@ -263,6 +263,11 @@ PcgBatchPlan *pcg_batch_create(const Scene<F> *const *scenes, const PcgScratch *
         pcg_batch_destroy(P);
         return fail("device allocation for the batched PCG tables failed");
     }
+    if (cudaMemset(P->dev + o_tj, 0xff, grid * sizeof(int)) != cudaSuccess) {  // no job yet: -1
+        cudaGetLastError();
+        pcg_batch_destroy(P);
+        return fail("initialising the batched PCG tables failed");
+    }
     P->jobs[0] = P->dev + o_jobs0;
     P->jobs[1] = P->dev + o_jobs1;
     P->B.block_team = (const int2 *)(P->dev + o_bt);

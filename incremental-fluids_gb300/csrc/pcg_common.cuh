@@ -263,7 +263,9 @@ static __device__ int2 batch_slot(const BatchTeams &B, int *s_slot) {
 }
 
 // The team's next job into sA (shared by the block); false when the queue of
-// its class is empty.
+// its class is empty.  After a barrier that timed out the team's word may still be
+// an earlier job's or -1 (its value at creation), and may change: one thread reads
+// it for the block.
 template <typename F>
 __device__ bool batch_take(const BatchTeams &B, Team &T, int team, int cls, const PcgArgs<F> *jobs, PcgArgs<F> &sA,
                            int mode, int heat, int pinned, int K, int stages) {
@@ -274,7 +276,10 @@ __device__ bool batch_take(const BatchTeams &B, Team &T, int team, int cls, cons
         *(volatile int *)(B.team_job + team) = k < cr.y ? B.class_jobs[cr.x + k] : -1;
     }
     team_barrier(T, fl);
-    const int j = *(volatile int *)(B.team_job + team);
+    __shared__ int s_job;
+    if (threadIdx.x == 0) s_job = *(volatile int *)(B.team_job + team);
+    __syncthreads();
+    const int j = s_job;
     if (j < 0) return false;
     for (int k = threadIdx.x; k < (int)(sizeof(PcgArgs<F>) / 4); k += blockDim.x)
         ((unsigned *)&sA)[k] = ((const unsigned *)(jobs + j))[k];
