@@ -73,8 +73,6 @@ __device__ __forceinline__ FF ff_add(FF x, FF y) {
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
     return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
 }
-__device__ __forceinline__ float lo2(unsigned long long w) { return __uint_as_float((unsigned)w); }
-__device__ __forceinline__ float hi2(unsigned long long w) { return __uint_as_float((unsigned)(w >> 32)); }
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
 // a*b + c, element by element.
@@ -109,7 +107,7 @@ __device__ __noinline__ void prepare_strip(const PcgArgs<float> &A, int s, Ring<
         __syncwarp();
         if (lane == 0) {
             mbar_arrive(R.bar(Ring<float>::PREPARED, R.st));
-            if (!in) mbar_arrive(R.bar(Ring<float>::READY, R.st));  // else the loader's, with the halo words
+            if (!in) mbar_arrive(R.bar(Ring<float>::READY, R.st));  // else the taker's, with the halo words
         }
         qq += to_f64((qs.x + qs.y) + (qs.z + qs.w));
         R.next();

@@ -56,7 +56,7 @@ __device__ __noinline__ void prepare_strip(const PcgArgs<double> &A, int s, Ring
         __syncwarp();
         if (lane == 0) {
             mbar_arrive(R.bar(Ring<double>::PREPARED, R.st));
-            if (!in) mbar_arrive(R.bar(Ring<double>::READY, R.st));  // else the loader's, with the halo words
+            if (!in) mbar_arrive(R.bar(Ring<double>::READY, R.st));  // else the taker's, with the halo words
         }
         R.next();
     }
@@ -209,7 +209,7 @@ __device__ __forceinline__ double matvec_row(const PcgArgs<double> &A, const Cel
 }
 
 // The matvec and z'.s over this warp's chunks.
-template <bool ROWSUM>
+template <bool ROWSUM>  // the FP32 form's: the pass is the same for every matrix here
 __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double beta, int c_begin, int c_end, int c_step,
                                     int kc) {
     const int lane = threadIdx.x & 31;

@@ -10,9 +10,6 @@ namespace ifl {
 // that every ring and halo access compiles to a shared-space instruction.
 extern __shared__ __align__(128) char g_smem[];
 
-// Warps of the largest block: 512 threads for a scene that has the GPU to
-// itself, at most 256 in the launch used when many scenes run concurrently.
-constexpr int kMaxWarps = 16;
 // Default polls of a halo-word or barrier wait (about a second); the host may
 // set another limit per solve (PcgConfig::wait_limit).  The mbarrier waits of
 // the bulk-copy rings keep their own fixed limit: they wait for copies this
@@ -137,19 +134,10 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_max(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = smax(v, __shfl_down_sync(FULL, v, o));
-    return v;
-}
 
 // ------------------------------------------------------------ halo words
 __device__ __forceinline__ unsigned long long henc(double v) { return (unsigned long long)__double_as_longlong(v); }
-__device__ __forceinline__ unsigned long long henc(float v) { return (unsigned long long)__float_as_uint(v); }
-template <typename V> __device__ __forceinline__ V hdec(unsigned long long w);
-template <> __device__ __forceinline__ double hdec<double>(unsigned long long w) {
-    return __longlong_as_double((long long)w);
-}
-template <> __device__ __forceinline__ float hdec<float>(unsigned long long w) { return __uint_as_float((unsigned)w); }
+__device__ __forceinline__ double hdec(unsigned long long w) { return __longlong_as_double((long long)w); }
 
 // Halo rows: shared memory between warps of one block, global memory between
 // blocks.  A channel holds the row's generic address, so one instruction
@@ -220,7 +208,7 @@ struct BatchTeams {
     const int *class_jobs;    // job indices, each class in queue order
     int *class_next;          // queue heads (zero at launch)
     int *team_job;            // job taken by each team
-    unsigned *team_bar;       // barrier counter of each team, 128 bytes apart (zero at launch)
+    unsigned *team_bar;       // barrier counter of each team, kBarStride words apart (zero at launch)
     unsigned *all;            // launch-wide status word
     const int4 *ctl;          // per job: {pinned pressure, pinned heat, limit pressure, limit heat}
     // Placement of teams across SMs: the hardware puts consecutive blocks of a

@@ -159,13 +159,14 @@ __device__ void pcg_job(const PcgArgs<F> &A, Team &T, Ring<F> &R, double *sm) {
             // block-uniform: every thread of the block leaves together
             if ((iter & 15) == 0 && __syncthreads_or(threadIdx.x == 0 && timed_out(A.fl))) break;
             if constexpr (REF) ref_matvec(A, T, iter, beta);
-            else if (pressure) matvec<true>(A, iter, (F)beta, c_begin, c_end, nwarps, kc);
-            else matvec<false>(A, iter, (F)beta, c_begin, c_end, nwarps, kc);
+            else if (sizeof(F) == 8 || !pressure) matvec<false>(A, iter, (F)beta, c_begin, c_end, nwarps, kc);
+            else matvec<true>(A, iter, (F)beta, c_begin, c_end, nwarps, kc);
             team_barrier(T, A.fl);
             const double alpha = sigma / dot_of();
+            constexpr bool kRowsum = sizeof(F) == 4;  // FP64 passes are the same for every matrix
             if (!pressure) axpy<REF, false, true>(A, iter, alpha, c_begin, c_end, nwarps, kc);
-            else if (masked) axpy<REF, true, true>(A, iter, alpha, c_begin, c_end, nwarps, kc);
-            else axpy<REF, true, false>(A, iter, alpha, c_begin, c_end, nwarps, kc);
+            else if (masked) axpy<REF, kRowsum, true>(A, iter, alpha, c_begin, c_end, nwarps, kc);
+            else axpy<REF, kRowsum, false>(A, iter, alpha, c_begin, c_end, nwarps, kc);
             team_barrier(T, A.fl);
             iterations = iter + 1;
             // z = M^-1 r; sigmaNew = z.r  (:372-376); a solve that has converged has
@@ -312,7 +313,7 @@ cudaError_t launch_single(PcgArgs<F> A, const PcgScratch &X, const PcgConfig &cf
     // FP32 grids with more chunks than the warps of 256-thread blocks (above about
     // 550^2): twice the warps for the elementwise passes.  Cycles per iteration of
     // matvec and AXPYs, without their barriers, 256 and 512 threads: 768^2 33K and 28K,
-    // 1536^2 88K and 58K; smaller grids only have more warps at the barriers.
+    // 1536^2 88K and 58K (clock counters of a scratch copy); smaller grids only have more warps at the barriers.
     const int threads = sizeof(F) == 4 && pcg_chunks(sd) > (size_t)sms * kSingleThreads / 32 ? kMaxThreads<F> : kSingleThreads;
     void *args[] = {&A};
     return cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), args, smem, st);

@@ -119,7 +119,7 @@ __device__ __forceinline__ F *coef(const PcgArgs<F> &A, size_t k, int arr) {
 //    and hands its boundary row on, and frees the stage.
 // Every wait is bounded.  A timeout elsewhere in the launch does not shorten the
 // mbarrier waits: the copies were issued from this GPU's memory and complete,
-// and the loader's halo polls give up by themselves, so a timed-out sweep still
+// and the taker's halo polls give up by themselves, so a timed-out sweep still
 // consumes every block it issued and no bulk copy is left behind in shared memory.
 // A ring is `dead` once an mbarrier wait ran out all the same: its warp then
 // waits and issues no more.
@@ -352,7 +352,7 @@ __device__ __noinline__ void factor_rows(const PcgArgs<F> &A, int q, const Chan 
         if constexpr (IN) {
             const bool need = lane == 0 && t < W;
             const unsigned long long w = halo_take_warp(in, t, need, nword, A.fl);
-            if (need) down = hdec<double>(w);
+            if (need) down = hdec(w);
         }
         if (t + 1 < W + 31) prefetch(t + 1);
         double ev = diag;
