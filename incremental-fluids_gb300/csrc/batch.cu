@@ -369,8 +369,8 @@ class BatchImpl final : public BatchBase {
     // strip s starts a hand-over (lag) after strip s-1 and not before its warp
     // finished strip s-P.  The elementwise passes cost a fixed time per cell and
     // warp; the totals and, for a team of more than one block, its barriers a fixed
-    // time.  Constants from per-phase timers in the batched kernel on GB300
-    // (512-scene batch, 128-thread blocks, three to an SM).
+    // time.  Constants from per-phase timers in a scratch copy of the batched kernel
+    // on GB300 (512-scene batch, 128-thread blocks, three to an SM).
     double plan_cost(int i, int g) const {
         constexpr bool f32 = sizeof(F) == 4;
         constexpr double kTau = f32 ? 0.14 : 0.11, kLag = 6.0, kElemNs = f32 ? 7.7 : 10.0;

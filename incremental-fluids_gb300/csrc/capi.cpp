@@ -103,7 +103,6 @@ int ifl_create(const ifl_params *p, ifl_solver **out) {
     *out = nullptr;
     if (p->variant < IFL_GS_EULER || p->variant > IFL_FLIP) return IFL_ERR_ARG;
     if (p->w < 2 || p->h < 2 || p->w > 32768 || p->h > 32768) return IFL_ERR_ARG;
-    if (p->variant <= IFL_GS && p->h > ifl::gs_max_rows()) return IFL_ERR_UNSUPPORTED;  // a worker per strip
     if (p->precision != IFL_FP64 && p->precision != IFL_FP32) return IFL_ERR_ARG;
     if (p->variant == IFL_FLIP && (int64_t)p->w * p->h * 12 > 0x7fffffff) return IFL_ERR_UNSUPPORTED;
     if (p->device < 0) return IFL_ERR_ARG;

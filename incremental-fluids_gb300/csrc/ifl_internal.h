@@ -174,9 +174,9 @@ struct PcgConfig {
 // Launch shape of the batched PCG kernel (chosen by the batch autotuner); a request
 // that pcg_shape (pcg_job.cuh) fits to threads and shared memory.
 struct PcgShape {
-    int threads;  // 32, 64, 128 or 256 threads per block
-    int K;        // strips (sweeping warps) per block, <= threads / 32
-    int stages;   // ring stages per strip, 2..4
+    int threads;  // 32, 64, 128 or 256 threads per block; a block gets at least 128 per strip
+    int K;        // strips per block, <= threads / 32; at most four, and as many as shared memory holds
+    int stages;   // ring stages per strip, 2..4, fewer where shared memory does not hold them
 };
 
 // Launchers (stream-ordered, no host synchronisation).
@@ -205,11 +205,10 @@ struct PcgF32 {
 };
 cudaError_t launch_pcg_f32(const Scene<double> &S, const PcgF32 &M, const PcgScratch &X, const PcgConfig &c,
                            cudaStream_t st, int *blocks_used);
-// Gauss-Seidel solve of steps 1-2 (k_gs.cu): h <= gs_max_rows().
+// Gauss-Seidel solve of steps 1-2 (k_gs.cu).
 template <typename F>
 cudaError_t launch_gs(const Scene<F> &S, const PcgScratch &X, double dt, int limit, int pinned, cudaStream_t st,
                       long long wait_limit = 0);
-int gs_max_rows();
 size_t gs_words(const SDIdx &sd, int sms);  // words of PcgScratch::gs
 
 // Batched PCG: many scenes in one cooperative launch (k_pcg.cu).  The plan

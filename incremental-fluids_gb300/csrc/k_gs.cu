@@ -359,8 +359,6 @@ void gs_plan(const SDIdx &sd, int sms, int *J, int *L) {
 
 }  // namespace
 
-int gs_max_rows() { return 32 * 4096; }
-
 size_t gs_words(const SDIdx &sd, int sms) {
     int J, L;
     gs_plan(sd, sms, &J, &L);

@@ -37,7 +37,7 @@
 // and in the backward sweep a preparer forms dd y and sigma.  What is left per step is 6 loads of 16
 // bytes from shared memory, 16 fused multiply-adds, two shuffles and three
 // stores: 150 cycles, of which the multiply-adds are 63, the loads 45, the
-// stores 30 (timed with each left out).
+// stores 30 (timed in a scratch copy with each left out).
 //
 // r and p are FP64; the matvec is FP32 (its results are stored as they are
 // formed), dot products, the maximum norm, alpha and beta are FP64.

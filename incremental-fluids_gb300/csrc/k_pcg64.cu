@@ -20,7 +20,9 @@
 // had (REF): for some placements of the bodies their conjugate gradients amplify
 // a last-bit difference, even of the order of a sum, by up to 1e8 (24 seeded
 // scenes of steps 5-7: velocities up to 1e-8 off; a 48 x 66 scene of step 7 in
-// one step 2e-8 off the oracle's, beyond the 1e-8 that this form holds).
+// one step 2e-8 off the oracle's).  Bit for bit the reference's are the factor and
+// each application of the preconditioner; the order of the sums, and with it the last
+// bits of alpha and beta, is this form's own.
 #include "pcg_ring.cuh"
 
 namespace ifl {
@@ -209,7 +211,7 @@ __device__ __forceinline__ double matvec_row(const PcgArgs<double> &A, const Cel
 }
 
 // The matvec and z'.s over this warp's chunks.
-template <bool ROWSUM>  // the FP32 form's: the pass is the same for every matrix here
+template <bool ROWSUM>  // the FP32 form's: always false here
 __device__ __noinline__ void matvec(const PcgArgs<double> &A, int iter, double beta, int c_begin, int c_end, int c_step,
                                     int kc) {
     const int lane = threadIdx.x & 31;
