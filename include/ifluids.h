@@ -265,7 +265,9 @@ int ifl_get_timing(ifl_solver *s, ifl_timing *out);
  * Solves the unmasked MIC(0)-preconditioned CG system of
  * 3-conjugate-gradients (buildPreconditioner + project) for a w x h grid:
  * adiag, aplusx, aplusy, rhs and p are DEVICE arrays, dense row-major
- * (idx = x + y*w), FP64; `stats` is a DEVICE ifl_pcg_stats the solve writes
+ * (idx = x + y*w), FP64.  Entries of neighbours that do not exist (aplusx in
+ * the last column, aplusy in the last row) need not be zero: as in the
+ * reference, buildPreconditioner reads them and nothing else does.  `stats` is a DEVICE ifl_pcg_stats the solve writes
  * its outcome into (status -1: a bounded device-side wait timed out).
  * Work is enqueued on `stream` (NULL: the default stream); nothing is
  * synchronised.

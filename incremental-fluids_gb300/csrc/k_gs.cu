@@ -38,7 +38,7 @@
 // before waits for an entry of its own (`decided`): the last sweeps, and with
 // them their verdicts, do not exist if an earlier one converged.
 //
-// 600 sweeps at 128 x 128: 2.2 ms; 116 ms with one sweep and the head of the next in
+// 600 sweeps at 128 x 128: 1.9 ms; 111 ms with one sweep and the head of the next in
 // flight, a hand-over with a fence every four diagonals and a division per cell.
 //
 // Every wait is bounded; a timeout sets the status word and an abort word that
@@ -345,7 +345,7 @@ size_t ring_words(const SDIdx &sd, int L) {
 // with four.  The verdict of a sweep comes after the last strip's last step (36
 // steps per strip: 32 rows and the hand-over).  The ring is kept below kRingBytes
 // with fewer sweeps in flight, but not below the three buffers of 16-byte entries
-// that one sweep and its successor need: 0.8 GB at 4096^2, 52 GB at 32768^2, where
+// that one sweep and its successor need: 0.9 GB at 4096^2, 55 GB at 32768^2, where
 // a handle has fewer arrays for it (solver.cu).
 constexpr size_t kRingBytes = (size_t)512 << 20;
 void gs_plan(const SDIdx &sd, int sms, int *J, int *L) {
