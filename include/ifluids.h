@@ -352,7 +352,7 @@ enum {
 
 typedef struct {
     int32_t members;
-    int32_t threads, strips_per_block, stages;  /* PCG shape in use            */
+    int32_t threads, strips_per_block, stages;  /* PCG shape requested or tuned */
     int32_t grid;                               /* blocks of the PCG launch    */
     int32_t graph;                              /* 1: steps replay a CUDA graph */
     int32_t candidates;                         /* shapes tried by the autotuner */
