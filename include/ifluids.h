@@ -267,8 +267,9 @@ int ifl_get_timing(ifl_solver *s, ifl_timing *out);
  * adiag, aplusx, aplusy, rhs and p are DEVICE arrays, dense row-major
  * (idx = x + y*w), FP64.  Entries of neighbours that do not exist (aplusx in
  * the last column, aplusy in the last row) need not be zero: as in the
- * reference, buildPreconditioner reads them and nothing else does.  `stats` is a DEVICE ifl_pcg_stats the solve writes
- * its outcome into (status -1: a bounded device-side wait timed out).
+ * reference, buildPreconditioner reads them and nothing else does.  `stats`
+ * is a DEVICE ifl_pcg_stats the solve writes its outcome into (status -1: a
+ * bounded device-side wait timed out).
  * Work is enqueued on `stream` (NULL: the default stream); nothing is
  * synchronised.
  *
